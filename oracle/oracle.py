@@ -27,14 +27,14 @@ _vp = ct.c_void_p
 
 
 def build(ref: bool | None = None) -> None:
-    """Compile liboracle.so (and the reference groups when the tree exists)."""
+    """Compile liboracle.so (and the reference groups when its sources are there)."""
     targets = ["all"]
     # the reference checkout: PAGANI_REF_ROOT, else a "reference" directory
     # beside the repository
     ref_root = os.environ.get("PAGANI_REF_ROOT", os.path.join(os.path.dirname(HERE), "..", "reference"))
     ref_root = os.path.abspath(ref_root)
     if ref is None:
-        ref = os.path.isdir(ref_root)
+        ref = os.path.isdir(os.path.join(ref_root, "src"))
     if ref:
         targets.append("ref")
     targets.append("big")
