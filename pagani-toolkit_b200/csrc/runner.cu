@@ -117,8 +117,7 @@ pg_status run_surrogates(pg_ctx* ctx, const pg_graph* g, int32_t subject, const 
     PG_TRY(ms_enqueue(ctx, g, &c.ms));
     PG_TRY(ms_rows_enqueue(ctx, g, &c.ms, c.sg.C, c.sg.V));
     if (c.weighted) {
-        const pg_graph* one[1] = {&c.sg};
-        PG_TRY(onnela_prepare(ctx, one, 1, 0, c.cp, c.cp_mean, &c.onn));
+        PG_TRY(onnela_prepare(ctx, &c.sg, 0, c.cp, c.cp_mean, &c.onn));
         PG_TRY(onnela_enqueue(ctx, &c.onn));
     } else {
         PG_TRY(binary_cp_prepare(ctx, g->n, &c.bin));

@@ -1,0 +1,74 @@
+"""Branches of the kernels' dispatch rules, at the sizes where they change,
+against the oracle or an FP64 restatement."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests import graphs as G
+
+pytestmark = pytest.mark.gpu
+
+
+# ------------------------------------------------------------------ Onnela
+def _hub(n):
+    """Node 0 connected to every other one, a ring and random chords among them."""
+    rng = np.random.default_rng(n)
+    edges = [(0, i) for i in range(1, n)] + [(i, i % (n - 1) + 1) for i in range(1, n)]
+    edges += [tuple(rng.integers(1, n, 2)) for _ in range(4 * n)]
+    return G.csr_from_edges(n, edges, [np.float32(x) for x in rng.uniform(0.1, 1.0, len(edges))])
+
+
+@pytest.mark.parametrize("n", [3, 31, 33, 257, 1537, 1538, 2100])
+def test_onnela_row_lengths(ctx, n):
+    """Rows on both sides of the roots kept in shared memory (1536)."""
+    R, C, V = _hub(n)
+    cp, _, mean = ctx.clustering(ctx.graph(R, C, V), kind="onnela")
+    cp_or, mean_or = O.onnela(R, C, V)
+    # FP64 sums of non-negative terms, rounded to float once: half an ulp each side
+    np.testing.assert_allclose(cp, cp_or, rtol=2.0 ** -23, atol=0)
+    assert mean == pytest.approx(mean_or, rel=2.0 ** -23)
+
+
+@pytest.mark.parametrize("change", ["negative", "zero", "all_zero", "infinite", "nan"])
+def test_onnela_unusual_weights(ctx, change):
+    """Weights that the product of cube roots does not cover take the general kernel."""
+    R, C, V = G.random_weighted(120, 0.3, 5)
+    rows = np.repeat(np.arange(120), np.diff(R))
+    lo, hi = np.minimum(rows, C), np.maximum(rows, C)
+    pick = (lo * 7 + hi * 13) % 11 == 0
+    V = V.copy()
+    if change == "all_zero":
+        V[:] = 0
+    else:
+        V[pick] = {"negative": -V[pick], "zero": 0.0, "infinite": np.inf, "nan": np.nan}[change]
+    cp, _, _ = ctx.clustering(ctx.graph(R, C, V), kind="onnela")
+    with np.errstate(all="ignore"):
+        A = np.zeros((120, 120))
+        has = np.zeros((120, 120), bool)
+        A[rows, C] = V / (np.nanmax(V) if change == "nan" else V.max())
+        has[rows, C] = True
+        want = np.zeros(120)
+        for u in range(120):
+            nb = np.nonzero(has[u])[0]
+            k = len(nb)
+            t = 0.0
+            for x, j in enumerate(nb):
+                for h in nb[x + 1:]:
+                    if has[j, h] and A[j, h] != 0:
+                        t += (A[j, h] * A[u, j] * A[u, h]) ** (1.0 / 3.0) if A[j, h] * A[u, j] * A[u, h] >= 0 \
+                            else np.nan
+            want[u] = 2.0 * t / k / (k - 1) if k >= 2 else 0.0
+    np.testing.assert_allclose(cp, want.astype(np.float32), rtol=2.0 ** -22, atol=0, equal_nan=True)
+
+
+def test_onnela_rows_out_of_order(ctx):
+    """Rows whose columns do not ascend: j's scan takes any order, as before
+    (u's own row is searched, so only rows without pairs above are shuffled)."""
+    R = np.array([0, 3, 6, 9, 12], np.int32)          # K4
+    C = np.array([1, 2, 3, 0, 2, 3, 0, 1, 3, 0, 1, 2], np.int32)
+    V = np.array([.5, .6, .7, .5, .8, .9, .6, .8, 1., .7, .9, 1.], np.float32)
+    want, _, _ = ctx.clustering(ctx.graph(R, C, V), kind="onnela")
+    C2, V2 = C.copy(), V.copy()
+    C2[9:12], V2[9:12] = [1, 0, 2], [.9, .7, 1.]      # node 3's row, swapped
+    got, _, _ = ctx.clustering(ctx.graph(R, C2, V2), kind="onnela")
+    np.testing.assert_allclose(got[:3], want[:3], rtol=2.0 ** -22)
