@@ -3,6 +3,7 @@
 #include "pg_internal.cuh"
 #include <cstring>
 #include <cstdlib>
+#include <algorithm>
 #include <cmath>
 #include <new>
 
@@ -455,13 +456,35 @@ __global__ void k_pair_degrees(const int2* __restrict__ pairs, long long np, int
     }
 }
 
-__global__ void k_off_to_rowptr(const long long* __restrict__ off, int32_t n, int32_t* __restrict__ R,
-                                int32_t* __restrict__ cursor)
+// Row offsets from the row counts in two launches: sums of 1024 rows, then
+// every block adds the sums before its own and scans its rows into R and the
+// scatter cursors (cnt itself).
+__global__ void __launch_bounds__(SCAN_B) k_row_sums(const int32_t* __restrict__ cnt, int32_t n,
+                                                     long long* __restrict__ bsum)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= n;
-         i += (long long)gridDim.x * blockDim.x) {
-        R[i] = (int32_t)off[i];
-        if (i < n) cursor[i] = (int32_t)off[i];
+    __shared__ long long sh[32];
+    const long long i = (long long)blockIdx.x * SCAN_B + threadIdx.x;
+    long long tot;
+    block_excl_scan_1024(i < n ? cnt[i] : 0, sh, &tot);
+    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(SCAN_B) k_row_offsets(int32_t* __restrict__ cnt, int32_t n,
+                                                        const long long* __restrict__ bsum, int32_t* __restrict__ R)
+{
+    __shared__ long long sh[32];
+    long long before = 0, tot;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += SCAN_B) before += bsum[b];
+    block_excl_scan_1024(before, sh, &tot);
+    before = tot;
+    __syncthreads();
+    const long long i = (long long)blockIdx.x * SCAN_B + threadIdx.x;
+    const int32_t c = i < n ? cnt[i] : 0;
+    const int32_t at = (int32_t)(before + block_excl_scan_1024(c, sh, &tot));
+    if (i < n) {
+        R[i] = at;
+        cnt[i] = at;
+        if (i == n - 1) R[n] = at + c;
     }
 }
 
@@ -600,22 +623,24 @@ pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const flo
 {
     if (2 * npairs > INT32_MAX)
         return pg_fail(ctx, PG_ERR_TOO_LARGE, "%lld directed entries exceed the int32 CSR", 2LL * npairs);
+    const int nb = ceil_div(std::max(n, 1), SCAN_B);
     int32_t* cnt;
-    long long* off;
+    long long* bsum;
     PG_TRY(pg_wst(ctx, "csr.cnt", (size_t)n + 1, &cnt));
-    PG_TRY(pg_wst(ctx, "csr.off", (size_t)n + 2, &off));
+    PG_TRY(pg_wst(ctx, "csr.bsum", (size_t)nb, &bsum));
     PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)n + 1), ctx->stream));
     int grid = ctx->sm_count * 8;
     if (npairs > 0) {
         k_pair_degrees<<<grid, 256, 0, ctx->stream>>>(pairs, npairs, cnt);
         PG_LAUNCHED(ctx);
     }
-    PG_TRY(pg_scan_counts(ctx, cnt, (int64_t*)off, n));
     pg_graph* g;
     PG_TRY(pg_graph_alloc(ctx, n, 2 * npairs, w != nullptr, &g));
-    int32_t* cursor = cnt;  // counts are no longer needed
-    k_off_to_rowptr<<<ceil_div((long long)n + 1, 256), 256, 0, ctx->stream>>>(off, n, g->R, cursor);
-    PG_LAUNCHED(ctx);
+    k_row_sums<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum);
+    ctx->launches++;
+    k_row_offsets<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum, g->R);
+    ctx->launches++;
+    int32_t* cursor = cnt;  // the counts became the offsets
     if (npairs > 0) {
         int32_t* Ct;
         float* Vt = nullptr;

@@ -12,31 +12,108 @@
 // Restates the normalisation of CorMat_gpu (U/CorMat/CUCorMat/CUCORMAT/
 // CorMat.cu:34-53) in FP64 with explicit round-to-nearest operations, so the
 // result is bit-identical to the oracle (no contraction into FMA).
-__global__ void k_zstats(const float* __restrict__ bold, int N, int T, double* __restrict__ mu,
-                         double* __restrict__ sd, int* __restrict__ nzero)
+// A block takes 32 voxels.  Warps 1-7 read the samples, two chunks of 56 time
+// points ahead in registers, and leave them in shared memory as the FP64
+// terms of the sum; warp 0 adds them in order, one voxel per lane.  Where the
+// voxels are few that chain of additions bounds it (8.7 cycles each), so
+// nothing else is left in it; where they are many, the two reads of the
+// series.  90 x 1200: 159 us when every lane loaded, converted and added its
+// own samples, 26 us now; 58,000 x 240: 39 us both ways.
+constexpr int ZT = 56, ZPROD = 7, ZROWS = (ZT + ZPROD - 1) / ZPROD;
+
+__device__ __forceinline__ void z_fetch(float (&v)[ZROWS], const float* __restrict__ bold, int N, int T, int c, int i,
+                                        int prod)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < ZROWS; k++) {
+        const int r = prod + k * ZPROD, t = c * ZT + r;
+        v[k] = (r < ZT && t < T && i < N) ? bold[(size_t)t * N + i] : 0.0f;
+    }
+}
+
+template <bool SQUARES>
+__device__ __forceinline__ void z_store(double (*buf)[32], const float (&v)[ZROWS], double mean, int lane, int prod)
+{
+#pragma unroll
+    for (int k = 0; k < ZROWS; k++) {
+        const int r = prod + k * ZPROD;
+        if (r >= ZT) break;
+        const double d = SQUARES ? __dsub_rn((double)v[k], mean) : (double)v[k];
+        buf[r][lane] = SQUARES ? __dmul_rn(d, d) : d;
+    }
+}
+
+// sum over t of x, or of (x - mean)^2, per lane of warp 0 (others return 0)
+template <bool SQUARES>
+__device__ __forceinline__ double z_sum(double (*buf)[ZT][32], const float* __restrict__ bold, int N, int T, int i,
+                                        double mean)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, prod = warp - 1;
+    const int nc = (T + ZT - 1) / ZT;
+    float v0[ZROWS], v1[ZROWS];
+    if (warp) {
+        z_fetch(v0, bold, N, T, 0, i, prod);
+        z_fetch(v1, bold, N, T, 1, i, prod);
+        z_store<SQUARES>(buf[0], v0, mean, lane, prod);
+    }
+    __syncthreads();
+    double s = 0.0;
+    auto add = [&](int c) {
+        const int cnt = min(ZT, T - c * ZT);
+        if (cnt == ZT) {
+#pragma unroll
+            for (int r = 0; r < ZT; r++) s = __dadd_rn(s, buf[c & 1][r][lane]);
+        } else {
+            for (int r = 0; r < cnt; r++) s = __dadd_rn(s, buf[c & 1][r][lane]);
+        }
+    };
+    // step c: chunk c is added while chunk c + 1 is stored and c + 2 is read
+    for (int c = 0; c < nc; c += 2) {
+        if (warp == 0) {
+            add(c);
+        } else {
+            z_fetch(v0, bold, N, T, c + 2, i, prod);
+            z_store<SQUARES>(buf[1], v1, mean, lane, prod);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (c + 1 < nc) add(c + 1);
+        } else {
+            z_fetch(v1, bold, N, T, c + 3, i, prod);
+            z_store<SQUARES>(buf[0], v0, mean, lane, prod);
+        }
+        __syncthreads();
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(32 * (1 + ZPROD), 5)
+k_zstats(const float* __restrict__ bold, int N, int T, double* __restrict__ mu, double* __restrict__ sd,
+         int* __restrict__ nzero)
+{
+    __shared__ double buf[2][ZT][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    const double s1 = __ddiv_rn(z_sum<false>(buf, bold, N, T, i, 0.0), (double)T);
+    if (warp == 0) buf[1][0][lane] = s1;
+    __syncthreads();
+    const double mean = buf[1][0][lane];
+    __syncthreads();
+    const double s2 = __dsqrt_rn(z_sum<true>(buf, bold, N, T, i, mean));
+    if (warp != 0) return;
     bool zero = false;
     if (i < N) {
-        double s1 = 0.0;
-        for (int t = 0; t < T; t++) s1 = __dadd_rn(s1, (double)bold[(size_t)t * N + i]);
-        s1 = __ddiv_rn(s1, (double)T);
-        double s2 = 0.0;
-        for (int t = 0; t < T; t++) {
-            double d = __dsub_rn((double)bold[(size_t)t * N + i], s1);
-            s2 = __dadd_rn(s2, __dmul_rn(d, d));
-        }
-        s2 = __dsqrt_rn(s2);
         zero = !(s2 > 0.0) || isinf(s2) || isnan(s2);
         mu[i] = s1;
         sd[i] = zero ? 0.0 : s2;
     }
-    unsigned m = __ballot_sync(0xffffffffu, zero);
-    if ((threadIdx.x & 31) == 0 && m) atomicAdd(nzero, __popc(m));
+    const unsigned m = __ballot_sync(0xffffffffu, zero);
+    if (lane == 0 && m) atomicAdd(nzero, __popc(m));
 }
 
 // 32x32 transposing tiles: reads bold[t][i] along i, writes z rows along t.
-__global__ void k_zwrite(const float* __restrict__ bold, int N, int T, int Tp, const double* __restrict__ mu,
+// Only the operands that the build needs are written (null: not needed).
+__global__ void k_zwrite(const float* __restrict__ bold, int N, int T, int Ts, int Tp, const double* __restrict__ mu,
                          const double* __restrict__ sd, double* __restrict__ z64, float* __restrict__ z32,
                          __nv_bfloat16* __restrict__ zhi, __nv_bfloat16* __restrict__ zlo)
 {
@@ -52,52 +129,133 @@ __global__ void k_zwrite(const float* __restrict__ bold, int N, int T, int Tp, c
         if (t >= Tp) continue;
         double z = 0.0;
         if (i < N && t < T && sd[i] > 0.0) z = __ddiv_rn(__dsub_rn((double)tile[threadIdx.x][r], mu[i]), sd[i]);
-        if (i < N && t < T) z64[(size_t)i * T + t] = z;
+        if (i < N && t < T) z64[(size_t)i * Ts + t] = z;
         float f = __double2float_rn(z);
-        __nv_bfloat16 h = __float2bfloat16_rn(f);
-        __nv_bfloat16 l = __float2bfloat16_rn(__fsub_rn(f, __bfloat162float(h)));
         size_t o = (size_t)i * Tp + t;
-        z32[o] = f;
-        zhi[o] = h;
-        zlo[o] = l;
+        if (z32) z32[o] = f;
+        if (zhi) {
+            __nv_bfloat16 h = __float2bfloat16_rn(f);
+            zhi[o] = h;
+            zlo[o] = __float2bfloat16_rn(__fsub_rn(f, __bfloat162float(h)));
+        }
     }
 }
 
 // --------------------------------------------------------- FP64 recheck
 // r(i,j) exactly as the oracle: sequential t, one fused multiply-add per
 // term; then the reference's range rule (post_block, CorMat.cpp:821 /
-// W CorMat.cpp:821).  Key = r or |r|.
-__device__ __forceinline__ double exact_r(const double* __restrict__ z64, int T, int i, int j, int weighted)
+// W CorMat.cpp:821).  Key = r or |r|.  Rows start on 32-byte boundaries
+// (stride Ts, a multiple of four), so a thread reads four samples of a row
+// per load, eight such loads ahead of the sixteen additions they feed.
+// KEEP: the compiler may not move the load towards its use.
+template <bool KEEP>
+__device__ __forceinline__ void load4(double (&x)[4], const double* p)
 {
-    const double* a = z64 + (size_t)i * T;
-    const double* b = z64 + (size_t)j * T;
+    if (KEEP)
+        asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
+                     : "l"(p));
+    else
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
+}
+
+struct Samples16 {
+    double x[4][4], y[4][4];
+    template <bool KEEP>
+    __device__ __forceinline__ void load(const double* a, const double* b)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            load4<KEEP>(x[q], a + 4 * q);
+            load4<KEEP>(y[q], b + 4 * q);
+        }
+    }
+    __device__ __forceinline__ double add(double r) const
+    {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) r = __fma_rn(x[q][c], y[q][c], r);
+        return r;
+    }
+};
+
+// AHEAD: the next sixteen samples are loaded before the last sixteen are
+// added (twice the registers): for lists too short to fill the GPU, where a
+// pair is one chain of load latencies.
+template <bool AHEAD>
+__device__ __forceinline__ double dot_exact(const double* __restrict__ a, const double* __restrict__ b, int T)
+{
     double r = 0.0;
-    for (int t = 0; t < T; t++) r = __fma_rn(a[t], b[t], r);
+    int t = 0;
+    if (AHEAD && T >= 16) {
+        Samples16 s0, s1;
+        s0.load<true>(a, b);
+        for (; t + 48 <= T; t += 32) {
+            s1.load<true>(a + t + 16, b + t + 16);
+            r = s0.add(r);
+            s0.load<true>(a + t + 32, b + t + 32);
+            r = s1.add(r);
+        }
+        r = s0.add(r);
+        t += 16;
+    }
+    for (; t + 16 <= T; t += 16) {
+        Samples16 s;
+        s.load<false>(a + t, b + t);
+        r = s.add(r);
+    }
+    for (; t + 4 <= T; t += 4) {
+        double x[4], y[4];
+        load4<false>(x, a + t);
+        load4<false>(y, b + t);
+#pragma unroll
+        for (int c = 0; c < 4; c++) r = __fma_rn(x[c], y[c], r);
+    }
+    for (; t < T; t++) r = __fma_rn(a[t], b[t], r);
+    return r;
+}
+
+__device__ __forceinline__ double range_rule(double r, int weighted)
+{
     if (weighted) return (r > -1.0 - 1e-6 && r < 1.0 + 1e-6) ? r : 0.0;
     return (r >= -1.0 && r <= 1.0) ? r : 0.0;
 }
 
 // FP64 r of every band pair, and the error of the tile's r against it:
 // err[0] = bits of max |r_tile - r| (non-negative doubles order as their
-// bits), err[1] = sum of |r_tile - r| (r before the range rule).
-__global__ void k_recheck(const int2* __restrict__ band, const float* __restrict__ band_r, long long nband,
-                          const double* __restrict__ z64, int T, int weighted, int abs_mode,
-                          double* __restrict__ key64, unsigned long long* __restrict__ err)
+// bits), err[1] = sum of |r_tile - r| (r before the range rule).  With pair_w
+// set, also the exact weight of every pair that the tiles decided (once per
+// undirected pair: both directions have the same terms).  The lists are in
+// tile order, so the pairs of a block share rows in L1; bound by those row
+// reads.  58,000 voxels, top 1 %: 1.07 ms, 2.86 ms with one 8-byte load per
+// term; the exact weights of 25,211 voxels (3.2M pairs, with
+// 0.3M of the band) 1.02 ms, 3.2 ms when
+// each of the 6.4M CSR entries was evaluated in row order.
+template <bool AHEAD>
+__global__ void __launch_bounds__(128, AHEAD ? 3 : 8)
+k_pair_exact(const int2* __restrict__ band, const float* __restrict__ band_r, const int2* __restrict__ pairs,
+             float* __restrict__ pair_w, const unsigned long long* __restrict__ counts, long long cap_pairs,
+             long long cap_band, const double* __restrict__ z64, int T, int Ts, int weighted, int abs_mode,
+             double* __restrict__ key64, unsigned long long* __restrict__ err)
 {
+    const long long nband = min((long long)counts[1], cap_band);
+    const long long total = nband + (pair_w ? min((long long)counts[0], cap_pairs) : 0LL);
     double emax = 0.0, esum = 0.0;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < nband;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
          q += (long long)gridDim.x * blockDim.x) {
-        int2 e = band[q];
-        const double* a = z64 + (long long)e.x * T;
-        const double* b = z64 + (long long)e.y * T;
-        double r = 0.0;
-        for (int t = 0; t < T; t++) r = __fma_rn(a[t], b[t], r);
-        const double d = fabs((double)band_r[q] - r);
-        emax = fmax(emax, d);
-        esum += d;
-        if (weighted) r = (r > -1.0 - 1e-6 && r < 1.0 + 1e-6) ? r : 0.0;
-        else r = (r >= -1.0 && r <= 1.0) ? r : 0.0;
-        key64[q] = abs_mode ? fabs(r) : r;
+        const bool in_band = q < nband;
+        const int2 e = in_band ? band[q] : pairs[q - nband];
+        double r = dot_exact<AHEAD>(z64 + (size_t)e.x * Ts, z64 + (size_t)e.y * Ts, T);
+        if (in_band) {
+            const double d = fabs((double)band_r[q] - r);
+            emax = fmax(emax, d);
+            esum += d;
+        }
+        r = range_rule(r, weighted);
+        if (abs_mode) r = fabs(r);
+        if (in_band) key64[q] = r;
+        else pair_w[q - nband] = (float)r;
     }
     for (int o = 16; o; o >>= 1) {
         emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
@@ -187,13 +345,25 @@ __global__ void k_tie_keys(const int2* __restrict__ band, const unsigned long lo
     }
 }
 
-// Appends band pairs that are edges: key > tau, or key == tau and
-// (i, j) <= tie_cut in lexicographic order.
-__global__ void k_band_emit(const int2* __restrict__ band, const double* __restrict__ key64, long long n,
+// Counters of one build in device memory, cleared at its start and read back
+// with each host round trip.
+struct BuildState {
+    unsigned long long n_pairs;   // pairs decided by the Gram tiles
+    unsigned long long n_band;    // pairs of the FP64 band
+    unsigned long long n_added;   // band pairs that are edges (listed behind the decided ones)
+    unsigned long long err_max;   // band error of the tiles: bits of the maximum, sum
+    double err_sum;
+    int zero;                     // zero-variance voxels
+    int timeout;                  // a Gram pipeline wait ran out
+};
+
+// Lists the band pairs that are edges behind the decided ones: key > tau, or
+// key == tau and (i, j) <= tie_cut in lexicographic order.
+__global__ void k_band_emit(const int2* __restrict__ band, const double* __restrict__ key64, long long cap_band,
                             double tau, int strict_only, unsigned long long tie_cut, int N, int weighted,
-                            int2* __restrict__ pairs, float* __restrict__ w, unsigned long long* __restrict__ npairs,
-                            long long cap)
+                            int2* __restrict__ pairs, float* __restrict__ w, BuildState* __restrict__ st, long long cap)
 {
+    const long long n = min((long long)st->n_band, cap_band), first = (long long)st->n_pairs;
     for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += (long long)gridDim.x * blockDim.x) {
         long long q = base + threadIdx.x;
         bool in = false;
@@ -206,29 +376,16 @@ __global__ void k_band_emit(const int2* __restrict__ band, const double* __restr
             else if (!strict_only && k == tau)
                 in = ((unsigned long long)e.x * (unsigned long long)N + (unsigned long long)e.y) <= tie_cut;
         }
-        long long s = warp_append(npairs, in);
-        if (s >= 0 && s < cap) {
-            pairs[s] = e;
-            if (weighted) w[s] = (float)k;
+        long long s = warp_append(&st->n_added, in);
+        if (s >= 0 && first + s < cap) {
+            pairs[first + s] = e;
+            if (weighted) w[first + s] = (float)k;
         }
     }
 }
 
-// Exact weights for every stored entry: V = key(r64) of (row, col).
-__global__ void k_exact_weights(const int32_t* __restrict__ R, const int32_t* __restrict__ C, int n,
-                                const double* __restrict__ z64, int T, int abs_mode, float* __restrict__ V)
-{
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i = warp; i < n; i += nw)
-        for (int32_t q = R[i] + lane; q < R[i + 1]; q += 32) {
-            double r = exact_r(z64, T, i, C[q], 1);
-            V[q] = (float)(abs_mode ? fabs(r) : r);
-        }
-}
-
 // ---------------------------------------------------------- packed r
-__global__ void k_packed_r(const double* __restrict__ z64, int N, int T, int weighted, long long row0,
+__global__ void k_packed_r(const double* __restrict__ z64, int N, int T, int Ts, int weighted, long long row0,
                            long long rows, float* __restrict__ out)
 {
     // one warp per row i, lanes over j > i; output offset of row i in the
@@ -240,18 +397,24 @@ __global__ void k_packed_r(const double* __restrict__ z64, int N, int T, int wei
         long long i = row0 + ii;
         long long off = i * N - i * (i + 1) / 2 - base0;
         for (long long j = i + 1 + lane; j < N; j += 32)
-            out[off + (j - i - 1)] = (float)exact_r(z64, T, (int)i, (int)j, weighted);
+            out[off + (j - i - 1)] = (float)range_rule(dot_exact<false>(z64 + (size_t)i * Ts, z64 + (size_t)j * Ts, T), weighted);
     }
 }
 
 // ------------------------------------------------------------- driver
-static pg_status prepare_operands(pg_ctx* ctx, const float* bold, int N, int T, bool on_device, ZOperands& z,
-                                  int* nzero_host)
+// Operands of one subject on the context stream (nothing is waited for).
+// zero_dev counts the zero-variance voxels; the caller has cleared it.
+enum : int { OPS_EXACT = 0, OPS_FP32 = 1, OPS_BF16 = 2 };   // z64 alone, with z32, with zhi and zlo
+static pg_status prepare_operands(pg_ctx* ctx, const float* bold, int N, int T, bool on_device, int ops, ZOperands& z,
+                                  int* zero_dev)
 {
     z.N = N;
     z.T = T;
+    z.Ts = (T + 3) / 4 * 4;
     z.Np = (N + 127) / 128 * 128;
     z.Tp = (T + 63) / 64 * 64;
+    z.z32 = nullptr;
+    z.zhi = z.zlo = nullptr;
     const float* dbold = bold;
     if (!on_device) {
         float* tmp;
@@ -260,28 +423,26 @@ static pg_status prepare_operands(pg_ctx* ctx, const float* bold, int N, int T, 
         dbold = tmp;
     }
     double *mu, *sd;
-    int* nz;
     PG_TRY(pg_wst(ctx, "z.mu", (size_t)N, &mu));
     PG_TRY(pg_wst(ctx, "z.sd", (size_t)N, &sd));
-    PG_TRY(pg_wst(ctx, "z.nzero", 1, &nz));
-    PG_TRY(pg_wst(ctx, "z.z64", (size_t)N * T, &z.z64));
-    PG_TRY(pg_wst(ctx, "z.z32", (size_t)z.Np * z.Tp, &z.z32));
-    PG_TRY(pg_wst(ctx, "z.zhi", (size_t)z.Np * z.Tp, &z.zhi));
-    PG_TRY(pg_wst(ctx, "z.zlo", (size_t)z.Np * z.Tp, &z.zlo));
-    PG_CUDA(ctx, cudaMemsetAsync(nz, 0, sizeof(int), ctx->stream));
-    k_zstats<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(dbold, N, T, mu, sd, nz);
+    PG_TRY(pg_wst(ctx, "z.z64", (size_t)N * z.Ts, &z.z64));
+    if (ops == OPS_FP32) PG_TRY(pg_wst(ctx, "z.z32", (size_t)z.Np * z.Tp, &z.z32));
+    if (ops == OPS_BF16) {
+        PG_TRY(pg_wst(ctx, "z.zhi", (size_t)z.Np * z.Tp, &z.zhi));
+        PG_TRY(pg_wst(ctx, "z.zlo", (size_t)z.Np * z.Tp, &z.zlo));
+    }
+    k_zstats<<<ceil_div(N, 32), 32 * (1 + ZPROD), 0, ctx->stream>>>(dbold, N, T, mu, sd, zero_dev);
     PG_LAUNCHED(ctx);
     dim3 g(ceil_div(z.Tp, 32), ceil_div(z.Np, 32));
-    k_zwrite<<<g, dim3(32, 8), 0, ctx->stream>>>(dbold, N, T, z.Tp, mu, sd, z.z64, z.z32, z.zhi, z.zlo);
+    k_zwrite<<<g, dim3(32, 8), 0, ctx->stream>>>(dbold, N, T, z.Ts, z.Tp, mu, sd, z.z64, z.z32, z.zhi, z.zlo);
     PG_LAUNCHED(ctx);
-    if (nzero_host) PG_TRY(pg_d2h(ctx, nzero_host, nz, sizeof(int)));
     return PG_OK;
 }
 
 pg_status pg_zstats(pg_ctx* ctx, const float* dbold, int N, int T, double* mu, double* sd, int* nz)
 {
     PG_CUDA(ctx, cudaMemsetAsync(nz, 0, sizeof(int), ctx->stream));
-    k_zstats<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(dbold, N, T, mu, sd, nz);
+    k_zstats<<<ceil_div(N, 32), 32 * (1 + ZPROD), 0, ctx->stream>>>(dbold, N, T, mu, sd, nz);
     PG_LAUNCHED(ctx);
     return PG_OK;
 }
@@ -300,13 +461,19 @@ extern "C" void pg_build_opts_default(pg_build_opts* o)
     o->exact_weights = 1;
 }
 
-static pg_status run_gram(pg_ctx* ctx, const ZOperands& z, int precision, int mode, const EpiParams& p)
+static pg_status run_gram(pg_ctx* ctx, const ZOperands& z, int precision, int mode, const EpiParams& p, int* err_dev)
 {
-    if (precision == PG_SPLIT_BF16 && gram_tc_supported(ctx, z)) return launch_gram_tc(ctx, z, mode, p);
+    if (precision == PG_SPLIT_BF16 && gram_tc_supported(ctx, z)) return launch_gram_tc(ctx, z, mode, p, err_dev);
     if (precision == PG_SPLIT_BF16)
         return pg_fail(ctx, PG_ERR_INVALID, "split-BF16 Gram unavailable for N=%d T=%d", z.N, z.T);
     return launch_gram_simt(ctx, z, mode, p);
 }
+
+// r mode: up to this many pairs the lists are simply sized for all of them
+// (28 bytes each, 120 MB); above, a histogram pass of the Gram sizes them.
+// At 2,896 nodes that pass and its host round trip cost 60 us of a 300 us
+// build; at 58,000 nodes lists for every pair would take 47 GB.
+constexpr long long LIST_ALL_PAIRS = 1LL << 22;
 
 extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, int32_t T,
                                     const pg_build_opts* opts_in, pg_graph** out, pg_build_info* info)
@@ -326,10 +493,25 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     cudaEvent_t* ev = ctx->ev;
     PG_CUDA(ctx, cudaEventRecord(ev[0], ctx->stream));
 
+    BuildState *ds, *hs;
+    unsigned char *hist_dev, *hist_host;   // the two "below" counters, then the bins
+    constexpr size_t HIST_BYTES = 2 * sizeof(unsigned long long) + HIST_BINS * sizeof(unsigned int);
+    PG_TRY(pg_wst(ctx, "b.state", 1, &ds));
+    PG_TRY(pg_hwst(ctx, "b.state", 1, &hs));
+    PG_TRY(pg_wst(ctx, "b.hist", HIST_BYTES, &hist_dev));
+    PG_TRY(pg_hwst(ctx, "b.hist", HIST_BYTES, &hist_host));
+    PG_CUDA(ctx, cudaMemsetAsync(ds, 0, sizeof *ds, ctx->stream));
+    // reads the counters (and waits for everything before them)
+    auto read_state = [&]() -> pg_status {
+        PG_CUDA(ctx, cudaMemcpyAsync(hs, ds, sizeof *ds, cudaMemcpyDeviceToHost, ctx->stream));
+        PG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (hs->timeout) return pg_fail(ctx, PG_ERR_TIMEOUT, "tcgen05 Gram: a pipeline wait timed out");
+        return PG_OK;
+    };
+
     ZOperands z;
-    int nzero = 0;
-    PG_TRY(prepare_operands(ctx, bold, N, T, o.input_on_device != 0, z, &nzero));
-    inf.zero_variance = nzero;
+    PG_TRY(prepare_operands(ctx, bold, N, T, o.input_on_device != 0, o.precision == PG_SPLIT_BF16 ? OPS_BF16 : OPS_FP32,
+                            z, &ds->zero));
     PG_CUDA(ctx, cudaEventRecord(ev[1], ctx->stream));
 
     // ---- histogram pass(es): only keys >= kmin are binned, the rest counted
@@ -337,29 +519,26 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     memset(&p, 0, sizeof p);
     p.N = N;
     p.abs_mode = o.sign == PG_ABS;
-    p.weighted = o.weighted != 0;
+    const int weighted = o.weighted != 0;
+    const bool exact_w = weighted && o.exact_weights;   // else the tile's r is the weight
+    p.weighted = weighted && !exact_w;
     p.tile_stride = 1;
     const double g = o.guard;
     const float key_lo = p.abs_mode ? 0.0f : -1.0f;
     const float edge_band = (float)(1.0 - g);
     p.edge_band = (g == 0.0 && o.mode == PG_THRESH_R) ? INFINITY : edge_band;
-    unsigned int* hist;
-    unsigned long long* below;
-    PG_TRY(pg_wst(ctx, "b.hist", HIST_BINS, &hist));
-    PG_TRY(pg_wst(ctx, "b.below", 4, &below));
-    p.hist = hist;
-    p.below = below;
-    std::vector<unsigned int> h(HIST_BINS);
-    unsigned long long hbelow[2] = {0, 0};
+    p.below = (unsigned long long*)hist_dev;
+    p.hist = (unsigned int*)(hist_dev + 2 * sizeof(unsigned long long));
+    const unsigned long long* hbelow = (const unsigned long long*)hist_host;
+    const unsigned int* h = (const unsigned int*)(hist_host + 2 * sizeof(unsigned long long));
     auto hist_pass = [&](float kmin, int stride) -> pg_status {
         p.kmin = kmin;
         p.scale = (float)HIST_BINS / (1.0f - kmin);
         p.tile_stride = stride;
-        PG_CUDA(ctx, cudaMemsetAsync(hist, 0, sizeof(unsigned int) * HIST_BINS, ctx->stream));
-        PG_CUDA(ctx, cudaMemsetAsync(below, 0, 2 * sizeof(unsigned long long), ctx->stream));
-        if (M1 > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_HIST, p));
-        PG_TRY(pg_d2h(ctx, h.data(), hist, sizeof(unsigned int) * HIST_BINS));
-        PG_TRY(pg_d2h(ctx, hbelow, below, 2 * sizeof(unsigned long long)));
+        PG_CUDA(ctx, cudaMemsetAsync(hist_dev, 0, HIST_BYTES, ctx->stream));
+        if (M1 > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_HIST, p, &ds->timeout));
+        PG_CUDA(ctx, cudaMemcpyAsync(hist_host, hist_dev, HIST_BYTES, cudaMemcpyDeviceToHost, ctx->stream));
+        PG_TRY(read_state());
         p.tile_stride = 1;
         return PG_OK;
     };
@@ -374,6 +553,7 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         for (int b = 0; b < HIST_BINS; b++) s += h[b];
         return s;
     };
+    const bool list_all = o.mode == PG_THRESH_R && M1 <= LIST_ALL_PAIRS;
     long long k_edges = -1;  // sparsity: wanted edges
     float lo_cut, hi_cut;
     if (o.mode == PG_THRESH_SPARSITY) {
@@ -417,16 +597,21 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         lo_cut = (float)(o.value - g);
         hi_cut = (float)(o.value + g);
         if (g == 0.0) lo_cut = hi_cut = nextafterf((float)o.value, INFINITY);  // tile decides alone: key > value
-        PG_TRY(hist_pass(std::max(key_lo, std::min(lo_cut, edge_band) - 1e-3f), 1));
+        if (!list_all) PG_TRY(hist_pass(std::max(key_lo, std::min(lo_cut, edge_band) - 1e-3f), 1));
     }
     PG_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
-    if (hist_total() + (long long)hbelow[0] != M1)
+    if (!list_all && hist_total() + (long long)hbelow[0] != M1)
         return pg_fail(ctx, PG_ERR_INTERNAL, "histogram holds %lld pairs, expected %lld",
                        hist_total() + (long long)hbelow[0], M1);
     if (lo_cut < key_lo) lo_cut = key_lo;
-    // capacities from the histogram (upper bounds: the bin mapping is monotone)
-    long long cap_pairs = 0, cap_band = 0;
-    {
+    // capacities: every pair, or from the histogram (upper bounds: the bin
+    // mapping is monotone)
+    const bool no_band = g == 0.0 && o.mode == PG_THRESH_R;
+    long long cap_pairs = 0, cap_band = 0, cap_total;
+    if (list_all) {
+        cap_pairs = cap_total = M1;
+        cap_band = no_band ? 0 : M1;
+    } else {
         int bh = std::isfinite(hi_cut) ? bin_of(hi_cut) : HIST_BINS;
         int bl = std::isfinite(lo_cut) ? bin_of(lo_cut) : HIST_BINS;
         int be = bin_of(edge_band);
@@ -437,55 +622,58 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         if (lo_cut < p.kmin) cap_band += (long long)hbelow[0];   // band reaches below the binned range
         if (hi_cut < p.kmin) cap_pairs += (long long)hbelow[0];
         cap_band += (long long)hbelow[1];                         // r <= -(1 - guard), signed keys
-        if (g == 0.0 && o.mode == PG_THRESH_R) cap_band = 0;
+        if (no_band) cap_band = 0;
+        cap_total = cap_pairs + cap_band;
     }
     if (cap_pairs > (long long)INT32_MAX) return pg_fail(ctx, PG_ERR_TOO_LARGE, "too many edges");
     // ---- emit pass
     int2 *pairs, *band;
     float* pw = nullptr;
     float* band_r;
-    unsigned long long* counters;
-    const long long cap_total = cap_pairs + cap_band;
+    double* key64;
     PG_TRY(pg_wst(ctx, "b.pairs", (size_t)std::max(1LL, cap_total), &pairs));
-    if (o.weighted) PG_TRY(pg_wst(ctx, "b.pw", (size_t)std::max(1LL, cap_total), &pw));
+    if (weighted) PG_TRY(pg_wst(ctx, "b.pw", (size_t)std::max(1LL, cap_total), &pw));
     PG_TRY(pg_wst(ctx, "b.band", (size_t)std::max(1LL, cap_band), &band));
     PG_TRY(pg_wst(ctx, "b.band_r", (size_t)std::max(1LL, cap_band), &band_r));
-    PG_TRY(pg_wst(ctx, "b.counters", 4, &counters));
-    PG_CUDA(ctx, cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), ctx->stream));
+    PG_TRY(pg_wst(ctx, "b.key64", (size_t)std::max(1LL, cap_band), &key64));
     p.lo_cut = lo_cut;
     p.hi_cut = hi_cut;
     p.pairs = pairs;
     p.pair_w = pw;
-    p.n_pairs = counters;
+    p.n_pairs = &ds->n_pairs;
     p.cap_pairs = cap_pairs;
     p.band = band;
     p.band_r = band_r;
-    p.n_band = counters + 1;
+    p.n_band = &ds->n_band;
     p.cap_band = cap_band;
-    if (M1 > 0 && cap_total > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p));
-    unsigned long long cnt[2];
-    PG_TRY(pg_d2h(ctx, cnt, counters, 2 * sizeof(unsigned long long)));
+    if (M1 > 0 && cap_total > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p, &ds->timeout));
     PG_CUDA(ctx, cudaEventRecord(ev[3], ctx->stream));
-    if ((long long)cnt[0] > cap_pairs || (long long)cnt[1] > cap_band)
-        return pg_fail(ctx, PG_ERR_INTERNAL, "emit overflow: %llu/%lld decided, %llu/%lld band", cnt[0], cap_pairs,
-                       cnt[1], cap_band);
-    const long long n_above = (long long)cnt[0], n_band = (long long)cnt[1];
-    inf.above_pairs = n_above;
-    inf.band_pairs = n_band;
 
-    // ---- FP64 recheck and decision
+    // ---- FP64 recheck (and exact weights of the decided pairs)
     double tau = o.value;
-    double* key64 = nullptr;
-    if (n_band > 0) {
-        PG_TRY(pg_wst(ctx, "b.key64", (size_t)n_band, &key64));
-        int grid = std::max(1, std::min(ctx->sm_count * 16, ceil_div(n_band, 128)));
-        k_recheck<<<grid, 128, 0, ctx->stream>>>(band, band_r, n_band, z.z64, T, p.weighted, p.abs_mode, key64,
-                                                 counters + 2);
+    const long long n_exact = cap_band + (exact_w ? cap_pairs : 0);
+    if (n_exact > 0) {
+        const int grid = (int)std::max(1LL, std::min(ctx->sm_count * 16LL, (n_exact + 127) / 128));
+        // the deeper pipeline where even a list of every pair leaves the SMs
+        // with a few warps each (N = 90 x 1200: 120 -> 47 us); above,
+        // the registers are better spent on more warps
+        auto kern = list_all && n_exact <= 1024LL * ctx->sm_count ? k_pair_exact<true> : k_pair_exact<false>;
+        kern<<<grid, 128, 0, ctx->stream>>>(band, band_r, pairs, exact_w ? pw : nullptr, &ds->n_pairs, cap_pairs, cap_band,
+                                            z.z64, T, z.Ts, weighted, p.abs_mode, key64, &ds->err_max);
         PG_LAUNCHED(ctx);
     }
+    auto check_caps = [&]() -> pg_status {
+        if ((long long)hs->n_pairs > cap_pairs || (long long)hs->n_band > cap_band)
+            return pg_fail(ctx, PG_ERR_INTERNAL, "emit overflow: %llu/%lld decided, %llu/%lld band", hs->n_pairs,
+                           cap_pairs, hs->n_band, cap_band);
+        return PG_OK;
+    };
     int strict_only = 1;
     unsigned long long tie_cut = 0;
     if (o.mode == PG_THRESH_SPARSITY && k_edges > 0) {
+        PG_TRY(read_state());
+        PG_TRY(check_caps());
+        const long long n_above = (long long)hs->n_pairs, n_band = (long long)hs->n_band;
         long long m = k_edges - n_above;  // rank inside the band
         if (m <= 0 || m > n_band)
             return pg_fail(ctx, PG_ERR_INTERNAL, "band does not contain the k-th key (k=%lld above=%lld band=%lld)",
@@ -522,15 +710,20 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     } else if (o.mode == PG_THRESH_SPARSITY) {
         tau = INFINITY;
     }
-    if (n_band > 0) {
-        int grid = std::max(1, std::min(ctx->sm_count * 8, ceil_div(n_band, 256)));
-        k_band_emit<<<grid, 256, 0, ctx->stream>>>(band, key64, n_band, tau, strict_only, tie_cut, N, p.weighted,
-                                                   pairs, pw, counters, cap_total);
+    if (cap_band > 0) {
+        const int grid = (int)std::max(1LL, std::min(ctx->sm_count * 8LL, (cap_band + 255) / 256));
+        k_band_emit<<<grid, 256, 0, ctx->stream>>>(band, key64, cap_band, tau, strict_only, tie_cut, N, weighted, pairs, pw,
+                                                   ds, cap_total);
         PG_LAUNCHED(ctx);
     }
-    PG_TRY(pg_d2h(ctx, cnt, counters, sizeof(unsigned long long)));
+    PG_TRY(read_state());
+    PG_TRY(check_caps());
     PG_CUDA(ctx, cudaEventRecord(ev[4], ctx->stream));
-    const long long n_edges = (long long)cnt[0];
+    const long long n_band = (long long)hs->n_band;
+    const long long n_edges = (long long)(hs->n_pairs + hs->n_added);
+    inf.above_pairs = (long long)hs->n_pairs;
+    inf.band_pairs = n_band;
+    inf.zero_variance = hs->zero;
     if (n_edges > cap_total) return pg_fail(ctx, PG_ERR_INTERNAL, "edge list overflow");
     if (k_edges >= 0 && k_edges > 0 && n_edges != k_edges)
         return pg_fail(ctx, PG_ERR_INTERNAL, "sparsity graph has %lld edges, expected %lld", n_edges, k_edges);
@@ -538,10 +731,6 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     // ---- CSR
     pg_graph* gph;
     PG_TRY(pg_csr_from_pairs(ctx, N, pairs, pw, n_edges, &gph));
-    if (o.weighted && o.exact_weights && n_edges > 0) {
-        k_exact_weights<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(gph->R, gph->C, N, z.z64, T, p.abs_mode, gph->V);
-        ctx->launches++;
-    }
     cudaError_t e = cudaEventRecord(ev[5], ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
@@ -555,13 +744,8 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     cudaEventElapsedTime(&ms, ev[3], ev[4]); inf.ms_select = ms;
     cudaEventElapsedTime(&ms, ev[4], ev[5]); inf.ms_csr = ms;
     if (n_band > 0) {
-        unsigned long long err[2];
-        PG_TRY(pg_d2h(ctx, err, counters + 2, sizeof err));
-        double emax, esum;
-        memcpy(&emax, &err[0], 8);
-        memcpy(&esum, &err[1], 8);
-        inf.band_err_max = emax;
-        inf.band_err_mean = esum / (double)n_band;
+        memcpy(&inf.band_err_max, &hs->err_max, 8);
+        inf.band_err_mean = hs->err_sum / (double)n_band;
     }
     inf.tau = tau;
     inf.edges = n_edges;
@@ -578,7 +762,10 @@ extern "C" pg_status pg_correlation_packed(pg_ctx* ctx, const float* bold, int32
         return pg_fail(ctx, PG_ERR_INVALID, "pg_correlation_packed: bad arguments");
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     ZOperands z;
-    PG_TRY(prepare_operands(ctx, bold, N, T, input_on_device != 0, z, nullptr));
+    int* nz;
+    PG_TRY(pg_wst(ctx, "z.nzero", 1, &nz));
+    PG_CUDA(ctx, cudaMemsetAsync(nz, 0, sizeof(int), ctx->stream));
+    PG_TRY(prepare_operands(ctx, bold, N, T, input_on_device != 0, OPS_EXACT, z, nz));
     const long long M1 = (long long)N * (N - 1) / 2;
     // rows in chunks of at most ~256 MB of output
     long long row = 0;
@@ -592,7 +779,7 @@ extern "C" pg_status pg_correlation_packed(pg_ctx* ctx, const float* bold, int32
             r1++;
         }
         long long off = row * N - row * (row + 1) / 2;
-        k_packed_r<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(z.z64, N, T, weighted, row, r1 - row, buf);
+        k_packed_r<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(z.z64, N, T, z.Ts, weighted, row, r1 - row, buf);
         PG_LAUNCHED(ctx);
         PG_TRY(pg_d2h(ctx, r_packed + off, buf, sizeof(float) * (size_t)elems));
         row = r1;

@@ -6,13 +6,14 @@
 
 // Operands, all row-major with one row per voxel (the K = time dimension
 // contiguous, i.e. "K-major" for both GEMM operands of Z * Z^T):
-//   z64 : N  x T  double  -- exact z-scores for the FP64 recheck
+//   z64 : N  x Ts double  -- exact z-scores for the FP64 recheck (T used, Ts a multiple of 4)
 //   z32 : Np x Tp float   -- rounded z-scores for the FP32 SIMT Gram
 //   zhi : Np x Tp bf16    -- bf16(z32)
 //   zlo : Np x Tp bf16    -- bf16(z32 - zhi)
-// Np = N rounded up to the 128-row tile, Tp = T rounded up to 64; padding is 0.
+// Np = N rounded up to the 128-row tile, Tp = T rounded up to 64; padding of the
+// Gram operands is 0.  A build writes z64 and its own Gram's operands only.
 struct ZOperands {
-    int N, T, Np, Tp;
+    int N, T, Ts, Np, Tp;
     double* z64;
     float* z32;
     __nv_bfloat16* zhi;
@@ -154,8 +155,10 @@ __device__ __forceinline__ void tri_tile(long long L, int nb, int& bi, int& bj)
 }
 
 // Kernel launchers (defined in gram_simt.cu / gram_tc.cu).
+// launch_gram_tc leaves a timed-out pipeline wait in *err_dev (cleared by the
+// caller, read with the pass's counters); nothing is waited for.
 pg_status launch_gram_simt(pg_ctx* ctx, const ZOperands& z, int mode, const EpiParams& p);
-pg_status launch_gram_tc(pg_ctx* ctx, const ZOperands& z, int mode, const EpiParams& p);
+pg_status launch_gram_tc(pg_ctx* ctx, const ZOperands& z, int mode, const EpiParams& p, int* err_dev);
 bool gram_tc_supported(pg_ctx* ctx, const ZOperands& z);
 
 // Radix selection state (device): the m-th largest of n uint64 keys is found

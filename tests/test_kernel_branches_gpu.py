@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
+from pagani import synth
 from tests import graphs as G
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,21 @@ def test_onnela_rows_out_of_order(ctx):
     C2[9:12], V2[9:12] = [1, 0, 2], [.9, .7, 1.]      # node 3's row, swapped
     got, _, _ = ctx.clustering(ctx.graph(R, C2, V2), kind="onnela")
     np.testing.assert_allclose(got[:3], want[:3], rtol=2.0 ** -22)
+
+
+# ------------------------------------------------------ network construction
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+@pytest.mark.parametrize("N,T", [(2, 1), (33, 3), (90, 4), (65, 15), (130, 16), (257, 63), (300, 65), (140, 1201),
+                                 (2896, 67), (2897, 66)])
+def test_weighted_build_sizes(ctx, N, T, precision):
+    """Lengths around the 4- and 16-sample steps of the FP64 recheck and the
+    64-sample chunks of the z-scores; both sides of the list-everything rule
+    (2,896 nodes).  Edge set and weights equal the FP64 oracle's."""
+    bold = synth.bold_series(N, T, 4, 100 + N + T)
+    for sign in ("signed", "abs"):
+        g, info = ctx.build_graph(bold, mode="r", value=0.3, sign=sign, weighted=True, precision=precision)
+        R, C, V = g.to_csr()
+        z, _ = O.zscore(bold)
+        Ro, Co, Vo = O.graph_r(O.corr_packed(z, weighted=True), N, 0.3, abs_mode=sign == "abs", weighted=True)
+        assert np.array_equal(R, Ro) and np.array_equal(C, Co) and np.array_equal(V, Vo)
+        assert info["edges"] == len(C) // 2
