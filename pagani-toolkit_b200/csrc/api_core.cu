@@ -488,6 +488,18 @@ __global__ void __launch_bounds__(SCAN_B) k_row_offsets(int32_t* __restrict__ cn
     }
 }
 
+pg_status pg_row_offsets(pg_ctx* ctx, int32_t* cnt, int32_t n, int32_t* R)
+{
+    const int nb = ceil_div(std::max(n, 1), SCAN_B);
+    long long* bsum;
+    PG_TRY(pg_wst(ctx, "csr.bsum", (size_t)nb, &bsum));
+    k_row_sums<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum);
+    PG_LAUNCHED(ctx);
+    k_row_offsets<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum, R);
+    PG_LAUNCHED(ctx);
+    return PG_OK;
+}
+
 __global__ void k_pair_scatter(const int2* __restrict__ pairs, const float* __restrict__ w, long long np,
                                int32_t* __restrict__ cursor, int32_t* __restrict__ C, float* __restrict__ V)
 {
@@ -623,11 +635,8 @@ pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const flo
 {
     if (2 * npairs > INT32_MAX)
         return pg_fail(ctx, PG_ERR_TOO_LARGE, "%lld directed entries exceed the int32 CSR", 2LL * npairs);
-    const int nb = ceil_div(std::max(n, 1), SCAN_B);
     int32_t* cnt;
-    long long* bsum;
     PG_TRY(pg_wst(ctx, "csr.cnt", (size_t)n + 1, &cnt));
-    PG_TRY(pg_wst(ctx, "csr.bsum", (size_t)nb, &bsum));
     PG_CUDA(ctx, cudaMemsetAsync(cnt, 0, sizeof(int32_t) * ((size_t)n + 1), ctx->stream));
     int grid = ctx->sm_count * 8;
     if (npairs > 0) {
@@ -636,10 +645,7 @@ pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const flo
     }
     pg_graph* g;
     PG_TRY(pg_graph_alloc(ctx, n, 2 * npairs, w != nullptr, &g));
-    k_row_sums<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum);
-    ctx->launches++;
-    k_row_offsets<<<nb, SCAN_B, 0, ctx->stream>>>(cnt, n, bsum, g->R);
-    ctx->launches++;
+    if (pg_status st = pg_row_offsets(ctx, cnt, n, g->R); st != PG_OK) { pg_graph_free(g); return st; }
     int32_t* cursor = cnt;  // the counts became the offsets
     if (npairs > 0) {
         int32_t* Ct;

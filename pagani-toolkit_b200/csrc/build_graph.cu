@@ -357,13 +357,16 @@ struct BuildState {
     int timeout;                  // a Gram pipeline wait ran out
 };
 
-// Lists the band pairs that are edges behind the decided ones: key > tau, or
-// key == tau and (i, j) <= tie_cut in lexicographic order.
+// Adds the band pairs that are edges to the adjacency bits, or lists them
+// behind the decided ones: key > tau, or key == tau and (i, j) <= tie_cut in
+// lexicographic order.
 __global__ void k_band_emit(const int2* __restrict__ band, const double* __restrict__ key64, long long cap_band,
                             double tau, int strict_only, unsigned long long tie_cut, int N, int weighted,
-                            int2* __restrict__ pairs, float* __restrict__ w, BuildState* __restrict__ st, long long cap)
+                            uint32_t* __restrict__ bits, int bit_words, int2* __restrict__ pairs,
+                            float* __restrict__ w, BuildState* __restrict__ st, long long cap)
 {
     const long long n = min((long long)st->n_band, cap_band), first = (long long)st->n_pairs;
+    int added = 0;
     for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += (long long)gridDim.x * blockDim.x) {
         long long q = base + threadIdx.x;
         bool in = false;
@@ -376,12 +379,103 @@ __global__ void k_band_emit(const int2* __restrict__ band, const double* __restr
             else if (!strict_only && k == tau)
                 in = ((unsigned long long)e.x * (unsigned long long)N + (unsigned long long)e.y) <= tie_cut;
         }
+        if (bits) {
+            if (in) {
+                atomicOr(&bits[(size_t)e.x * bit_words + (e.y >> 5)], 1u << (e.y & 31));
+                atomicOr(&bits[(size_t)e.y * bit_words + (e.x >> 5)], 1u << (e.x & 31));
+                added++;
+            }
+            continue;
+        }
         long long s = warp_append(&st->n_added, in);
         if (s >= 0 && first + s < cap) {
             pairs[first + s] = e;
             if (weighted) w[first + s] = (float)k;
         }
     }
+    added = __reduce_add_sync(0xffffffffu, added);
+    if ((threadIdx.x & 31) == 0 && added) atomicAdd(&st->n_added, (unsigned long long)added);
+}
+
+// ------------------------------------------- adjacency bits -> CSR
+// Rows of the bit matrix in column order are the sorted CSR rows: one pass
+// counts them (a warp per row, 16 bytes per lane), one writes the columns.
+// Bound by the two reads of the bits: 58,000 nodes / 33.6M entries 340 us for
+// both, against 1.05 ms for degrees, scatter and row sort of a pair list.
+__global__ void __launch_bounds__(256)
+k_bits_count(const uint32_t* __restrict__ bits, int words, int n, int32_t* __restrict__ cnt)
+{
+    const int lane = threadIdx.x & 31, quads = words >> 2;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = gw; i < n; i += nw) {
+        const uint4* row = (const uint4*)(bits + (size_t)i * words);
+        int c = 0;
+#pragma unroll 4
+        for (int q = lane; q < quads; q += 32) {
+            const uint4 m = row[q];
+            c += __popc(m.x) + __popc(m.y) + __popc(m.z) + __popc(m.w);
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) cnt[i] = c;
+    }
+}
+
+__global__ void __launch_bounds__(256)
+k_bits_csr(const uint32_t* __restrict__ bits, int words, int n, const int32_t* __restrict__ R, int32_t* __restrict__ C,
+           long long nnz)
+{
+    const int lane = threadIdx.x & 31, quads = words >> 2;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int i = gw; i < n; i += nw) {
+        const uint4* row = (const uint4*)(bits + (size_t)i * words);
+        long long base = R[i];
+        for (int q0 = 0; q0 < quads; q0 += 128) {
+            uint4 v[4];   // four reads in flight
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                const int q = q0 + 32 * z + lane;
+                v[z] = q < quads ? row[q] : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                const unsigned long long m[2] = {v[z].x | ((unsigned long long)v[z].y << 32),
+                                                 v[z].z | ((unsigned long long)v[z].w << 32)};
+                const int c = __popcll(m[0]) + __popcll(m[1]);
+                int x = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                long long at = base + x - c;
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    for (unsigned long long b = m[k]; b; b &= b - 1ULL, at++)
+                        if (at < nnz) C[at] = ((q0 + 32 * z + lane) << 7) + (k << 6) + __ffsll((long long)b) - 1;
+                base += __shfl_sync(0xffffffffu, x, 31);
+            }
+        }
+    }
+}
+
+static pg_status csr_from_bits(pg_ctx* ctx, int n, const uint32_t* bits, int words, long long n_edges, pg_graph** out)
+{
+    int32_t* cnt;
+    PG_TRY(pg_wst(ctx, "csr.cnt", (size_t)n + 1, &cnt));
+    const int grid = std::min(ctx->sm_count * 8, ceil_div(n, 8));
+    k_bits_count<<<grid, 256, 0, ctx->stream>>>(bits, words, n, cnt);
+    PG_LAUNCHED(ctx);
+    pg_graph* g;
+    PG_TRY(pg_graph_alloc(ctx, n, 2 * n_edges, false, &g));
+    if (pg_status st = pg_row_offsets(ctx, cnt, n, g->R); st != PG_OK) {
+        pg_graph_free(g);
+        return st;
+    }
+    if (n_edges > 0) {
+        k_bits_csr<<<grid, 256, 0, ctx->stream>>>(bits, words, n, g->R, g->C, g->nnz);
+        ctx->launches++;
+    }
+    *out = g;
+    return PG_OK;
 }
 
 // ---------------------------------------------------------- packed r
@@ -626,18 +720,36 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         cap_total = cap_pairs + cap_band;
     }
     if (cap_pairs > (long long)INT32_MAX) return pg_fail(ctx, PG_ERR_TOO_LARGE, "too many edges");
+    // Decided edges of a binary graph go into adjacency bits where about four
+    // passes over N^2 bits (0.45 ms at 58,000 nodes) beat the list's degree
+    // count, scatter and sort (62 us per million edges): from 1.3e-3 N^2 edges
+    // on, and always where every pair would be listed (at most 1 MB of bits).
+    // Weights need the list; the bits may take 8 GiB.
+    const int bit_words = z.Np / 32;
+    const size_t bit_bytes = (size_t)N * bit_words * sizeof(uint32_t);
+    const long long expect = k_edges >= 0 ? k_edges : cap_pairs;
+    const bool use_bits = !weighted && bit_bytes <= (8ULL << 30) &&
+                          (list_all || (double)expect >= 1.3e-3 * (double)N * (double)N);
     // ---- emit pass
-    int2 *pairs, *band;
+    int2 *pairs = nullptr, *band;
     float* pw = nullptr;
     float* band_r;
     double* key64;
-    PG_TRY(pg_wst(ctx, "b.pairs", (size_t)std::max(1LL, cap_total), &pairs));
+    uint32_t* bits = nullptr;
+    if (use_bits) {
+        PG_TRY(pg_wst(ctx, "b.bits", (size_t)N * bit_words, &bits));
+        PG_CUDA(ctx, cudaMemsetAsync(bits, 0, bit_bytes, ctx->stream));
+    } else {
+        PG_TRY(pg_wst(ctx, "b.pairs", (size_t)std::max(1LL, cap_total), &pairs));
+    }
     if (weighted) PG_TRY(pg_wst(ctx, "b.pw", (size_t)std::max(1LL, cap_total), &pw));
     PG_TRY(pg_wst(ctx, "b.band", (size_t)std::max(1LL, cap_band), &band));
     PG_TRY(pg_wst(ctx, "b.band_r", (size_t)std::max(1LL, cap_band), &band_r));
     PG_TRY(pg_wst(ctx, "b.key64", (size_t)std::max(1LL, cap_band), &key64));
     p.lo_cut = lo_cut;
     p.hi_cut = hi_cut;
+    p.bits = bits;
+    p.bit_words = bit_words;
     p.pairs = pairs;
     p.pair_w = pw;
     p.n_pairs = &ds->n_pairs;
@@ -712,8 +824,8 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     }
     if (cap_band > 0) {
         const int grid = (int)std::max(1LL, std::min(ctx->sm_count * 8LL, (cap_band + 255) / 256));
-        k_band_emit<<<grid, 256, 0, ctx->stream>>>(band, key64, cap_band, tau, strict_only, tie_cut, N, weighted, pairs, pw,
-                                                   ds, cap_total);
+        k_band_emit<<<grid, 256, 0, ctx->stream>>>(band, key64, cap_band, tau, strict_only, tie_cut, N, weighted, bits, bit_words,
+                                                   pairs, pw, ds, cap_total);
         PG_LAUNCHED(ctx);
     }
     PG_TRY(read_state());
@@ -730,7 +842,10 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
 
     // ---- CSR
     pg_graph* gph;
-    PG_TRY(pg_csr_from_pairs(ctx, N, pairs, pw, n_edges, &gph));
+    if (2 * n_edges > INT32_MAX)
+        return pg_fail(ctx, PG_ERR_TOO_LARGE, "%lld directed entries exceed the int32 CSR", 2LL * n_edges);
+    if (use_bits) PG_TRY(csr_from_bits(ctx, N, bits, bit_words, n_edges, &gph));
+    else PG_TRY(pg_csr_from_pairs(ctx, N, pairs, pw, n_edges, &gph));
     cudaError_t e = cudaEventRecord(ev[5], ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {

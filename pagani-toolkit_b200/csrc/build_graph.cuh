@@ -37,6 +37,11 @@ struct EpiParams {
     // EMIT: key >= hi_cut -> decided edge; key >= lo_cut -> FP64 band;
     // |r| >= edge_band -> band (range rule near +-1).
     float lo_cut, hi_cut, edge_band;
+    // decided edges: bits of the symmetric adjacency matrix (cleared before
+    // the pass; row i holds bit_words words, bit j of row i and bit i of row j),
+    // or, with bits null, a list
+    uint32_t* bits;
+    int bit_words;
     int2* pairs;                   // decided edges (i < j)
     float* pair_w;                 // their weights (weighted only)
     unsigned long long* n_pairs;

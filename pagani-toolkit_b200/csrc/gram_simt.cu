@@ -15,6 +15,17 @@ constexpr int BM = 128, BK = 32, PAD = 4, LDS = BM + PAD;
 constexpr int THREADS = 256;
 constexpr size_t SMEM_TILES = (size_t)2 * 2 * BK * LDS * sizeof(float);  // 2 stages x (A,B)
 
+// transpose of an 8 x 8 bit matrix (row x in byte x)
+__device__ __forceinline__ unsigned long long transpose8(unsigned long long m)
+{
+    unsigned long long t = (m ^ (m >> 7)) & 0x00AA00AA00AA00AAULL;
+    m ^= t ^ (t << 7);
+    t = (m ^ (m >> 14)) & 0x0000CCCC0000CCCCULL;
+    m ^= t ^ (t << 14);
+    t = (m ^ (m >> 28)) & 0x00000000F0F0F0F0ULL;
+    return m ^ t ^ (t << 28);
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 2)
 k_gram_simt(const float* __restrict__ Z, int Tp, int nb, EpiParams p)
@@ -30,7 +41,7 @@ k_gram_simt(const float* __restrict__ Z, int Tp, int nb, EpiParams p)
     }
     const long long nt = (long long)nb * (nb + 1) / 2;
     const int nk = Tp / BK;
-    unsigned int below = 0u, neg = 0u;
+    unsigned int below = 0u, neg = 0u, decided = 0u;
     const long long stride = MODE == EPI_HIST ? (long long)p.tile_stride : 1LL;
     for (long long L = blockIdx.x * stride; L < nt; L += (long long)gridDim.x * stride) {
         int bi, bj;
@@ -98,6 +109,7 @@ k_gram_simt(const float* __restrict__ Z, int Tp, int nb, EpiParams p)
                     if (i < j && j < p.N) epi_hist(acc[x][y], p, sh_hist, below, neg);
                 }
         } else {
+            unsigned long long rows = 0ULL;   // bits mode: byte x holds row i0 + x's decided columns
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 unsigned int m1 = 0u, m2 = 0u;
@@ -110,6 +122,11 @@ k_gram_simt(const float* __restrict__ Z, int Tp, int nb, EpiParams p)
                         m1 |= (unsigned)(cls == 1) << (x * 8 + y);
                         m2 |= (unsigned)(cls == 2) << (x * 8 + y);
                     }
+                if (p.bits) {
+                    rows |= (unsigned long long)m1 << (32 * h);
+                    decided += __popc(m1);
+                    m1 = 0u;
+                }
                 epi_emit_masks(m1, m2, p, [&](int q, int& i, int& j, float& r) {
                     int x = q >> 3, y = q & 7;
                     i = i0 + 4 * h + x;
@@ -117,7 +134,26 @@ k_gram_simt(const float* __restrict__ Z, int Tp, int nb, EpiParams p)
                     r = acc[4 * h + x][y];
                 });
             }
+            if (rows) {
+                unsigned char* bytes = (unsigned char*)p.bits;
+                const size_t pitch = (size_t)p.bit_words * 4;
+                unsigned long long cols = transpose8(rows);
+                if (i0 == j0) {
+                    rows |= cols;
+                    cols = 0ULL;
+                }
+#pragma unroll
+                for (int x = 0; x < 8; x++) {
+                    const unsigned char a = (unsigned char)(rows >> (8 * x)), b = (unsigned char)(cols >> (8 * x));
+                    if (a) bytes[(size_t)(i0 + x) * pitch + (j0 >> 3)] = a;
+                    if (b) bytes[(size_t)(j0 + x) * pitch + (i0 >> 3)] = b;
+                }
+            }
         }
+    }
+    if (MODE == EPI_EMIT) {
+        decided = __reduce_add_sync(0xffffffffu, decided);
+        if ((t & 31) == 0 && decided) atomicAdd(p.n_pairs, (unsigned long long)decided);
     }
     if (MODE == EPI_HIST) {
         epi_hist_flush(below, neg, p);

@@ -22,9 +22,12 @@
 //     (rows), the four warps of a lane quarter 32 columns each, with
 //     tcgen05.ld 32x32b.x32, classify every pair (histogram, decided edge,
 //     FP64 band) in registers and hand the accumulator back (16 arrivals),
-//     so the next tile's MMAs run while this tile's epilogue does.  The
-//     epilogue, not the tensor pipe or the TMA stream, bounds a tile (ncu:
-//     fixed-latency waits on top), hence several warps per lane quarter.
+//     so the next tile's MMAs run while this tile's epilogue does.  The emit
+//     pass only tests for candidates there and then handles the columns that
+//     hold one (about ten of 32 at 1 %): branching on each of the 32 register
+//     values and one list atomic per block made the pass take 5.3 ms at
+//     58,000 voxels, 2.8 ms now (2.85 ms when nothing is kept, so the operand
+//     stream -- 26 GB through L2 per pass -- bounds it).
 // Every mbarrier wait is bounded by the global timer and gives up at once
 // when another warp has given up; the kernel then records an error, waits
 // (bounded) for its own MMAs and TMA copies, frees TMEM and returns.
@@ -56,7 +59,70 @@ struct Ctl {
     int abort;
 };
 
-constexpr size_t SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + sizeof(Ctl) + 64;
+// A warp's part of an output list, gathered in shared memory and written out
+// when it is nearly full: one atomic per flush instead of one per 32 x 32
+// block on the list's counter (all atomics on one address are served one
+// after the other), and coalesced stores.
+constexpr int LIST_CAP = 80;   // a column adds at most 32
+struct WarpList {
+    int2* ij;
+    float* r;
+    int count;
+    static constexpr size_t BYTES = LIST_CAP * (sizeof(int2) + sizeof(float));
+    __device__ void init(unsigned char* base, int slot)
+    {
+        ij = (int2*)(base + (size_t)slot * BYTES);
+        r = (float*)(ij + LIST_CAP);
+        count = 0;
+    }
+    // all lanes: append (i, j, v) of the lanes in `who` (this lane: `mine`)
+    __device__ void push(bool mine, unsigned who, int i, int j, float v, unsigned long long* counter, int2* out,
+                         float* out_r, long long cap)
+    {
+        if (mine) {
+            const int at = count + __popc(who & ((1u << (threadIdx.x & 31)) - 1u));
+            ij[at] = make_int2(i, j);
+            r[at] = v;
+        }
+        count += __popc(who);
+        if (count > LIST_CAP - 32) flush(counter, out, out_r, cap);
+    }
+    __device__ void flush(unsigned long long* counter, int2* out, float* out_r, long long cap)
+    {
+        if (!count) return;
+        __syncwarp();
+        const int lane = threadIdx.x & 31;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(counter, (unsigned long long)count);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int e = lane; e < count; e += 32) {
+            const long long at = (long long)base + e;
+            if (at < cap) {
+                out[at] = ij[e];
+                if (out_r) out_r[at] = r[e];
+            }
+        }
+        __syncwarp();
+        count = 0;
+    }
+};
+
+constexpr size_t LIST_BYTES = 2 * EPI_WARPS * WarpList::BYTES;
+static_assert(sizeof(Ctl) % 8 == 0, "the lists behind Ctl hold int2");
+constexpr size_t smem_bytes(int mode)
+{
+    return 1024 /*align slack*/ + STAGES * STAGE_BYTES + sizeof(Ctl) + (mode == EPI_EMIT ? LIST_BYTES : 0);
+}
+static_assert(smem_bytes(EPI_EMIT) <= 227 * 1024 - 64, "shared memory of the emit pass");
+
+// one column of this warp's 32 TMEM lanes
+__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr)
+{
+    uint32_t v;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    return v;
+}
 
 // Instruction descriptor, kind::f16: F32 accumulate, BF16 A and B, both
 // K-major, N = 128, M = 128.
@@ -191,6 +257,13 @@ k_gram_tc(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CU
         const int quarter = warp & 3;
         const int part = (warp - 2) >> 2;               // 0 .. EPI_WARPS / 4 - 1
         constexpr int CHUNKS = (BN / 32) / (EPI_WARPS / 4);
+        WarpList pair_list, band_list;
+        if (MODE == EPI_EMIT) {
+            unsigned char* lists = smem + STAGES * STAGE_BYTES + sizeof(Ctl);
+            pair_list.init(lists, 2 * (warp - 2));
+            band_list.init(lists, 2 * (warp - 2) + 1);
+        }
+        unsigned decided = 0u;
         int tl = 0;
         for (long long L = first; L < nt; L += stride, tl++) {
             int bi, bj;
@@ -215,25 +288,69 @@ k_gram_tc(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CU
                         if (i < j && j < p.N) epi_hist(__uint_as_float(r[c]), p, sh_hist, below, neg);
                     }
                 } else {
-                    unsigned int m1 = 0u, m2 = 0u;
+                    // columns of this lane's row that may be kept: above the
+                    // diagonal, inside the matrix, key at or above the band
+                    const int below_diag = i - j0 + 1, inside = p.N - j0;
+                    unsigned cand = 0u;
+                    if (p.abs_mode) {
+                        const float cut = fminf(p.lo_cut, p.edge_band);
 #pragma unroll
-                    for (int c = 0; c < 32; c++) {
-                        const int j = j0 + c;
-                        const int cls = (i < j && j < p.N) ? epi_class(__uint_as_float(r[c]), p) : 0;
-                        m1 |= (unsigned)(cls == 1) << c;
-                        m2 |= (unsigned)(cls == 2) << c;
+                        for (int c = 0; c < 32; c++) cand |= (unsigned)(fabsf(__uint_as_float(r[c])) >= cut) << c;
+                    } else {
+                        const float cut = fminf(p.lo_cut, p.edge_band);
+#pragma unroll
+                        for (int c = 0; c < 32; c++) {
+                            const float v = __uint_as_float(r[c]);
+                            cand |= (unsigned)(v >= cut || v <= -p.edge_band) << c;
+                        }
                     }
-                    epi_emit_masks(m1, m2, p, [&](int q, int& ii, int& jj, float& v) {
-                        ii = i;
-                        jj = j0 + q;
-                        v = __uint_as_float(r[q]);
-                    });
+                    if (below_diag > 0) cand &= below_diag >= 32 ? 0u : ~0u << below_diag;
+                    if (inside < 32) cand &= inside <= 0 ? 0u : (1u << inside) - 1u;
+                    // column by column: a column's value is read once more from
+                    // TMEM (registers cannot be indexed), its decided rows are
+                    // one ballot
+                    unsigned todo = __reduce_or_sync(0xffffffffu, cand), m1 = 0u, mt = 0u;
+                    while (todo) {
+                        const int q = __ffs(todo) - 1;
+                        todo &= todo - 1u;
+                        const float v = __uint_as_float(tmem_ld1(src + (uint32_t)(cb * 32 + q)));
+                        const int cls = ((cand >> q) & 1u) ? epi_class(v, p) : 0;
+                        const unsigned b1 = __ballot_sync(0xffffffffu, cls == 1), b2 = __ballot_sync(0xffffffffu, cls == 2);
+                        if (b1) {
+                            if (p.bits) {
+                                m1 |= (unsigned)(cls == 1) << q;
+                                if (lane == q) mt = b1;
+                            } else {
+                                pair_list.push(cls == 1, b1, i, j0 + q, epi_key(v, p.abs_mode), p.n_pairs, p.pairs,
+                                               p.weighted ? p.pair_w : nullptr, p.cap_pairs);
+                            }
+                        }
+                        if (b2) band_list.push(cls == 2, b2, i, j0 + q, v, p.n_band, p.band, p.band_r, p.cap_band);
+                    }
+                    if (p.bits) {
+                        // row i, columns j0..; row j0 + lane, columns of this
+                        // warp's rows: one word each (the same one on the diagonal)
+                        decided += __popc(m1);
+                        const int i0 = i - lane;
+                        if (i0 == j0) {
+                            m1 |= mt;
+                            mt = 0u;
+                        }
+                        if (m1) p.bits[(size_t)i * p.bit_words + (j0 >> 5)] = m1;
+                        if (mt) p.bits[(size_t)(j0 + lane) * p.bit_words + (i0 >> 5)] = mt;
+                    }
                 }
             }
             // the accumulator may be overwritten once every epilogue warp has read it
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl->tempty[buf]);
+        }
+        if (MODE == EPI_EMIT) {
+            pair_list.flush(p.n_pairs, p.pairs, p.weighted ? p.pair_w : nullptr, p.cap_pairs);
+            band_list.flush(p.n_band, p.band, p.band_r, p.cap_band);
+            decided = __reduce_add_sync(0xffffffffu, decided);
+            if (lane == 0 && decided) atomicAdd(p.n_pairs, (unsigned long long)decided);
         }
     }
     // the MMA thread waits (bounded) until its own MMAs have completed: TMEM
@@ -294,12 +411,12 @@ pg_status launch_gram_tc(pg_ctx* ctx, const ZOperands& z, int mode, const EpiPar
     ctx->debug_gram_stall_ns = 0;
     if (mode == EPI_HIST) {
         PG_CUDA(ctx, cudaFuncSetAttribute(k_gram_tc<EPI_HIST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)SMEM_BYTES));
-        k_gram_tc<EPI_HIST><<<(int)grid, THREADS, SMEM_BYTES, ctx->stream>>>(mhi, mlo, nb, nk, p, stall, err);
+                                          (int)smem_bytes(EPI_HIST)));
+        k_gram_tc<EPI_HIST><<<(int)grid, THREADS, smem_bytes(EPI_HIST), ctx->stream>>>(mhi, mlo, nb, nk, p, stall, err);
     } else {
         PG_CUDA(ctx, cudaFuncSetAttribute(k_gram_tc<EPI_EMIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)SMEM_BYTES));
-        k_gram_tc<EPI_EMIT><<<(int)grid, THREADS, SMEM_BYTES, ctx->stream>>>(mhi, mlo, nb, nk, p, stall, err);
+                                          (int)smem_bytes(EPI_EMIT)));
+        k_gram_tc<EPI_EMIT><<<(int)grid, THREADS, smem_bytes(EPI_EMIT), ctx->stream>>>(mhi, mlo, nb, nk, p, stall, err);
     }
     PG_LAUNCHED(ctx);
     return PG_OK;

@@ -122,6 +122,8 @@ pg_status pg_graph_alloc(pg_ctx* ctx, int32_t n, int64_t nnz, bool weighted, pg_
 // w may be null.  Result graph owns its arrays.
 pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const float* w,
                             int64_t npairs, pg_graph** out);
+// Row offsets R[n+1] from the row counts; the counts become the row starts.
+pg_status pg_row_offsets(pg_ctx* ctx, int32_t* cnt, int32_t n, int32_t* R);
 // Sorts the columns of every row ascending (carrying V when present).
 pg_status pg_csr_sort_rows(pg_ctx* ctx, pg_graph* g);
 // Row sort of a CSR whose rows are filled but unordered: Cin/Vin -> Cout/Vout

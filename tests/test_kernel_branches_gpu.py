@@ -91,3 +91,32 @@ def test_weighted_build_sizes(ctx, N, T, precision):
         Ro, Co, Vo = O.graph_r(O.corr_packed(z, weighted=True), N, 0.3, abs_mode=sign == "abs", weighted=True)
         assert np.array_equal(R, Ro) and np.array_equal(C, Co) and np.array_equal(V, Vo)
         assert info["edges"] == len(C) // 2
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+@pytest.mark.parametrize("N,value", [(31, 40.0), (128, 30.0), (129, 5.0), (255, 0.26), (257, 0.24), (900, 100.0),
+                                     (1030, 0.3), (1030, 0.2)])
+def test_adjacency_bits_and_pair_list(ctx, N, value, precision):
+    """Both forms of the decided edges (bits from 0.26 % of the pairs on, a
+    list below), at tile edges, up to the complete graph."""
+    bold = synth.bold_series(N, 60, 4, 300 + N)
+    z, _ = O.zscore(bold)
+    r = O.corr_packed(z)
+    for sign in ("signed", "abs"):
+        g, _ = ctx.build_graph(bold, mode="s", value=value, sign=sign, precision=precision, guard=1e-3)
+        R, C, _ = g.to_csr()
+        Ro, Co, _, _ = O.graph_k(r, N, O.sparsity_k(N, value), abs_mode=sign == "abs")
+        assert np.array_equal(R, Ro) and np.array_equal(C, Co)
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+def test_wide_band_flushes(ctx, precision):
+    """A guard so wide that most pairs go through the FP64 band."""
+    bold = synth.bold_series(700, 90, 4, 12)
+    z, _ = O.zscore(bold)
+    for guard, thr in ((0.5, 0.1), (0.2, 0.0)):
+        g, info = ctx.build_graph(bold, mode="r", value=thr, precision=precision, guard=guard)
+        R, C, _ = g.to_csr()
+        Ro, Co, _ = O.graph_r(O.corr_packed(z), 700, thr)
+        assert np.array_equal(R, Ro) and np.array_equal(C, Co)
+        assert info["band_pairs"] > 100000
