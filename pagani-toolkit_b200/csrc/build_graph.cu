@@ -350,6 +350,7 @@ __global__ void k_tie_keys(const int2* __restrict__ band, const unsigned long lo
 struct BuildState {
     unsigned long long n_pairs;   // pairs decided by the Gram tiles
     unsigned long long n_band;    // pairs of the FP64 band
+    unsigned long long n_wide;    // pairs listed between the sampled cuts
     unsigned long long n_added;   // band pairs that are edges (listed behind the decided ones)
     unsigned long long err_max;   // band error of the tiles: bits of the maximum, sum
     double err_sum;
@@ -555,6 +556,89 @@ extern "C" void pg_build_opts_default(pg_build_opts* o)
     o->exact_weights = 1;
 }
 
+// Histogram of the listed keys (bins of p, keys below p.kmin left out).
+__global__ void __launch_bounds__(256)
+k_wide_hist(const float* __restrict__ r, const unsigned long long* __restrict__ count, long long cap, EpiParams p)
+{
+    __shared__ unsigned int h[HIST_BINS];
+    for (int b = threadIdx.x; b < HIST_BINS; b += 256) h[b] = 0u;
+    __syncthreads();
+    const long long n = min((long long)*count, cap);
+    for (long long q = blockIdx.x * 256LL + threadIdx.x; q < n; q += gridDim.x * 256LL) {
+        const float k = epi_key(r[q], p.abs_mode);
+        if (!(k < p.kmin)) atomicAdd(&h[epi_bin(k, p)], 1u);
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < HIST_BINS; b += 256)
+        if (h[b]) atomicAdd(&p.hist[b], h[b]);
+}
+
+// Splits the list between the sampled cuts by the final ones: decided edges
+// (bits or list), band, dropped.  Eight entries per thread, one atomic per
+// block and output for 2048 entries.
+__global__ void __launch_bounds__(256)
+k_wide_split(const int2* __restrict__ ij, const float* __restrict__ r, const unsigned long long* __restrict__ count,
+             long long cap, EpiParams p)
+{
+    constexpr int U = 8;
+    __shared__ unsigned int s_warp[8];
+    __shared__ unsigned long long s_base[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long n = min((long long)*count, cap);
+    for (long long c0 = blockIdx.x * 256LL * U; c0 < n; c0 += gridDim.x * 256LL * U) {
+        float v[U];
+        int cls[U];
+        unsigned int mine = 0u;   // decided in the low half, band in the high half
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const long long q = c0 + k * 256 + threadIdx.x;
+            v[k] = q < n ? r[q] : 0.0f;
+            cls[k] = q < n ? epi_class(v[k], p) : 0;
+            mine += cls[k] == 1 ? 1u : cls[k] == 2 ? 0x10000u : 0u;
+        }
+        unsigned int x = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_warp[warp] = x;
+        __syncthreads();
+        unsigned int before = x - mine, total = 0u;
+        for (int w = 0; w < 8; w++) {
+            if (w < warp) before += s_warp[w];
+            total += s_warp[w];
+        }
+        if (threadIdx.x < 2) {
+            const unsigned int c = threadIdx.x ? total >> 16 : total & 0xffffu;
+            s_base[threadIdx.x] = c ? atomicAdd(threadIdx.x ? p.n_band : p.n_pairs, (unsigned long long)c) : 0ULL;
+        }
+        __syncthreads();
+        long long s1 = (long long)s_base[0] + (before & 0xffffu), s2 = (long long)s_base[1] + (before >> 16);
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            if (!cls[k]) continue;
+            const int2 e = ij[c0 + k * 256 + threadIdx.x];
+            if (cls[k] == 2) {
+                if (s2 < p.cap_band) {
+                    p.band[s2] = e;
+                    p.band_r[s2] = v[k];
+                }
+                s2++;
+            } else if (p.bits) {
+                atomicOr(&p.bits[(size_t)e.x * p.bit_words + (e.y >> 5)], 1u << (e.y & 31));
+                atomicOr(&p.bits[(size_t)e.y * p.bit_words + (e.x >> 5)], 1u << (e.x & 31));
+            } else {
+                if (s1 < p.cap_pairs) {
+                    p.pairs[s1] = e;
+                    if (p.weighted) p.pair_w[s1] = epi_key(v[k], p.abs_mode);
+                }
+                s1++;
+            }
+        }
+        __syncthreads();   // s_warp and s_base are reused
+    }
+}
+
 static pg_status run_gram(pg_ctx* ctx, const ZOperands& z, int precision, int mode, const EpiParams& p, int* err_dev)
 {
     if (precision == PG_SPLIT_BF16 && gram_tc_supported(ctx, z)) return launch_gram_tc(ctx, z, mode, p, err_dev);
@@ -625,9 +709,12 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     p.hist = (unsigned int*)(hist_dev + 2 * sizeof(unsigned long long));
     const unsigned long long* hbelow = (const unsigned long long*)hist_host;
     const unsigned int* h = (const unsigned int*)(hist_host + 2 * sizeof(unsigned long long));
-    auto hist_pass = [&](float kmin, int stride) -> pg_status {
+    auto set_bins = [&](float kmin) {
         p.kmin = kmin;
         p.scale = (float)HIST_BINS / (1.0f - kmin);
+    };
+    auto hist_pass = [&](float kmin, int stride) -> pg_status {
+        set_bins(kmin);
         p.tile_stride = stride;
         PG_CUDA(ctx, cudaMemsetAsync(hist_dev, 0, HIST_BYTES, ctx->stream));
         if (M1 > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_HIST, p, &ds->timeout));
@@ -648,117 +735,247 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         return s;
     };
     const bool list_all = o.mode == PG_THRESH_R && M1 <= LIST_ALL_PAIRS;
+    const bool no_band = g == 0.0 && o.mode == PG_THRESH_R;
+    const long long ntiles = (long long)(z.Np / 128) * (z.Np / 128 + 1) / 2;
+    const int bit_words = z.Np / 32;
+    const size_t bit_bytes = (size_t)N * bit_words * sizeof(uint32_t);
     long long k_edges = -1;  // sparsity: wanted edges
     float lo_cut, hi_cut;
-    if (o.mode == PG_THRESH_SPARSITY) {
-        if (!(o.value >= 0.0) || o.value > 100.0)
-            return pg_fail(ctx, PG_ERR_INVALID, "sparsity %g%% out of range", o.value);
-        k_edges = pg_sparsity_edges(N, (float)o.value);
-        if (k_edges > M1) k_edges = M1;
-        // floor for the binned range: from a sampled pass over every 8th tile
-        // when the problem is large, with room for twice the wanted edges
-        float floor_key = key_lo;
-        const long long ntiles = (long long)(z.Np / 128) * (z.Np / 128 + 1) / 2;
-        if (k_edges > 0 && ntiles >= 64LL * ctx->sm_count) {
-            PG_TRY(hist_pass(key_lo, 8));
-            const long long ps = hist_total();
-            const double f = M1 > 0 ? (double)ps / (double)M1 : 1.0;
-            const double want = 2.0 * (double)k_edges * f + 1024.0;
-            long long acc = 0;
-            int bf = 0;
-            for (int b = HIST_BINS - 1; b >= 0; b--) {
-                acc += h[b];
-                if ((double)acc >= want) { bf = b; break; }
-            }
-            floor_key = (float)std::max((double)key_lo, p.kmin + (double)bf / p.scale - g - 4.0 / p.scale);
-        }
-        PG_TRY(hist_pass(floor_key, 1));
-        if (floor_key > key_lo && hist_total() < k_edges) PG_TRY(hist_pass(key_lo, 1));  // sample misled us
-        if (k_edges <= 0) {
-            lo_cut = hi_cut = INFINITY;
-        } else {
-            long long acc = 0;
-            int bk = 0;
-            for (int b = HIST_BINS - 1; b >= 0; b--) {
-                acc += h[b];
-                if (acc >= k_edges) { bk = b; break; }
-            }
-            const double lo_b = p.kmin + (double)bk / p.scale, hi_b = p.kmin + (double)(bk + 1) / p.scale;
-            lo_cut = (float)(lo_b - g - 1.0 / p.scale);
-            hi_cut = (float)(hi_b + g + 1.0 / p.scale);
-        }
-    } else {
-        lo_cut = (float)(o.value - g);
-        hi_cut = (float)(o.value + g);
-        if (g == 0.0) lo_cut = hi_cut = nextafterf((float)o.value, INFINITY);  // tile decides alone: key > value
-        if (!list_all) PG_TRY(hist_pass(std::max(key_lo, std::min(lo_cut, edge_band) - 1e-3f), 1));
-    }
-    PG_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
-    if (!list_all && hist_total() + (long long)hbelow[0] != M1)
-        return pg_fail(ctx, PG_ERR_INTERNAL, "histogram holds %lld pairs, expected %lld",
-                       hist_total() + (long long)hbelow[0], M1);
-    if (lo_cut < key_lo) lo_cut = key_lo;
-    // capacities: every pair, or from the histogram (upper bounds: the bin
-    // mapping is monotone)
-    const bool no_band = g == 0.0 && o.mode == PG_THRESH_R;
-    long long cap_pairs = 0, cap_band = 0, cap_total;
-    if (list_all) {
-        cap_pairs = cap_total = M1;
-        cap_band = no_band ? 0 : M1;
-    } else {
-        int bh = std::isfinite(hi_cut) ? bin_of(hi_cut) : HIST_BINS;
-        int bl = std::isfinite(lo_cut) ? bin_of(lo_cut) : HIST_BINS;
-        int be = bin_of(edge_band);
-        for (int b = 0; b < HIST_BINS; b++) {
-            if (b >= bh) cap_pairs += h[b];
-            if (b >= bl || b >= be) cap_band += h[b];
-        }
-        if (lo_cut < p.kmin) cap_band += (long long)hbelow[0];   // band reaches below the binned range
-        if (hi_cut < p.kmin) cap_pairs += (long long)hbelow[0];
-        cap_band += (long long)hbelow[1];                         // r <= -(1 - guard), signed keys
-        if (no_band) cap_band = 0;
-        cap_total = cap_pairs + cap_band;
-    }
-    if (cap_pairs > (long long)INT32_MAX) return pg_fail(ctx, PG_ERR_TOO_LARGE, "too many edges");
+    long long cap_pairs = 0, cap_band = 0, cap_total = 0;
+    bool use_bits = false;
+    int2 *pairs = nullptr, *band = nullptr;
+    float* pw = nullptr;
+    float* band_r = nullptr;
+    double* key64 = nullptr;
+    uint32_t* bits = nullptr;
+
     // Decided edges of a binary graph go into adjacency bits where about four
     // passes over N^2 bits (0.45 ms at 58,000 nodes) beat the list's degree
     // count, scatter and sort (62 us per million edges): from 1.3e-3 N^2 edges
     // on, and always where every pair would be listed (at most 1 MB of bits).
     // Weights need the list; the bits may take 8 GiB.
-    const int bit_words = z.Np / 32;
-    const size_t bit_bytes = (size_t)N * bit_words * sizeof(uint32_t);
-    const long long expect = k_edges >= 0 ? k_edges : cap_pairs;
-    const bool use_bits = !weighted && bit_bytes <= (8ULL << 30) &&
-                          (list_all || (double)expect >= 1.3e-3 * (double)N * (double)N);
-    // ---- emit pass
-    int2 *pairs = nullptr, *band;
-    float* pw = nullptr;
-    float* band_r;
-    double* key64;
-    uint32_t* bits = nullptr;
-    if (use_bits) {
-        PG_TRY(pg_wst(ctx, "b.bits", (size_t)N * bit_words, &bits));
-        PG_CUDA(ctx, cudaMemsetAsync(bits, 0, bit_bytes, ctx->stream));
+    auto bits_pay = [&](long long edges) {
+        return !weighted && bit_bytes <= (8ULL << 30) && (list_all || (double)edges >= 1.3e-3 * (double)N * (double)N);
+    };
+    // room for the decided edges (cap_total with the band's)
+    auto prepare_decided = [&]() -> pg_status {
+        bits = nullptr;
+        pairs = nullptr;
+        if (use_bits) {
+            PG_TRY(pg_wst(ctx, "b.bits", (size_t)N * bit_words, &bits));
+            PG_CUDA(ctx, cudaMemsetAsync(bits, 0, bit_bytes, ctx->stream));
+        } else {
+            PG_TRY(pg_wst(ctx, "b.pairs", (size_t)std::max(1LL, cap_total), &pairs));
+        }
+        if (weighted) PG_TRY(pg_wst(ctx, "b.pw", (size_t)std::max(1LL, cap_total), &pw));
+        p.bits = bits;
+        p.bit_words = bit_words;
+        p.pairs = pairs;
+        p.pair_w = pw;
+        p.n_pairs = &ds->n_pairs;
+        p.cap_pairs = cap_pairs;
+        return PG_OK;
+    };
+    auto prepare_band = [&]() -> pg_status {
+        PG_TRY(pg_wst(ctx, "b.band", (size_t)std::max(1LL, cap_band), &band));
+        PG_TRY(pg_wst(ctx, "b.band_r", (size_t)std::max(1LL, cap_band), &band_r));
+        PG_TRY(pg_wst(ctx, "b.key64", (size_t)std::max(1LL, cap_band), &key64));
+        p.band = band;
+        p.band_r = band_r;
+        p.n_band = &ds->n_band;
+        p.cap_band = cap_band;
+        return PG_OK;
+    };
+    // the sparsity cuts that follow from the histogram bin of the k-th key
+    auto cuts_of_bin = [&](int bk) {
+        const double lo_b = p.kmin + (double)bk / p.scale, hi_b = p.kmin + (double)(bk + 1) / p.scale;
+        lo_cut = (float)(lo_b - g - 1.0 / p.scale);
+        hi_cut = (float)(hi_b + g + 1.0 / p.scale);
+    };
+
+    if (o.mode == PG_THRESH_SPARSITY) {
+        if (!(o.value >= 0.0) || o.value > 100.0)
+            return pg_fail(ctx, PG_ERR_INVALID, "sparsity %g%% out of range", o.value);
+        k_edges = pg_sparsity_edges(N, (float)o.value);
+        if (k_edges > M1) k_edges = M1;
     } else {
-        PG_TRY(pg_wst(ctx, "b.pairs", (size_t)std::max(1LL, cap_total), &pairs));
+        lo_cut = (float)(o.value - g);
+        hi_cut = (float)(o.value + g);
+        if (g == 0.0) lo_cut = hi_cut = nextafterf((float)o.value, INFINITY);  // tile decides alone: key > value
     }
-    if (weighted) PG_TRY(pg_wst(ctx, "b.pw", (size_t)std::max(1LL, cap_total), &pw));
-    PG_TRY(pg_wst(ctx, "b.band", (size_t)std::max(1LL, cap_band), &band));
-    PG_TRY(pg_wst(ctx, "b.band_r", (size_t)std::max(1LL, cap_band), &band_r));
-    PG_TRY(pg_wst(ctx, "b.key64", (size_t)std::max(1LL, cap_band), &key64));
-    p.lo_cut = lo_cut;
-    p.hi_cut = hi_cut;
-    p.bits = bits;
-    p.bit_words = bit_words;
-    p.pairs = pairs;
-    p.pair_w = pw;
-    p.n_pairs = &ds->n_pairs;
-    p.cap_pairs = cap_pairs;
-    p.band = band;
-    p.band_r = band_r;
-    p.n_band = &ds->n_band;
-    p.cap_band = cap_band;
-    if (M1 > 0 && cap_total > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p, &ds->timeout));
+    const float r_floor = std::max(key_lo, std::min(o.mode == PG_THRESH_R ? lo_cut : 0.0f, edge_band) - 1e-3f);
+
+    // ---- Large problems: a histogram of every 8th tile, then ONE full Gram
+    // pass.  r mode takes the sizes of its lists from the sample.  Sparsity
+    // mode takes two cuts from it that enclose the final band with 5 % of the
+    // wanted edges (and four standard deviations) to spare: pairs above are
+    // decided, pairs between go to a list, and the list's histogram places the
+    // k-th key in the same bin that a full histogram pass would.  Where the
+    // sample misled (a list overflows, or the k-th key or its band lies
+    // outside the cuts) the full histogram below decides, as for small
+    // problems.  58,000 voxels: the second full pass cost 2.3 of 7.9 ms; below
+    // two sampled tiles per SM it costs no more than the sample.
+    float floor_key = key_lo;
+    bool one_pass = false;
+    const bool sampled = !list_all && (o.mode == PG_THRESH_R || k_edges > 0) && ntiles >= 16LL * ctx->sm_count;
+    if (sampled) {
+        PG_TRY(hist_pass(o.mode == PG_THRESH_R ? r_floor : key_lo, 8));
+        const double f = (double)(hist_total() + (o.mode == PG_THRESH_R ? (long long)hbelow[0] : 0)) / (double)M1;
+        const int be = bin_of(edge_band);
+        auto room = [&](double n) { return std::min(M1, (long long)(1.3 * n / f) + 65536); };
+        double n_above = 0.0, n_list = (double)hbelow[1];   // sampled pairs above the cuts and between them
+        bool fits = f > 0.0;
+        if (o.mode == PG_THRESH_R) {
+            const int bh = bin_of(hi_cut), bl = bin_of(lo_cut);
+            for (int b = 0; b < HIST_BINS; b++) {
+                if (b >= bh) n_above += h[b];
+                if ((b >= bl && b <= bh) || b >= be) n_list += h[b];
+            }
+            fits = fits && lo_cut >= p.kmin;
+        } else {
+            const double ks = (double)k_edges * f, slack = 0.05 * ks + 4.0 * std::sqrt(ks) + 16.0;
+            const double want = 2.0 * ks + 1024.0;
+            long long acc = 0;
+            int b_hi = -1, b_lo = -1, bf = 0;
+            for (int b = HIST_BINS - 1; b >= 0; b--) {
+                acc += h[b];
+                if (b_hi < 0 && (double)acc >= ks - slack) b_hi = b;
+                if (b_lo < 0 && (double)acc >= ks + slack) b_lo = b;
+                if ((double)acc >= want) { bf = b; break; }
+            }
+            const double s_min = p.kmin, s_scale = p.scale;
+            // floor of the binned range, with room for twice the wanted edges
+            if (ntiles >= 64LL * ctx->sm_count)
+                floor_key = (float)std::max((double)key_lo, s_min + (double)bf / s_scale - g - 4.0 / s_scale);
+            set_bins(floor_key);
+            hi_cut = (float)(s_min + (b_hi + 1) / s_scale + g + 3.0 / p.scale);
+            lo_cut = (float)(s_min + b_lo / s_scale - g - 3.0 / p.scale);
+            fits = fits && ks > slack && b_lo >= 0 && lo_cut > p.kmin && lo_cut > key_lo && hi_cut < edge_band;
+            for (int b = b_lo < 0 ? 0 : b_lo; b < HIST_BINS; b++) {
+                const double key = s_min + (b + 1) / s_scale;   // upper edge of the sampled bin
+                if (key > hi_cut) n_above += h[b];
+                else n_list += h[b];
+                if (b >= be) n_list += h[b];
+            }
+            n_list *= 1.25;   // the bins that the cuts divide
+        }
+        cap_pairs = room(n_above);
+        cap_band = no_band ? 0 : room(n_list);
+        cap_total = cap_pairs + cap_band;
+        if (fits && cap_pairs <= (long long)INT32_MAX) {
+            use_bits = bits_pay(k_edges >= 0 ? k_edges : cap_pairs);
+            if (use_bits) cap_pairs = cap_total = M1;
+            PG_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
+            PG_TRY(prepare_decided());
+            PG_TRY(prepare_band());
+            p.lo_cut = lo_cut;
+            p.hi_cut = hi_cut;
+            if (o.mode == PG_THRESH_R) {
+                PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p, &ds->timeout));
+                PG_TRY(read_state());
+                one_pass = (long long)hs->n_pairs <= cap_pairs && (long long)hs->n_band <= cap_band;
+            } else {
+                int2* wide;
+                float* wide_r;
+                PG_TRY(pg_wst(ctx, "b.wide", (size_t)cap_band, &wide));
+                PG_TRY(pg_wst(ctx, "b.wide_r", (size_t)cap_band, &wide_r));
+                p.band = wide;
+                p.band_r = wide_r;
+                p.n_band = &ds->n_wide;
+                PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p, &ds->timeout));
+                PG_CUDA(ctx, cudaMemsetAsync(hist_dev, 0, HIST_BYTES, ctx->stream));
+                k_wide_hist<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(wide_r, &ds->n_wide, cap_band, p);
+                PG_LAUNCHED(ctx);
+                PG_CUDA(ctx, cudaMemcpyAsync(hist_host, hist_dev, HIST_BYTES, cudaMemcpyDeviceToHost, ctx->stream));
+                PG_TRY(read_state());
+                // every key at or above a bin below bin(hi_cut) and above
+                // bin(lo_cut) has been decided or listed
+                const float w_lo = lo_cut, w_hi = hi_cut;
+                const int top = bin_of(w_hi), bottom = bin_of(w_lo);
+                long long acc = (long long)hs->n_pairs;
+                for (int b = HIST_BINS - 1; b >= top; b--) acc += h[b];
+                one_pass = (long long)hs->n_pairs <= cap_pairs && (long long)hs->n_wide <= cap_band && acc < k_edges;
+                if (one_pass) {
+                    int bk = top - 1;
+                    for (; bk > bottom; bk--)
+                        if ((acc += h[bk]) >= k_edges) break;
+                    cuts_of_bin(bk);
+                    one_pass = bk > bottom && lo_cut >= w_lo && hi_cut <= w_hi;
+                }
+                if (one_pass) {
+                    cap_pairs = p.cap_pairs = cap_total;   // the list's decided pairs join the others
+                    p.lo_cut = lo_cut;
+                    p.hi_cut = hi_cut;
+                    p.band = band;
+                    p.band_r = band_r;
+                    p.n_band = &ds->n_band;
+                    k_wide_split<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(wide, wide_r, &ds->n_wide, cap_band, p);
+                    PG_LAUNCHED(ctx);
+                }
+            }
+            if (!one_pass) {
+                PG_CUDA(ctx, cudaMemsetAsync(&ds->n_pairs, 0, sizeof ds->n_pairs, ctx->stream));
+                PG_CUDA(ctx, cudaMemsetAsync(&ds->n_band, 0, sizeof ds->n_band, ctx->stream));
+            }
+        }
+        if (o.mode == PG_THRESH_R) {   // the cuts are the caller's
+            p.lo_cut = lo_cut;
+            p.hi_cut = hi_cut;
+        }
+    }
+
+    // ---- Otherwise: a full histogram pass, then the emit pass
+    if (!one_pass) {
+        if (o.mode == PG_THRESH_SPARSITY) {
+            PG_TRY(hist_pass(floor_key, 1));
+            if (floor_key > key_lo && hist_total() < k_edges) PG_TRY(hist_pass(key_lo, 1));  // sample misled us
+            if (k_edges <= 0) {
+                lo_cut = hi_cut = INFINITY;
+            } else {
+                long long acc = 0;
+                int bk = 0;
+                for (int b = HIST_BINS - 1; b >= 0; b--) {
+                    acc += h[b];
+                    if (acc >= k_edges) { bk = b; break; }
+                }
+                cuts_of_bin(bk);
+            }
+        } else if (!list_all) {
+            PG_TRY(hist_pass(r_floor, 1));
+        }
+        PG_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
+        if (!list_all && hist_total() + (long long)hbelow[0] != M1)
+            return pg_fail(ctx, PG_ERR_INTERNAL, "histogram holds %lld pairs, expected %lld",
+                           hist_total() + (long long)hbelow[0], M1);
+        if (lo_cut < key_lo) lo_cut = key_lo;
+        // capacities: every pair, or from the histogram (upper bounds: the bin
+        // mapping is monotone)
+        cap_pairs = cap_band = 0;
+        if (list_all) {
+            cap_pairs = cap_total = M1;
+            cap_band = no_band ? 0 : M1;
+        } else {
+            int bh = std::isfinite(hi_cut) ? bin_of(hi_cut) : HIST_BINS;
+            int bl = std::isfinite(lo_cut) ? bin_of(lo_cut) : HIST_BINS;
+            int be = bin_of(edge_band);
+            for (int b = 0; b < HIST_BINS; b++) {
+                if (b >= bh) cap_pairs += h[b];
+                if (b >= bl || b >= be) cap_band += h[b];
+            }
+            if (lo_cut < p.kmin) cap_band += (long long)hbelow[0];   // band reaches below the binned range
+            if (hi_cut < p.kmin) cap_pairs += (long long)hbelow[0];
+            cap_band += (long long)hbelow[1];                         // r <= -(1 - guard), signed keys
+            if (no_band) cap_band = 0;
+            cap_total = cap_pairs + cap_band;
+        }
+        if (cap_pairs > (long long)INT32_MAX) return pg_fail(ctx, PG_ERR_TOO_LARGE, "too many edges");
+        use_bits = bits_pay(k_edges >= 0 ? k_edges : cap_pairs);
+        PG_TRY(prepare_decided());
+        PG_TRY(prepare_band());
+        p.lo_cut = lo_cut;
+        p.hi_cut = hi_cut;
+        if (M1 > 0 && cap_total > 0) PG_TRY(run_gram(ctx, z, o.precision, EPI_EMIT, p, &ds->timeout));
+    }
     PG_CUDA(ctx, cudaEventRecord(ev[3], ctx->stream));
 
     // ---- FP64 recheck (and exact weights of the decided pairs)

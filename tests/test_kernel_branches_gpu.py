@@ -120,3 +120,47 @@ def test_wide_band_flushes(ctx, precision):
         Ro, Co, _ = O.graph_r(O.corr_packed(z), 700, thr)
         assert np.array_equal(R, Ro) and np.array_equal(C, Co)
         assert info["band_pairs"] > 100000
+
+
+@pytest.fixture(scope="module")
+def large():
+    """9,000 voxels: 71 tile rows, beyond the size from which one sampled
+    histogram replaces the full one (16 tiles per SM)."""
+    bold = synth.bold_series(9000, 48, 6, 77)
+    z, _ = O.zscore(bold)
+    return bold, O.corr_packed(z, weighted=True)   # no r near +-1: both range rules agree
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+@pytest.mark.parametrize("mode,value,sign,weighted", [("s", 1.0, "abs", False), ("s", 0.1, "signed", False),
+                                                      ("s", 0.5, "signed", True), ("r", 0.45, "abs", False),
+                                                      ("r", 0.55, "signed", True)])
+def test_one_full_gram_pass(ctx, large, mode, value, sign, weighted, precision):
+    bold, r = large
+    g, info = ctx.build_graph(bold, mode=mode, value=value, sign=sign, weighted=weighted, precision=precision)
+    R, C, V = g.to_csr()
+    if mode == "s":
+        Ro, Co, Vo, tau = O.graph_k(r, 9000, O.sparsity_k(9000, value), abs_mode=sign == "abs", weighted=weighted)
+        assert info["tau"] == tau
+    else:
+        Ro, Co, Vo = O.graph_r(r, 9000, value, abs_mode=sign == "abs", weighted=weighted)
+    assert np.array_equal(R, Ro) and np.array_equal(C, Co)
+    if weighted:
+        assert np.array_equal(V, Vo)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_sample_that_misses_the_edges(ctx, large, weighted):
+    """Voxels 128..255 share one signal: their tile (linear index 71, not a
+    multiple of 8) is not sampled and holds all of the wanted edges."""
+    bold = large[0].copy()
+    rng = np.random.default_rng(3)
+    bold[:, 128:256] = rng.standard_normal((48, 1)) + 0.2 * rng.standard_normal((48, 128))
+    z, _ = O.zscore(bold.astype(np.float32))
+    r = O.corr_packed(z, weighted=True)
+    g, info = ctx.build_graph(bold, mode="s", value=0.01, sign="signed", weighted=weighted)
+    R, C, V = g.to_csr()
+    Ro, Co, Vo, tau = O.graph_k(r, 9000, O.sparsity_k(9000, 0.01), weighted=weighted)
+    assert info["tau"] == tau and np.array_equal(R, Ro) and np.array_equal(C, Co)
+    if weighted:
+        assert np.array_equal(V, Vo)
