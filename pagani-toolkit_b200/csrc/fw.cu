@@ -4,33 +4,24 @@
 // weighted clustering (Cp_2, W/Cp/Cp/Cp_2.cpp:23-130) for one graph or a
 // batch of graphs in ONE persistent cooperative launch.
 //
-// Every graph's dense distance matrix (padded to a multiple of 64) stays in
-// HBM for the whole sweep (the reference streams 3072^2 blocks over PCIe per
-// phase and pads every graph to 3072).  The launch runs, with grid-wide
-// barriers between them:
-//   A  matrices set to +inf (0 on the diagonal); the weight maximum of every
-//      graph (the Onnela normalisation);
-//   B  edge distances 1/w and the cube roots of the normalised weights;
-//      then Onnela clustering of every node of every graph (one CTA per
-//      node, dynamic scheduler, the node's row dense in shared memory);
-//   then for every 64-wide k-block round kb, over all graphs with more than
-//   kb blocks at once (graphs are sorted by block count, so the active ones
-//   are a prefix of the order):
-//   1  closure of the diagonal block in shared memory, 64 steps, one barrier
-//      per step (row and column k are fixed during step k: d_kk = 0);
-//   2  the row and column panels against the closed diagonal block, in
-//      place, likewise;
-//   3  every other block: d_ij = min(d_ij, d_i,kb (x) d_kb,j) as a register-
-//      tiled min-plus product -- 4 x 4 outputs per thread, the kb column
-//      block transposed into shared memory so both operands are 16-byte
-//      vector loads, no barrier inside the k loop (the reference's phase 3
-//      keeps 6 x 6 per thread with scalar shared loads, CUBFW_ph3.cu:32-222);
-//   C  per-row sums of 1/d (CUBFW_Lp.cpp:77-104), then per graph Lp and the
-//      mean clustering.
-// The k-block width is fixed (64), so the distances do not depend on any
-// tuning; the autotuner only picks the CTAs per SM.
+// Every graph's dense distance matrix (padded to a multiple of 64) stays on
+// the device (the reference streams 3072^2 blocks over PCIe per phase and
+// pads every graph to 3072).  The launch first computes, over the whole grid,
+// the weight maxima, the cube roots of the normalised weights and the Onnela
+// clustering of every node; then its CTAs work in teams, each of which takes
+// one graph after another from a queue (largest first), so that the matrices
+// being swept stay in L2 and a barrier has only the team's arrivals:
+//   A  the team's rows: +inf, 0 on the diagonal, 1/w for the edges;
+//   then for every 64-wide k-block round kb:
+//   1  the row and column panels: the min-plus product with the closed
+//      diagonal block (its diagonal is 0, so the product keeps the panel);
+//   2  every other block: d_ij = min(d_ij, d_i,kb (x) d_kb,j); the diagonal
+//      block of the next round comes first and is closed at once (64 steps in
+//      registers), so no phase of its own waits for it;
+//   C  per-row sums of 1/d (CUBFW_Lp.cpp:77-104);
+// and at the end, per graph, Lp and the mean clustering.  The k-block width
+// is fixed (64), so the distances depend neither on the teams nor on the grid.
 #include "pg_internal.cuh"
-#include "tune.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cooperative_groups.h>
@@ -40,7 +31,14 @@ namespace cg = cooperative_groups;
 
 namespace {
 constexpr int B = 64;           // k-block width
-constexpr int FW_THREADS = 256; // 16 x 16 threads, 4 x 4 outputs each
+// One CTA per SM of four groups of 128 threads; a group works on a block (or
+// a node) of its own and synchronises by itself (named barrier), so that a
+// grid barrier has 148 arrivals and an SM still holds four blocks at once
+// (592 CTAs of 128 threads spent 13 us per panel phase, mostly in barriers).
+constexpr int GROUPS = 4, GT = 128;
+constexpr int FW_THREADS = GROUPS * GT;
+constexpr int TR = 8;   // a thread's tile: rows t / 16 + 8 r, columns 2 (t % 16), + 1, + 32, + 33
+constexpr int MAX_TEAMS = 64;
 constexpr int ONNELA_MAX_N = 4096; // largest graph of a batch for the Onnela row (n doubles in shared memory)
 
 struct FWGraph {
@@ -48,30 +46,38 @@ struct FWGraph {
     const int32_t* C;
     const float* V;     // null: every edge has distance 1
     int32_t n, np, nb;  // nodes, padded size, blocks per side
+    int32_t index;      // the caller's graph number
     long long off;      // matrix offset (elements)
-    int32_t node0;      // offset of its nodes in concatenated outputs
+    long long edge0;    // offset of its entries in cw
+    int32_t node0;      // its nodes in processing order
+    int32_t out0;       // and in the caller's concatenated outputs
+};
+
+struct FwControl {
+    int onnela_next;    // dynamic node scheduler
+    int queue;          // next graph
+    int timeout;        // a team barrier gave up
+    int pad;
+    unsigned arrived[MAX_TEAMS];
+    int graph[MAX_TEAMS];   // the graph a team works on
 };
 
 struct FwBatch {
     const FWGraph* gs;          // in processing order (blocks per side descending)
     int ng;
     int total_nodes;
-    int max_nb;
-    const int* active;          // [kb]: graphs with more than kb blocks (a prefix of gs)
-    const long long* p2;        // prefix over gs of 2 (nb - 1): panel tasks
-    const long long* p3;        // prefix over gs of (nb - 1)^2: phase-3 tasks
-    const long long* edge0;     // offset of each graph's edges in cw
-    const int* node_graph;      // concatenated node -> index in gs
+    int teams;
+    FwControl* ctl;
     float* D;
-    float* vmax;
-    double* cw;                 // per edge of every graph: (V / vmax)^(1/3)
-    int* onnela_next;           // dynamic node scheduler
+    float* vmax;                // per graph
+    double* cw;                 // per entry of every graph: (V / vmax)^(1/3)
+    int32_t* up;                // per node: where the entries of its row with a column above it begin
     int onnela;                 // compute the clustering
-    double* rowsum;             // per node
-    float* eff;                 // per node
-    double* lp;                 // per graph (in gs order)
-    float* cp;                  // per node
-    double* cp_mean;            // per graph (in gs order)
+    double* rowsum;             // per node, in processing order
+    float* eff;                 // per node, in the caller's order
+    double* lp;                 // per graph, in the caller's order; then 1.0 after a timeout
+    float* cp;                  // per node, in the caller's order
+    double* cp_mean;            // per graph, in the caller's order
 };
 
 __device__ __forceinline__ float* blk(float* D, const FWGraph& g, int bi, int bj)
@@ -79,15 +85,10 @@ __device__ __forceinline__ float* blk(float* D, const FWGraph& g, int bi, int bj
     return D + g.off + (long long)bi * B * g.np + (long long)bj * B;
 }
 
-// graph of task t in a prefix array of `count` graphs
-__device__ __forceinline__ int task_graph(const long long* pre, int count, long long t)
+__device__ __forceinline__ int group_thread() { return threadIdx.x & (GT - 1); }
+__device__ __forceinline__ void group_sync()
 {
-    int lo = 0, hi = count - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pre[mid] <= t) lo = mid; else hi = mid - 1;
-    }
-    return lo;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + ((int)threadIdx.x >> 7)), "n"(GT) : "memory");
 }
 
 // Onnela for node x of the batch (W/Cp/Cp/Cp_2.cpp:23-130, GPU weight maximum
@@ -97,74 +98,75 @@ __device__ __forceinline__ int task_graph(const long long* pre, int count, long 
 // same value up to rounding).  u's row is spread into a dense shared-memory
 // array (zero where h is not a neighbour), so the weight of (u, h) is one
 // shared load.
-__device__ void onnela_node(const FwBatch& p, int x, double* row, double* red)
+__device__ void onnela_node(const FwBatch& p, const FWGraph& g, int u, double* row, double* red)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = FW_THREADS / 32;
-    const int gi = p.node_graph[x];
-    const FWGraph g = p.gs[gi];
-    const long long e0 = p.edge0[gi];
-    const int u = x - g.node0;
+    const int lane = group_thread() & 31, warp = group_thread() >> 5, nwarp = GT / 32;
     const int32_t s = g.R[u], e = g.R[u + 1];
     const int k = e - s;
     double acc = 0.0;
     if (k >= 2) {
-        for (int32_t q = s + threadIdx.x; q < e; q += FW_THREADS) row[g.C[q]] = p.cw[e0 + q];
-        __syncthreads();
-        for (int32_t q = s + warp; q < e; q += nwarp) {
-            const int j = g.C[q];
-            const double cuj = p.cw[e0 + q];
-            double part = 0.0;
-            for (int32_t f = g.R[j] + lane; f < g.R[j + 1]; f += 32) {
-                const int h = g.C[f];
-                if (h > j) part += p.cw[e0 + f] * row[h];
+        const double* cw = p.cw + g.edge0;
+        for (int32_t q = s + group_thread(); q < e; q += GT) row[g.C[q]] = cw[q];
+        group_sync();
+        // a warp takes every fourth neighbour j, the ranges of 32 of them read
+        // at once; row j from its first column above j
+        for (int32_t q0 = s + warp; q0 < e; q0 += 32 * nwarp) {
+            const int32_t q = q0 + lane * nwarp;
+            int j = 0, f0 = 0, f1 = 0;
+            double cuj = 0.0;
+            if (q < e) {
+                j = g.C[q];
+                f0 = p.up[g.node0 + j];
+                f1 = g.R[j + 1];
+                cuj = cw[q];
             }
-            acc += cuj * part;
+            const int cnt = min(32, (e - q0 + nwarp - 1) / nwarp);
+            // four chunks of 32 entries from entry f on, up to b
+            auto fetch = [&](int f, int b, int (&h)[4], double (&w)[4]) {
+#pragma unroll
+                for (int z = 0; z < 4; z++) {
+                    h[z] = f + 32 * z < b ? g.C[f + 32 * z] : -1;
+                    w[z] = f + 32 * z < b ? cw[f + 32 * z] : 0.0;
+                }
+            };
+            int h[4], hn[4];
+            double w[4], wn[4];
+            int a = __shfl_sync(0xffffffffu, f0, 0), b = __shfl_sync(0xffffffffu, f1, 0);
+            fetch(a + lane, b, hn, wn);
+            for (int t = 0; t < cnt; t++) {
+#pragma unroll
+                for (int z = 0; z < 4; z++) {
+                    h[z] = hn[z];
+                    w[z] = wn[z];
+                }
+                const int jt = __shfl_sync(0xffffffffu, j, t), f_next = a + lane + 128, b_here = b;
+                // the next neighbour's row is on its way while this one is added
+                a = __shfl_sync(0xffffffffu, f0, min(t + 1, 31));
+                b = t + 1 < cnt ? __shfl_sync(0xffffffffu, f1, t + 1) : 0;
+                fetch(a + lane, b, hn, wn);
+                double part = 0.0;
+                for (int f = f_next;; f += 128) {
+#pragma unroll
+                    for (int z = 0; z < 4; z++)
+                        if (h[z] > jt) part += w[z] * row[h[z]];
+                    if (f - lane >= b_here) break;
+                    fetch(f, b_here, h, w);
+                }
+                acc += __shfl_sync(0xffffffffu, cuj, t) * part;
+            }
         }
-        __syncthreads();
-        for (int32_t q = s + threadIdx.x; q < e; q += FW_THREADS) row[g.C[q]] = 0.0;
+        group_sync();
+        for (int32_t q = s + group_thread(); q < e; q += GT) row[g.C[q]] = 0.0;
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    group_sync();
+    if (group_thread() == 0) {
         double t = 0.0;
         for (int w = 0; w < nwarp; w++) t += red[w];
-        p.cp[x] = k >= 2 ? (float)(2.0 * t / k / (k - 1)) : 0.0f;
+        p.cp[g.out0 + u] = k >= 2 ? (float)(2.0 * t / k / (k - 1)) : 0.0f;
     }
-    __syncthreads();
-}
-
-// Closure of a 64 x 64 block held in registers (4 x 4 per thread, rows
-// 4 ty.., columns 4 tx..) against the diagonal block: mode 0 the diagonal
-// block itself, 1 a row panel (s = min(s, dg (x) s)), 2 a column panel
-// (s = min(s, s (x) dg)).  Row k and column k do not change in step k
-// (d_kk = 0), so at every step their owners publish them to shared rows
-// (double-buffered: one barrier per step) and every thread updates its tile
-// from 16-byte loads; the closed diagonal block is read from dgT (its
-// columns stored as rows) or dg.
-__device__ __forceinline__ void closure(float (&acc)[4][4], const float (*dg)[B + 4], const float (*dgT)[B + 4],
-                                        float (*rowbuf)[B], float (*colbuf)[B], int mode)
-{
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll 1
-    for (int k0 = 0; k0 < B; k0 += 4) {
-#pragma unroll
-        for (int kk = 0; kk < 4; kk++) {
-            const int k = k0 + kk, buf = k & 1;
-            if (mode != 2 && ty == (k >> 2))   // row k of s: its owners are the threads of row block k/4
-                *(float4*)&rowbuf[buf][tx * 4] = make_float4(acc[kk][0], acc[kk][1], acc[kk][2], acc[kk][3]);
-            if (mode != 1 && tx == (k >> 2))   // column k of s
-                *(float4*)&colbuf[buf][ty * 4] = make_float4(acc[0][kk], acc[1][kk], acc[2][kk], acc[3][kk]);
-            __syncthreads();
-            const float4 a = mode == 1 ? *(const float4*)&dgT[k][ty * 4] : *(const float4*)&colbuf[buf][ty * 4];
-            const float4 b = mode == 2 ? *(const float4*)&dg[k][tx * 4] : *(const float4*)&rowbuf[buf][tx * 4];
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) acc[r][c] = fminf(acc[r][c], av[r] + bv[c]);
-        }
-    }
+    group_sync();
 }
 
 // min(a, b, c) in one instruction (sm_100)
@@ -175,247 +177,363 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     return r;
 }
 
-__device__ __forceinline__ void tile_load(float (&acc)[4][4], const float* src, int ld)
+// two FP32 additions in one instruction (sm_100)
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
 {
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const float4 v = *(const float4*)(src + (long long)(ty * 4 + r) * ld + tx * 4);
-        acc[r][0] = v.x; acc[r][1] = v.y; acc[r][2] = v.z; acc[r][3] = v.w;
-    }
-}
-
-__device__ __forceinline__ void tile_store(float* dst, int ld, const float (&acc)[4][4])
-{
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-        *(float4*)(dst + (long long)(ty * 4 + r) * ld + tx * 4) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-}
-
-// A 64 x 64 block into shared memory, row-major (rm) and/or transposed (tr).
-// Thread q reads the 4 floats at row q % 64, columns 4 (q / 64) + 16 it..:
-// a warp covers 32 consecutive rows of one column group, so the transposed
-// stores of a warp hit 32 consecutive words (no bank conflict).
-__device__ __forceinline__ void block_to_smem(const float* src, int ld, float (*rm)[B + 4], float (*tr)[B + 4])
-{
-#pragma unroll
-    for (int it = 0; it < B * B / 4 / FW_THREADS; it++) {
-        const int q = threadIdx.x + it * FW_THREADS;
-        const int i = q & (B - 1), j4 = (q >> 6) << 2;
-        const float4 v = *(const float4*)(src + (long long)i * ld + j4);
-        if (rm) *(float4*)&rm[i][j4] = v;
-        if (tr) {
-            tr[j4][i] = v.x; tr[j4 + 1][i] = v.y; tr[j4 + 2][i] = v.z; tr[j4 + 3][i] = v.w;
-        }
-    }
+    unsigned long long x, y, z;
+    memcpy(&x, &a, 8);
+    memcpy(&y, &b, 8);
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(z) : "l"(x), "l"(y));
+    float2 r;
+    memcpy(&r, &z, 8);
+    return r;
 }
 
 struct __align__(16) FwSmem {
     union {
         struct {
-            float dg[B][B + 4];     // the closed diagonal block, row-major
-            float dgT[B][B + 4];    // and transposed
-            float rowbuf[2][B];     // row k of the tile being closed
-            float colbuf[2][B];     // column k
-        } panel;
-        struct {
-            float at[B][B + 4];     // the (bi, kb) block transposed: at[k][i]
-            float bk[B][B + 4];     // the (kb, bj) block: bk[k][j]
+            float a[B][B + 4];      // left operand, row-major: a[i][k]
+            float2 b[B / 2][B];     // right operand, rows k and k + 1 interleaved: b[k / 2][j]
         } prod;
-        double row[ONNELA_MAX_N];  // Onnela: the node's row, dense
+        struct {
+            float row[2][B];        // row k of the block being closed
+            float col[2][B];        // column k
+        } close;
+        double row[ONNELA_MAX_N];   // Onnela: the node's row, dense
     };
-    double red[FW_THREADS / 32];
+    double red[GT / 32];
+    int next;                       // Onnela: the node taken
 };
 
-__device__ __forceinline__ void fw_batch_body(const FwBatch& p)
+// The thread's 8 x 4 outputs of a 64 x 64 block.
+struct Tile {
+    float v[TR][4];
+    __device__ __forceinline__ void load(const float* src, int ld)
+    {
+        const int i0 = group_thread() >> 4, j = 2 * (group_thread() & 15);
+#pragma unroll
+        for (int r = 0; r < TR; r++) {
+            const float2 x = *(const float2*)(src + (long long)(i0 + 8 * r) * ld + j);
+            const float2 y = *(const float2*)(src + (long long)(i0 + 8 * r) * ld + j + 32);
+            v[r][0] = x.x; v[r][1] = x.y; v[r][2] = y.x; v[r][3] = y.y;
+        }
+    }
+    __device__ __forceinline__ void store(float* dst, int ld) const
+    {
+        const int i0 = group_thread() >> 4, j = 2 * (group_thread() & 15);
+#pragma unroll
+        for (int r = 0; r < TR; r++) {
+            *(float2*)(dst + (long long)(i0 + 8 * r) * ld + j) = make_float2(v[r][0], v[r][1]);
+            *(float2*)(dst + (long long)(i0 + 8 * r) * ld + j + 32) = make_float2(v[r][2], v[r][3]);
+        }
+    }
+};
+
+// c = min(c, a (x) b) over 64 x 64 blocks, the first kn of their 64 steps
+// (the others are padding).  Two k per step: the sums of rows k and k + 1 are
+// one packed addition (the left operand holds consecutive k, the right one
+// interleaves its rows), and one three-input minimum folds both; min is
+// exact, so the order does not matter.  Per four k a thread issues 64 packed
+// additions, 64 minima and 12 16-byte shared loads for 128 updates.  Bound by
+// the minima: the loop alone runs at 65 updates per clock and SM whether two-
+// or three-input minima are used (60 with scalar additions), four blocks at
+// once in an SM at 51 with their loads and stores.
+__device__ __forceinline__ void min_plus(FwSmem& sm, Tile& c, const float* a, const float* b, int ld, int kn)
 {
-    cg::grid_group grid = cg::this_grid();
-    __shared__ FwSmem sm;
-    const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long nt = (long long)gridDim.x * blockDim.x;
-    // ---- A: +inf matrices with a zero diagonal; weight maxima
-    for (int gi = 0; gi < p.ng; gi++) {
-        const FWGraph g = p.gs[gi];
-        const long long tot4 = (long long)g.np * g.np / 4;
-        float4* d = (float4*)(p.D + g.off);
-        for (long long q = tid; q < tot4; q += nt) {
-            const long long e = q * 4, i = e / g.np, j = e % g.np;
+    const int t = group_thread();
+    // operands into shared memory: 64 rows x 16 float4 each
+#pragma unroll
+    for (int it = 0; it < B * B / 4 / GT; it++) {
+        const int q = t + it * GT, i = q >> 4, j = (q & 15) << 2;
+        *(float4*)&sm.prod.a[i][j] = *(const float4*)(a + (long long)i * ld + j);
+    }
+#pragma unroll
+    for (int it = 0; it < B * B / 8 / GT; it++) {
+        const int q = t + it * GT, k2 = q >> 4, j = (q & 15) << 2;
+        const float4 x = *(const float4*)(b + (long long)(2 * k2) * ld + j);
+        const float4 y = *(const float4*)(b + (long long)(2 * k2 + 1) * ld + j);
+        *(float4*)&sm.prod.b[k2][j] = make_float4(x.x, y.x, x.y, y.y);
+        *(float4*)&sm.prod.b[k2][j + 2] = make_float4(x.z, y.z, x.w, y.w);
+    }
+    group_sync();
+    const int i0 = t >> 4, j0 = 2 * (t & 15);
+#pragma unroll 2
+    for (int k = 0; k < kn; k += 4) {
+        float4 bl[2], bh[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            bl[h] = *(const float4*)&sm.prod.b[k / 2 + h][j0];
+            bh[h] = *(const float4*)&sm.prod.b[k / 2 + h][j0 + 32];
+        }
+#pragma unroll
+        for (int r = 0; r < TR; r++) {
+            const float4 x = *(const float4*)&sm.prod.a[i0 + 8 * r][k];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float2 ak = h ? make_float2(x.z, x.w) : make_float2(x.x, x.y);
+                const float2 s0 = add2(ak, make_float2(bl[h].x, bl[h].y)), s1 = add2(ak, make_float2(bl[h].z, bl[h].w));
+                const float2 s2 = add2(ak, make_float2(bh[h].x, bh[h].y)), s3 = add2(ak, make_float2(bh[h].z, bh[h].w));
+                c.v[r][0] = min3f(c.v[r][0], s0.x, s0.y);
+                c.v[r][1] = min3f(c.v[r][1], s1.x, s1.y);
+                c.v[r][2] = min3f(c.v[r][2], s2.x, s2.y);
+                c.v[r][3] = min3f(c.v[r][3], s3.x, s3.y);
+            }
+        }
+    }
+    group_sync();   // the operands are overwritten next
+}
+
+// Closure of a diagonal block held in registers: row k and column k do not
+// change in step k (d_kk = 0), so at every step their owners publish them to
+// shared rows (double-buffered: one barrier per step).
+__device__ __forceinline__ void close_block(FwSmem& sm, Tile& c)
+{
+    const int ti = group_thread() >> 4, tj = group_thread() & 15;
+#pragma unroll
+    for (int rk = 0; rk < TR; rk++) {
+#pragma unroll 1
+        for (int k8 = 0; k8 < 8; k8 += 2) {
+#pragma unroll
+            for (int kk = 0; kk < 2; kk++) {   // step k = 8 rk + k8 + kk
+                constexpr int half = 32 / 8;
+                if (ti == k8 + kk) {
+                    *(float2*)&sm.close.row[kk][2 * tj] = make_float2(c.v[rk][0], c.v[rk][1]);
+                    *(float2*)&sm.close.row[kk][2 * tj + 32] = make_float2(c.v[rk][2], c.v[rk][3]);
+                }
+                if (tj == ((8 * rk) & 31) / 2 + k8 / 2) {
+#pragma unroll
+                    for (int r = 0; r < TR; r++) sm.close.col[kk][ti + 8 * r] = c.v[r][kk + (rk >= half ? 2 : 0)];
+                }
+                group_sync();
+                const float2 b0 = *(const float2*)&sm.close.row[kk][2 * tj], b1 = *(const float2*)&sm.close.row[kk][2 * tj + 32];
+#pragma unroll
+                for (int r = 0; r < TR; r++) {
+                    const float a = sm.close.col[kk][ti + 8 * r];
+                    c.v[r][0] = fminf(c.v[r][0], a + b0.x);
+                    c.v[r][1] = fminf(c.v[r][1], a + b0.y);
+                    c.v[r][2] = fminf(c.v[r][2], a + b1.x);
+                    c.v[r][3] = fminf(c.v[r][3], a + b1.y);
+                }
+            }
+        }
+    }
+    group_sync();
+}
+
+// Barrier of a team's CTAs (all resident: the launch is cooperative).  The
+// wait is bounded; after a timeout nobody waits any more and the host reports
+// an error.
+struct Team {
+    unsigned* arrived;
+    int* timeout;
+    unsigned size, target;
+    __device__ void sync()
+    {
+        __syncthreads();
+        target += size;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(arrived, 1u);
+            volatile unsigned* seen = arrived;
+            for (unsigned spins = 0; *seen < target; spins++) {
+                if (spins > (1u << 27) || *(volatile int*)timeout) {
+                    atomicExch(timeout, 1);
+                    break;
+                }
+            }
+            __threadfence();
+        }
+        __syncthreads();
+    }
+};
+
+// the graph of node x (processing order), searched upwards from gi
+__device__ __forceinline__ int graph_at(const FwBatch& p, int gi, long long x)
+{
+    while (x >= p.gs[gi].node0 + p.gs[gi].n) gi++;
+    return gi;
+}
+
+// Floyd-Warshall of one graph by the CTAs of a team; this group is number vb
+// of the team's nvb.
+__device__ __forceinline__ void fw_graph(const FwBatch& p, const FWGraph& g, Team& team, FwSmem& sm, int vb, int nvb)
+{
+    const int lane = group_thread() & 31, gw = vb * (GT / 32) + (group_thread() >> 5), nw = nvb * (GT / 32);
+    // ---- A: a warp per row (init_block, FormBlock.cpp:64)
+    for (int i = gw; i < g.np; i += nw) {
+        float* d = p.D + g.off + (long long)i * g.np;
+        for (int j = 4 * lane; j < g.np; j += 128) {
             float4 v = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
             if (i >= j && i < j + 4) ((float*)&v)[i - j] = 0.0f;
-            d[q] = v;
+            *(float4*)(d + j) = v;
+        }
+        __syncwarp();   // the row is filled before its edges are written
+        if (i >= g.n) continue;
+        const int32_t s = g.R[i], e = g.R[i + 1];
+        for (int32_t q = s + lane; q < e; q += 32) {
+            const int j = g.C[q];
+            if (j != i) d[j] = g.V ? __fdiv_rn(1.0f, g.V[q]) : 1.0f;
         }
     }
-    if (p.onnela) {
-        for (int gi = blockIdx.x; gi < p.ng; gi += gridDim.x) {
-            const FWGraph g = p.gs[gi];
-            const int32_t nnz = g.R[g.n];
-            float m = -INFINITY;
-            for (int32_t q = threadIdx.x; q < nnz; q += FW_THREADS) m = fmaxf(m, g.V[q]);
-            for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            __shared__ float mx[FW_THREADS / 32];
-            if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5] = m;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                float t = -INFINITY;
-                for (int w = 0; w < FW_THREADS / 32; w++) t = fmaxf(t, mx[w]);
-                p.vmax[gi] = t;
-            }
-            __syncthreads();
-        }
+    team.sync();
+    Tile c;
+    if (vb == 0) {   // the first diagonal block; the others are closed as soon as they are final
+        float* d = blk(p.D, g, 0, 0);
+        c.load(d, g.np);
+        close_block(sm, c);
+        c.store(d, g.np);
     }
-    grid.sync();
-    // ---- B: edge distances 1/w (init_block, FormBlock.cpp:64); per-edge cube
-    // roots of the normalised weights for Onnela
-    for (int gi = 0; gi < p.ng; gi++) {
-        const FWGraph g = p.gs[gi];
-        const long long warps = nt >> 5;
-        const float vm = p.onnela ? p.vmax[gi] : 1.0f;
-        const long long e0 = p.onnela ? p.edge0[gi] : 0;
-        for (long long i = tid >> 5; i < g.n; i += warps)
-            for (int32_t q = g.R[i] + (threadIdx.x & 31); q < g.R[i + 1]; q += 32) {
-                const int j = g.C[q];
-                if (p.onnela) p.cw[e0 + q] = cbrt((double)__fdiv_rn(g.V[q], vm));
-                if (j == i) continue;
-                p.D[g.off + i * g.np + j] = g.V ? __fdiv_rn(1.0f, g.V[q]) : 1.0f;
-            }
-    }
-    if (p.onnela) {
-        grid.sync();
-        for (int q = threadIdx.x; q < ONNELA_MAX_N; q += FW_THREADS) sm.row[q] = 0.0;
-        __shared__ int s_x;
-        for (;;) {
-            __syncthreads();
-            if (threadIdx.x == 0) s_x = atomicAdd(p.onnela_next, 1);
-            __syncthreads();
-            const int x = s_x;
-            if (x >= p.total_nodes) break;
-            onnela_node(p, x, sm.row, sm.red);
-        }
-    }
-    grid.sync();
-    // ---- FW rounds over all graphs with more than kb blocks
-    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    for (int kb = 0; kb < p.max_nb; kb++) {
-        const int act = p.active[kb];
-        // 1: diagonal blocks
-        for (int gi = blockIdx.x; gi < act; gi += gridDim.x) {
-            const FWGraph g = p.gs[gi];
-            float* d = blk(p.D, g, kb, kb);
-            float acc[4][4];
-            tile_load(acc, d, g.np);
-            closure(acc, sm.panel.dg, sm.panel.dgT, sm.panel.rowbuf, sm.panel.colbuf, 0);
-            tile_store(d, g.np, acc);
-            __syncthreads();
-        }
-        grid.sync();
-        // 2: row and column panels
-        const long long n2 = p.p2[act];
-        for (long long t = blockIdx.x; t < n2; t += gridDim.x) {
-            const int gi = task_graph(p.p2, act, t);
-            const FWGraph g = p.gs[gi];
-            const int local = (int)(t - p.p2[gi]);
-            const bool row = local < g.nb - 1;
-            int other = row ? local : local - (g.nb - 1);
+    team.sync();
+    const int m = g.nb - 1;
+    for (int kb = 0; kb < g.nb && m > 0; kb++) {
+        // 1: row and column panels
+        const float* dg = blk(p.D, g, kb, kb);
+        const int kn = min(B, g.n - kb * B);   // rows and columns kb * B + kn.. are padding
+        for (int t = vb; t < 2 * m; t += nvb) {
+            const bool row = t < m;
+            int other = row ? t : t - m;
             if (other >= kb) other++;
             float* d = row ? blk(p.D, g, kb, other) : blk(p.D, g, other, kb);
-            block_to_smem(blk(p.D, g, kb, kb), g.np, row ? nullptr : sm.panel.dg, row ? sm.panel.dgT : nullptr);
-            float acc[4][4];
-            tile_load(acc, d, g.np);
-            __syncthreads();
-            closure(acc, sm.panel.dg, sm.panel.dgT, sm.panel.rowbuf, sm.panel.colbuf, row ? 1 : 2);
-            tile_store(d, g.np, acc);
-            __syncthreads();
+            c.load(d, g.np);
+            min_plus(sm, c, row ? dg : d, row ? d : dg, g.np, kn);
+            c.store(d, g.np);
         }
-        grid.sync();
-        // 3: the other blocks, register-tiled min-plus
-        const long long n3 = p.p3[act];
-        for (long long t = blockIdx.x; t < n3; t += gridDim.x) {
-            const int gi = task_graph(p.p3, act, t);
-            const FWGraph g = p.gs[gi];
-            const int m = g.nb - 1;
-            const int local = (int)(t - p.p3[gi]);
+        team.sync();
+        // 2: the other blocks, the next round's diagonal block first
+        const bool last = kb + 1 == g.nb;
+        for (int t = vb; t < m * m; t += nvb) {
+            // block (kb + 1, kb + 1) is number kb (m + 1) of the m x m others
+            int local = t;
+            if (!last) local = t == 0 ? kb * (m + 1) : t <= kb * (m + 1) ? t - 1 : t;
             int bi = local / m, bj = local % m;
             if (bi >= kb) bi++;
             if (bj >= kb) bj++;
-            block_to_smem(blk(p.D, g, bi, kb), g.np, nullptr, sm.prod.at);
-            block_to_smem(blk(p.D, g, kb, bj), g.np, sm.prod.bk, nullptr);
-            float* c = blk(p.D, g, bi, bj);
-            float acc[4][4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const float4 v = *(const float4*)(c + (long long)(ty * 4 + r) * g.np + tx * 4);
-                acc[r][0] = v.x; acc[r][1] = v.y; acc[r][2] = v.z; acc[r][3] = v.w;
-            }
-            __syncthreads();
-            // two k per step through the three-input minimum: one ALU
-            // instruction per two updates (the min-plus is bound by that
-            // pipe); min is exact, so the result equals the one-k loop's
-#pragma unroll 4
-            for (int k = 0; k < B; k += 2) {
-                const float4 ai = *(const float4*)&sm.prod.at[k][ty * 4];
-                const float4 bj4 = *(const float4*)&sm.prod.bk[k][tx * 4];
-                const float4 ai1 = *(const float4*)&sm.prod.at[k + 1][ty * 4];
-                const float4 bj1 = *(const float4*)&sm.prod.bk[k + 1][tx * 4];
-                const float av[4] = {ai.x, ai.y, ai.z, ai.w}, av1[4] = {ai1.x, ai1.y, ai1.z, ai1.w};
-                const float bv[4] = {bj4.x, bj4.y, bj4.z, bj4.w}, bv1[4] = {bj1.x, bj1.y, bj1.z, bj1.w};
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) acc[r][q] = min3f(acc[r][q], av[r] + bv[q], av1[r] + bv1[q]);
-            }
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-                *(float4*)(c + (long long)(ty * 4 + r) * g.np + tx * 4) =
-                    make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-            __syncthreads();
+            float* d = blk(p.D, g, bi, bj);
+            c.load(d, g.np);
+            min_plus(sm, c, blk(p.D, g, bi, kb), blk(p.D, g, kb, bj), g.np, kn);
+            if (!last && t == 0) close_block(sm, c);
+            c.store(d, g.np);
         }
-        grid.sync();
+        team.sync();
     }
     // ---- C: row sums of 1/d over finite, non-tiny distances (CUBFW_Lp.cpp:77-83,99-104)
-    {
-        const int lane = threadIdx.x & 31;
-        const long long warps = nt >> 5;
-        for (long long x = tid >> 5; x < p.total_nodes; x += warps) {
-            const int gi = p.node_graph[x];
-            const FWGraph g = p.gs[gi];
-            const int u = (int)x - g.node0;
-            const float* row = p.D + g.off + (long long)u * g.np;
-            double acc = 0.0;
-            for (int v = lane; v < g.n; v += 32) {
-                const float d = row[v];
-                if (v == u || !(d >= 0.1f)) continue;
-                acc += 1.0 / (double)d;
-            }
-            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == 0) {
-                p.rowsum[x] = acc;
-                float e = g.n > 1 ? (float)(acc / (double)(g.n - 1)) : 0.0f;
-                if (e < 1.0f / (float)g.n) e = 0.0f;
-                p.eff[x] = e;
-            }
+    for (int u = gw; u < g.n; u += nw) {
+        const float* row = p.D + g.off + (long long)u * g.np;
+        double acc = 0.0;
+        for (int v0 = lane; v0 < g.n; v0 += 128) {
+            float d[4];
+#pragma unroll
+            for (int z = 0; z < 4; z++) d[z] = v0 + 32 * z < g.n ? row[v0 + 32 * z] : 0.0f;
+#pragma unroll
+            for (int z = 0; z < 4; z++)
+                if (v0 + 32 * z != u && d[z] >= 0.1f) acc += 1.0 / (double)d[z];
         }
-    }
-    grid.sync();
-    for (long long gi = tid; gi < p.ng; gi += nt) {
-        const FWGraph g = p.gs[gi];
-        double t = 0.0;
-        for (int u = 0; u < g.n; u++) t += p.rowsum[g.node0 + u];
-        p.lp[gi] = t > 0.0 ? 1.0 / (t / g.n / (g.n - 1)) : INFINITY;
-        if (p.onnela) {
-            double c = 0.0;
-            for (int u = 0; u < g.n; u++) c += (double)p.cp[g.node0 + u];
-            p.cp_mean[gi] = g.n > 0 ? c / g.n : 0.0;
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) {
+            p.rowsum[g.node0 + u] = acc;
+            float e = g.n > 1 ? (float)(acc / (double)(g.n - 1)) : 0.0f;
+            if (e < 1.0f / (float)g.n) e = 0.0f;
+            p.eff[g.out0 + u] = e;
         }
     }
 }
 
-// The kernel under two register budgets (2 or 4 resident CTAs per SM); the
-// autotuner times both on the real batch (same arithmetic, same results).
-template <int MINB>
-__global__ void __launch_bounds__(FW_THREADS, MINB) k_fw_batch(FwBatch p)
+__global__ void __launch_bounds__(FW_THREADS, 1) k_fw_batch(FwBatch p)
 {
-    fw_batch_body(p);
+    cg::grid_group grid = cg::this_grid();
+    extern __shared__ __align__(16) unsigned char fw_smem[];
+    FwSmem& sm = ((FwSmem*)fw_smem)[threadIdx.x >> 7];
+    const int grp = threadIdx.x >> 7, vb = grp * gridDim.x + blockIdx.x, nvb = GROUPS * gridDim.x;
+    const int lane = group_thread() & 31;
+    const long long gw = (long long)vb * (GT / 32) + (group_thread() >> 5), nw = (long long)nvb * (GT / 32);
+    if (p.onnela) {
+        // ---- weight maxima
+        for (int gi = vb; gi < p.ng; gi += nvb) {
+            const FWGraph g = p.gs[gi];
+            const int32_t nnz = g.R[g.n];
+            float m = -INFINITY;
+#pragma unroll 4
+            for (int32_t q = group_thread(); q < nnz; q += GT) m = fmaxf(m, g.V[q]);
+            for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (lane == 0) sm.red[group_thread() >> 5] = m;
+            group_sync();
+            if (group_thread() == 0) {
+                float t = -INFINITY;
+                for (int w = 0; w < GT / 32; w++) t = fmaxf(t, (float)sm.red[w]);
+                p.vmax[gi] = t;
+            }
+            group_sync();
+        }
+        grid.sync();
+        // ---- per-entry cube roots of the normalised weights, a warp per node
+        int gi = 0;
+        for (long long x = gw; x < p.total_nodes; x += nw) {
+            gi = graph_at(p, gi, x);
+            const FWGraph g = p.gs[gi];
+            const int i = (int)x - g.node0;
+            const float vm = p.vmax[gi];
+            const int32_t s = g.R[i], e = g.R[i + 1];
+            int upto = 0;
+            bool ascending = true;
+            for (int32_t q = s + lane; q < e; q += 32) {
+                const int j = g.C[q];
+                upto += j <= i;
+                ascending &= q == s || g.C[q - 1] < j;
+                p.cw[g.edge0 + q] = cbrt((double)__fdiv_rn(g.V[q], vm));
+            }
+            upto = __reduce_add_sync(0xffffffffu, upto);
+            if (!__all_sync(0xffffffffu, ascending)) upto = 0;   // any order: the whole row is scanned
+            if (lane == 0) p.up[x] = s + upto;
+        }
+        grid.sync();
+        // ---- Onnela, a group per node
+        for (int q = group_thread(); q < ONNELA_MAX_N; q += GT) sm.row[q] = 0.0;
+        gi = 0;
+        for (;;) {
+            group_sync();
+            if (group_thread() == 0) sm.next = atomicAdd(&p.ctl->onnela_next, 1);
+            group_sync();
+            const int x = sm.next;
+            if (x >= p.total_nodes) break;
+            gi = graph_at(p, gi, x);
+            const FWGraph g = p.gs[gi];
+            onnela_node(p, g, x - g.node0, sm.row, sm.red);
+        }
+    }
+    // ---- Floyd-Warshall by teams; CTAs of a team are neighbours
+    {
+        const int n_cta = gridDim.x, t = (int)((long long)blockIdx.x * p.teams / n_cta);
+        const int first = (int)(((long long)t * n_cta + p.teams - 1) / p.teams);
+        const int end = (int)(((long long)(t + 1) * n_cta + p.teams - 1) / p.teams);
+        Team team{&p.ctl->arrived[t], &p.ctl->timeout, (unsigned)(end - first), 0u};
+        for (;;) {
+            if (blockIdx.x == first && threadIdx.x == 0) *(volatile int*)&p.ctl->graph[t] = atomicAdd(&p.ctl->queue, 1);
+            team.sync();
+            const int gi = *(volatile int*)&p.ctl->graph[t];
+            if (gi >= p.ng || *(volatile int*)&p.ctl->timeout) break;
+            const FWGraph g = p.gs[gi];
+            fw_graph(p, g, team, sm, grp * (end - first) + (blockIdx.x - first), GROUPS * (end - first));
+        }
+    }
+    grid.sync();
+    // ---- a warp per graph: fixed strided sums and a shuffle tree
+    for (long long gi = gw; gi < p.ng; gi += nw) {
+        const FWGraph g = p.gs[gi];
+        double t = 0.0, m = 0.0;
+        for (int u = lane; u < g.n; u += 32) {
+            t += p.rowsum[g.node0 + u];
+            if (p.onnela) m += (double)p.cp[g.out0 + u];
+        }
+        for (int o = 16; o; o >>= 1) {
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+            m += __shfl_xor_sync(0xffffffffu, m, o);
+        }
+        if (lane == 0) {
+            p.lp[g.index] = t > 0.0 ? 1.0 / (t / g.n / (g.n - 1)) : INFINITY;
+            if (p.onnela) p.cp_mean[g.index] = g.n > 0 ? m / g.n : 0.0;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.lp[p.ng] = p.ctl->timeout ? 1.0 : 0.0;
 }
 
 __global__ void k_fw_copy_out(const FWGraph* __restrict__ gs, const float* __restrict__ D, float* __restrict__ out)
@@ -426,169 +544,97 @@ __global__ void k_fw_copy_out(const FWGraph* __restrict__ gs, const float* __res
         out[q] = D[g.off + (q / g.n) * g.np + q % g.n];
 }
 
-// outputs in processing order -> caller's order
-__global__ void k_fw_unpermute(const int* __restrict__ perm, const FWGraph* __restrict__ gs, int ng,
-                               const int* __restrict__ node0_out, const float* __restrict__ eff,
-                               const double* __restrict__ lp, const float* __restrict__ cp,
-                               const double* __restrict__ cpm, float* __restrict__ eff_o, double* __restrict__ lp_o,
-                               float* __restrict__ cp_o, double* __restrict__ cpm_o, int onnela)
-{
-    for (int gi = blockIdx.x; gi < ng; gi += gridDim.x) {
-        const FWGraph g = gs[gi];
-        const int dst = perm[gi];
-        const int o = node0_out[dst];
-        for (int u = threadIdx.x; u < g.n; u += blockDim.x) {
-            eff_o[o + u] = eff[g.node0 + u];
-            if (onnela) cp_o[o + u] = cp[g.node0 + u];
-        }
-        if (threadIdx.x == 0) {
-            lp_o[dst] = lp[gi];
-            if (onnela) cpm_o[dst] = cpm[gi];
-        }
-    }
-}
 }  // namespace
 
-// Graph table in processing order and the device batch description.
-struct FwPlan {
-    FwBatch b;
-    FWGraph* dtab;
-    int* perm;          // processing index -> caller's index
-    int* node0_out;     // caller's node offsets
-    long long total;
-    int grid;
-    int minb;           // register budget of the kernel instance (resident CTAs per SM)
-};
-
-static pg_status fw_launch(pg_ctx* ctx, FwPlan* P, bool profiled);
-
-static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, bool onnela, FwPlan* P)
+static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, bool onnela, FwBatch* P)
 {
     std::vector<int> order(ng);
     std::iota(order.begin(), order.end(), 0);
     auto nb_of = [&](int i) { return std::max(1, (graphs[i]->n + B - 1) / B); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return nb_of(x) > nb_of(y); });
     std::vector<FWGraph> tab(ng);
-    std::vector<long long> p2(ng + 1, 0), p3(ng + 1, 0), edge0(ng, 0);
-    long long edges = 0;
-    std::vector<int> perm(ng), node0_out(ng), node_graph;
-    long long off = 0;
-    int node0 = 0, nmax = 1, max_nb = 0;
-    int o = 0;
+    std::vector<int> out0(ng);
+    long long edges = 0, off = 0;
+    int nodes = 0, nmax = 1;
     for (int i = 0; i < ng; i++) {
-        node0_out[i] = o;
-        o += graphs[i]->n;
+        out0[i] = nodes;
+        nodes += graphs[i]->n;
     }
+    nodes = 0;
+    double work = 0.0, work_max = 0.0;
     for (int q = 0; q < ng; q++) {
         const pg_graph* g = graphs[order[q]];
         if (onnela && !g->V) return pg_fail(ctx, PG_ERR_INVALID, "Onnela clustering needs a weighted graph");
         const int nb = nb_of(order[q]);
-        tab[q] = {g->R, g->C, g->V, g->n, nb * B, nb, off, node0};
-        perm[q] = order[q];
+        tab[q] = {g->R, g->C, g->V, g->n, nb * B, nb, order[q], off, edges, nodes, out0[order[q]]};
         off += (long long)nb * B * nb * B;
-        for (int u = 0; u < g->n; u++) node_graph.push_back(q);
-        node0 += g->n;
-        nmax = std::max(nmax, (int)g->n);
-        max_nb = std::max(max_nb, nb);
-        edge0[q] = edges;
+        nodes += g->n;
         edges += g->nnz;
-        p2[q + 1] = p2[q] + 2LL * (nb - 1);
-        p3[q + 1] = p3[q] + (long long)(nb - 1) * (nb - 1);
+        nmax = std::max(nmax, (int)g->n);
+        const double w = (double)nb * nb * nb;
+        work += w;
+        work_max = std::max(work_max, w);
     }
     if (onnela && nmax > ONNELA_MAX_N)
         return pg_fail(ctx, PG_ERR_TOO_LARGE, "Onnela in the batched launch: n=%d above %d", nmax, ONNELA_MAX_N);
-    std::vector<int> active(max_nb);
-    for (int kb = 0; kb < max_nb; kb++) {
-        int a = 0;
-        while (a < ng && tab[a].nb > kb) a++;
-        active[kb] = a;
-    }
-    FwBatch& b = P->b;
+    FwBatch& b = *P;
     memset(&b, 0, sizeof b);
-    int *dact, *dng, *dperm, *dn0;
-    long long *dp2, *dp3, *de0;
+    FWGraph* dtab;
     PG_TRY(pg_wst(ctx, "fw.D", (size_t)off, &b.D));
-    PG_TRY(pg_wst(ctx, "fw.tab", (size_t)ng, &P->dtab));
-    PG_TRY(pg_wst(ctx, "fw.active", (size_t)max_nb, &dact));
-    PG_TRY(pg_wst(ctx, "fw.p2", (size_t)ng + 1, &dp2));
-    PG_TRY(pg_wst(ctx, "fw.p3", (size_t)ng + 1, &dp3));
-    PG_TRY(pg_wst(ctx, "fw.edge0", (size_t)ng, &de0));
-    PG_TRY(pg_wst(ctx, "fw.cw", (size_t)(onnela ? edges : 0) + 1, &b.cw));
-    PG_TRY(pg_wst(ctx, "fw.ngraph", (size_t)node0 + 1, &dng));
-    PG_TRY(pg_wst(ctx, "fw.perm", (size_t)ng, &dperm));
-    PG_TRY(pg_wst(ctx, "fw.node0o", (size_t)ng, &dn0));
-    PG_TRY(pg_wst(ctx, "fw.vmax", (size_t)ng, &b.vmax));
-    PG_TRY(pg_wst(ctx, "fw.next", 1, &b.onnela_next));
-    PG_TRY(pg_wst(ctx, "fw.rows", (size_t)node0 + 1, &b.rowsum));
-    PG_TRY(pg_wst(ctx, "fw.eff", (size_t)node0 + 1, &b.eff));
-    PG_TRY(pg_wst(ctx, "fw.lp", (size_t)ng, &b.lp));
-    PG_TRY(pg_wst(ctx, "fw.cp", (size_t)node0 + 1, &b.cp));
-    PG_TRY(pg_wst(ctx, "fw.cpm", (size_t)ng, &b.cp_mean));
-    PG_CUDA(ctx, cudaMemcpyAsync(P->dtab, tab.data(), sizeof(FWGraph) * ng, cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(dact, active.data(), sizeof(int) * max_nb, cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(dp2, p2.data(), sizeof(long long) * (ng + 1), cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(dp3, p3.data(), sizeof(long long) * (ng + 1), cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(de0, edge0.data(), sizeof(long long) * ng, cudaMemcpyHostToDevice, ctx->stream));
-    if (node0 > 0)
-        PG_CUDA(ctx, cudaMemcpyAsync(dng, node_graph.data(), sizeof(int) * node0, cudaMemcpyHostToDevice,
-                                     ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(dperm, perm.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaMemcpyAsync(dn0, node0_out.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, ctx->stream));
-    PG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));   // host tables' lifetime
-    b.gs = P->dtab;
+    PG_TRY(pg_wst(ctx, "fw.tab", (size_t)ng, &dtab));
+    PG_TRY(pg_wst(ctx, "fw.ctl", 1, &b.ctl));
+    if (onnela) {
+        PG_TRY(pg_wst(ctx, "fw.cw", (size_t)edges + 1, &b.cw));
+        PG_TRY(pg_wst(ctx, "fw.up", (size_t)nodes + 1, &b.up));
+        PG_TRY(pg_wst(ctx, "fw.vmax", (size_t)ng, &b.vmax));
+        PG_TRY(pg_wst(ctx, "fw.cp", (size_t)nodes + 1, &b.cp));
+        PG_TRY(pg_wst(ctx, "fw.cpm", (size_t)ng, &b.cp_mean));
+    }
+    PG_TRY(pg_wst(ctx, "fw.rows", (size_t)nodes + 1, &b.rowsum));
+    PG_TRY(pg_wst(ctx, "fw.eff", (size_t)nodes + 1, &b.eff));
+    PG_TRY(pg_wst(ctx, "fw.lp", (size_t)ng + 1, &b.lp));
+    PG_TRY(pg_h2d(ctx, dtab, tab.data(), sizeof(FWGraph) * ng));
+    b.gs = dtab;
     b.ng = ng;
-    b.total_nodes = node0;
-    b.max_nb = max_nb;
-    b.active = dact;
-    b.p2 = dp2;
-    b.p3 = dp3;
-    b.edge0 = de0;
-    b.node_graph = dng;
+    b.total_nodes = nodes;
     b.onnela = onnela;
-    P->perm = dperm;
-    P->node0_out = dn0;
-    P->total = node0;
-    int per2 = 0, per4 = 0;
-    PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_fw_batch<2>, FW_THREADS, 0));
-    PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per4, k_fw_batch<4>, FW_THREADS, 0));
-    if (per2 < 1) return pg_fail(ctx, PG_ERR_INTERNAL, "FW: kernel does not fit an SM");
-    // choices: (register budget, resident CTAs per SM)
-    std::vector<TuneChoice> cands;
-    for (int c = 1; c <= std::min(per2, 2); c++) cands.push_back({2, c});
-    for (int c = 3; c <= std::min(per4, 4); c++) cands.push_back({4, c});
-    TuneChoice best{2, std::min(per2, 2)};
-    // shape bucket: log2 of the rms padded graph size and log2 of the number
-    // of graphs (passed as the "mean degree" of the key); a 160- and a
-    // 512-graph batch of the same sizes must not share a choice
-    const long long rms = off > 0 ? (long long)std::sqrt((double)off / ng) : 0;
-    const std::string key = tune_key("fw_batch", rms, (long long)ng * std::max(1LL, rms));
-    PG_TRY(tune_pick(ctx, key, cands, &best, [&](const TuneChoice& c) -> pg_status {
-        P->minb = c.a;
-        P->grid = ctx->sm_count * c.b;
-        return fw_launch(ctx, P, false);
-    }));
-    P->minb = best.a;
-    P->grid = ctx->sm_count * best.b;
+    // As many teams as leave the largest graph, alone on its team, at most
+    // half of the batch's time, and at least four SMs (16 blocks at once) per
+    // team: one graph gets the whole GPU, 512 region graphs 37 teams (17.9 ms;
+    // with every phase over all graphs and the whole grid 20.7 ms).
+    b.teams = (int)std::max(1.0, std::min({(double)MAX_TEAMS, ctx->sm_count / 4.0, 0.5 * work / std::max(work_max, 1.0)}));
+    PG_CUDA(ctx, cudaFuncSetAttribute(k_fw_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(GROUPS * sizeof(FwSmem))));
     return PG_OK;
 }
 
-static pg_status fw_launch(pg_ctx* ctx, FwPlan* P, bool profiled)
+static pg_status fw_launch(pg_ctx* ctx, const FwBatch& b)
 {
-    PG_CUDA(ctx, cudaMemsetAsync(P->b.onnela_next, 0, sizeof(int), ctx->stream));
+    PG_CUDA(ctx, cudaMemsetAsync(b.ctl, 0, sizeof(FwControl), ctx->stream));
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(P->grid);
+    cfg.gridDim = dim3(ctx->sm_count);
     cfg.blockDim = dim3(FW_THREADS);
+    cfg.dynamicSmemBytes = GROUPS * sizeof(FwSmem);
     cfg.stream = ctx->stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const int h = profiled ? pg_prof_begin(ctx, "k_fw_batch") : -1;
-    if (P->minb == 4) PG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_fw_batch<4>, P->b));
-    else PG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_fw_batch<2>, P->b));
+    const int h = pg_prof_begin(ctx, "k_fw_batch");
+    PG_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_fw_batch, b));
     PG_LAUNCHED(ctx);
     pg_prof_end(ctx, h);
+    return PG_OK;
+}
+
+// The per-graph Lp (to lp, may be null) and the timeout mark behind them.
+static pg_status fw_read_lp(pg_ctx* ctx, const FwBatch& b, double* lp)
+{
+    std::vector<double> h((size_t)b.ng + 1);
+    PG_TRY(pg_d2h(ctx, h.data(), b.lp, sizeof(double) * h.size()));
+    if (h[b.ng] != 0.0) return pg_fail(ctx, PG_ERR_TIMEOUT, "FW: a team barrier timed out");
+    if (lp) std::copy(h.begin(), h.begin() + b.ng, lp);
     return PG_OK;
 }
 
@@ -598,18 +644,18 @@ extern "C" pg_status pg_fw_paths(pg_ctx* ctx, const pg_graph* g, float* dist, fl
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     const int n = g->n;
     const pg_graph* one[1] = {g};
-    FwPlan P;
-    PG_TRY(fw_plan(ctx, one, 1, false, &P));
-    PG_TRY(fw_launch(ctx, &P, true));
+    FwBatch b;
+    PG_TRY(fw_plan(ctx, one, 1, false, &b));
+    PG_TRY(fw_launch(ctx, b));
+    PG_TRY(fw_read_lp(ctx, b, lp));
     if (dist) {
         float* tmp;
         PG_TRY(pg_wst(ctx, "fw.out", (size_t)n * n + 1, &tmp));
-        k_fw_copy_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(P.dtab, P.b.D, tmp);
+        k_fw_copy_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(b.gs, b.D, tmp);
         PG_LAUNCHED(ctx);
         PG_TRY(pg_d2h(ctx, dist, tmp, sizeof(float) * (size_t)n * n));
     }
-    if (eff) PG_TRY(pg_d2h(ctx, eff, P.b.eff, sizeof(float) * n));
-    if (lp) PG_TRY(pg_d2h(ctx, lp, P.b.lp, sizeof(double)));
+    if (eff) PG_TRY(pg_d2h(ctx, eff, b.eff, sizeof(float) * n));
     return PG_OK;
 }
 
@@ -620,23 +666,12 @@ extern "C" pg_status pg_fw_batched(pg_ctx* ctx, const pg_graph* const* graphs, i
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     for (int i = 0; i < count; i++)
         if (!graphs[i]) return pg_fail(ctx, PG_ERR_INVALID, "graph %d is null", i);
-    const bool onnela = cp || cp_mean;
-    FwPlan P;
-    PG_TRY(fw_plan(ctx, graphs, count, onnela, &P));
-    PG_TRY(fw_launch(ctx, &P, true));
-    float *deff, *dcp;
-    double *dlp, *dcpm;
-    PG_TRY(pg_wst(ctx, "fwb.eff", (size_t)P.total + 1, &deff));
-    PG_TRY(pg_wst(ctx, "fwb.cp", (size_t)P.total + 1, &dcp));
-    PG_TRY(pg_wst(ctx, "fwb.lp", (size_t)count, &dlp));
-    PG_TRY(pg_wst(ctx, "fwb.cpm", (size_t)count, &dcpm));
-    k_fw_unpermute<<<std::min(count, 4096), 256, 0, ctx->stream>>>(P.perm, P.dtab, count, P.node0_out, P.b.eff, P.b.lp,
-                                                                   P.b.cp, P.b.cp_mean, deff, dlp, dcp, dcpm,
-                                                                   onnela);
-    PG_LAUNCHED(ctx);
-    if (eff) PG_TRY(pg_d2h(ctx, eff, deff, sizeof(float) * P.total));
-    if (lp) PG_TRY(pg_d2h(ctx, lp, dlp, sizeof(double) * count));
-    if (cp) PG_TRY(pg_d2h(ctx, cp, dcp, sizeof(float) * P.total));
-    if (cp_mean) PG_TRY(pg_d2h(ctx, cp_mean, dcpm, sizeof(double) * count));
+    FwBatch b;
+    PG_TRY(fw_plan(ctx, graphs, count, cp || cp_mean, &b));
+    PG_TRY(fw_launch(ctx, b));
+    PG_TRY(fw_read_lp(ctx, b, lp));
+    if (eff) PG_TRY(pg_d2h(ctx, eff, b.eff, sizeof(float) * b.total_nodes));
+    if (cp) PG_TRY(pg_d2h(ctx, cp, b.cp, sizeof(float) * b.total_nodes));
+    if (cp_mean) PG_TRY(pg_d2h(ctx, cp_mean, b.cp_mean, sizeof(double) * count));
     return PG_OK;
 }

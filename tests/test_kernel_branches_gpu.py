@@ -164,3 +164,38 @@ def test_sample_that_misses_the_edges(ctx, large, weighted):
     assert info["tau"] == tau and np.array_equal(R, Ro) and np.array_equal(C, Co)
     if weighted:
         assert np.array_equal(V, Vo)
+
+
+# ------------------------------------------------------- Floyd-Warshall batch
+@pytest.mark.parametrize("sizes", [[1], [2, 63], [64], [65, 3, 130], [127, 128, 129, 190, 64, 1, 66],
+                                   [257] * 3 + [70] * 90, [30 + 7 * q for q in range(60)]])
+def test_fw_team_batches(ctx, sizes):
+    """One team, several, and the most (a batch of many graphs), with sizes at
+    the 64-wide block edges, against the dense FP32 closure and the oracle's
+    clustering; the results come back in the caller's order."""
+    gs, csr = [], []
+    for q, n in enumerate(sizes):
+        R, C, V = G.random_weighted(n, 0.15 if n > 20 else 0.6, 1000 + q)
+        V = np.zeros(0, np.float32) if len(C) == 0 else V
+        csr.append((R, C, V))
+        gs.append(ctx.graph(R, C, V))
+    out = ctx.fw_batched(gs)
+    for (R, C, V), (eff, lp, cp, cpm) in zip(csr, out):
+        n = len(R) - 1
+        D = np.full((n, n), np.inf, np.float32)
+        rows = np.repeat(np.arange(n), np.diff(R))
+        D[rows, C] = np.float32(1.0) / V
+        np.fill_diagonal(D, 0.0)
+        D = O.fw_dense(D)
+        E = np.zeros((n, n))
+        ok = (D >= 0.1) & ~np.eye(n, dtype=bool)
+        E[ok] = 1.0 / D[ok].astype(np.float64)
+        want = E.sum(1) / max(n - 1, 1)
+        want[want < 1.0 / n] = 0.0
+        # distances: sums of at most ~10 FP32 terms in any order
+        np.testing.assert_allclose(eff, want, rtol=1e-5)
+        t = E.sum()
+        assert lp == pytest.approx(n * (n - 1) / t, rel=1e-5) if t > 0 else np.isinf(lp)
+        cp_or, m_or = O.onnela(R, C, V)
+        np.testing.assert_allclose(cp, cp_or, rtol=2.0 ** -22)
+        assert cpm == pytest.approx(m_or, rel=2.0 ** -22)
