@@ -13,7 +13,7 @@
 // MAX_D are added to inv[v] directly as they are found.
 //
 // One cooperative launch runs every batch and level (grid-wide barriers
-// between levels, the "any source still growing" flag in device memory), so
+// between levels, the set of sources still growing in device memory), so
 // the computation needs no host round trip and can be captured in a CUDA
 // graph.  The sources per batch (NW) and the CTAs per SM are picked by the
 // autotuner; the result is the same for every choice.
@@ -33,6 +33,46 @@ struct Words {
     unsigned long long w[NW];
 };
 
+// OR of a node's words into acc, 32 bytes per load
+template <int NW>
+__device__ __forceinline__ void or_words(Words<NW>& acc, const Words<NW>* p)
+{
+#pragma unroll
+    for (int q = 0; q < NW; q += 4) {
+        unsigned long long a, b, c, d;
+        asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(a), "=l"(b), "=l"(c), "=l"(d)
+                     : "l"((const char*)p + 8 * q));
+        acc.w[q] |= a;
+        acc.w[q + 1] |= b;
+        acc.w[q + 2] |= c;
+        acc.w[q + 3] |= d;
+    }
+}
+
+// Publishes the sources that grew at this level: the words of all warps are
+// combined in the CTA, and only bits that the level's words did not show yet
+// reach L2 (an atomic per CTA and word would serialise there).  The caller's
+// grid barrier follows, so the shared array is free again.
+template <int NW>
+__device__ __forceinline__ void publish_active(const Words<NW>& mine, unsigned long long* slot)
+{
+    __shared__ unsigned long long s_act[THREADS / 32][NW];
+    unsigned long long shown = 0ULL;
+    if (threadIdx.x < NW) shown = *(volatile unsigned long long*)&slot[threadIdx.x];
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int q = 0; q < NW; q++) s_act[threadIdx.x >> 5][q] = mine.w[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < NW) {
+        unsigned long long a = 0ULL;
+#pragma unroll
+        for (int w = 0; w < THREADS / 32; w++) a |= s_act[w][threadIdx.x];
+        if (a & ~shown) atomicOr(&slot[threadIdx.x], a);
+    }
+}
+
 template <int NW>
 __global__ void __launch_bounds__(THREADS)
 k_msbfs_all(PathArgs p)
@@ -43,73 +83,88 @@ k_msbfs_all(PathArgs p)
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long nt = (long long)gridDim.x * blockDim.x;
     const int gw = (int)(tid >> 5), nw = (int)(nt >> 5);
-    Words<NW>* front = (Words<NW>*)p.front;
-    Words<NW>* next = (Words<NW>*)p.next;
-    Words<NW>* seen_a = (Words<NW>*)p.seen_a;
-    Words<NW>* seen_b = (Words<NW>*)p.seen_b;
+    Words<NW>*cur = (Words<NW>*)p.front, *nxt = (Words<NW>*)p.next;
     constexpr int SRC = 64 * NW;
     int diam = 0;
     for (int s0 = 0; s0 < n; s0 += SRC) {
         const int ns = min(SRC, n - s0);
-        Words<NW> full;
-#pragma unroll
-        for (int q = 0; q < NW; q++) {
-            const int c = max(0, min(64, ns - q * 64));
-            full.w[q] = c == 64 ? ~0ULL : (c ? ((1ULL << c) - 1ULL) : 0ULL);
-        }
         // level 1 by push: the batch's sources OR their bit into their
-        // neighbours' frontier words (a pull sweep would read every edge)
-        for (int v = (int)tid; v < n; v += (int)nt) {
-            Words<NW> f, z;
-#pragma unroll
-            for (int q = 0; q < NW; q++) f.w[q] = z.w[q] = 0ULL;
-            const int b = v - s0;
-            if (b >= 0 && b < ns) f.w[b >> 6] = 1ULL << (b & 63);
-            front[v] = z;
-            seen_a[v] = f;
-        }
-        if (tid == 0) p.flags[0] = p.flags[1] = p.flags[2] = 0;
-        grid.sync();
+        // neighbours' frontier words (a pull sweep would read every edge).
+        // `cur` is all zero: cleared before the launch, then left so by the
+        // last level of each batch, which finds nothing.
+        if (tid < 3 * NW) p.active[tid] = 0ULL;
         for (int b = gw; b < ns; b += nw) {
             const int src = s0 + b;
             const unsigned long long bit = 1ULL << (b & 63);
-            for (int32_t q = p.R[src] + lane; q < p.R[src + 1]; q += 32) atomicOr(&front[p.C[q]].w[b >> 6], bit);
+            for (int32_t q = p.R[src] + lane; q < p.R[src + 1]; q += 32) atomicOr(&cur[p.C[q]].w[b >> 6], bit);
         }
         grid.sync();
-        {
-            unsigned long long found_total = 0;
-            for (int v = (int)tid; v < n; v += (int)nt) {
-                const Words<NW> f = front[v], sv = seen_a[v];
-                Words<NW> so;
-                int cnt = 0;
-#pragma unroll
-                for (int q = 0; q < NW; q++) {
-                    so.w[q] = sv.w[q] | f.w[q];
-                    cnt += __popcll(f.w[q]);
-                }
-                seen_b[v] = so;
-                if (cnt) p.cnt[(long long)v * MAX_D] += (unsigned)cnt;
-                found_total += (unsigned)cnt;
-            }
-            for (int o = 16; o; o >>= 1) found_total += __shfl_xor_sync(0xffffffffu, found_total, o);
-            if (lane == 0 && found_total && p.hist && 1 <= p.max_hop) atomicAdd(&p.hist[1], found_total);
-            // one store per CTA: a store per warp to the same flag serialised in L2
-            if (__syncthreads_or(found_total != 0) && threadIdx.x == 0) p.flags[1] = 1;
-        }
-        grid.sync();
-        if (tid == 0) p.flags[0] = 0;
-        if (!((volatile int*)p.flags)[1]) continue;   // no source has a neighbour
-        diam = max(diam, 1);
-        Words<NW>*sin = seen_b, *sout = seen_a, *cur = front, *nxt = next;
+        Words<NW>*sin = (Words<NW>*)p.seen_a, *sout = (Words<NW>*)p.seen_b;
         for (int d = 2;; d++) {
+            // Sources that grew at level d - 1 (level 1: those with a
+            // neighbour).  The others, isolated or done, find nothing any more
+            // and would keep every node scanning its whole row for them; with
+            // this and one barrier instead of three before level 2, 40,009
+            // nodes / 8.0M entries (a few of them isolated) take 20.0 ms, not
+            // 38.7.  Bound by the L2 reads of the frontier words (two full
+            // levels of 36 bytes per entry and 256 sources, 4.9 TB/s).
+            // (Read once per CTA: every warp reading one L2 sector took 4 us a
+            // level.)
+            __shared__ unsigned long long s_want[NW];
+            if (d == 2) {
+                for (int b = threadIdx.x; b < SRC; b += THREADS) {
+                    const bool has = b < ns && p.R[s0 + b + 1] > p.R[s0 + b];
+                    const unsigned m = __ballot_sync(0xffffffffu, has);
+                    if (lane == 0) ((unsigned*)s_want)[b >> 5] = m;
+                }
+            } else if (threadIdx.x < NW) {
+                s_want[threadIdx.x] = ((volatile unsigned long long*)p.active)[((d - 1) % 3) * NW + threadIdx.x];
+            }
+            __syncthreads();
+            Words<NW> want;
+            bool live = false;
+#pragma unroll
+            for (int q = 0; q < NW; q++) {
+                want.w[q] = s_want[q];
+                live |= want.w[q] != 0ULL;
+            }
+            if (!live) break;
+            diam = max(diam, d - 1);
             unsigned long long found_total = 0;
+            if (d == 2) {   // count level 1, a thread per node
+                for (int v = (int)tid; v < n; v += (int)nt) {
+                    const Words<NW> f = cur[v];
+                    int first = 0;
+#pragma unroll
+                    for (int q = 0; q < NW; q++) first += __popcll(f.w[q]);
+                    if (first) p.cnt[(long long)v * MAX_D] += (unsigned)first;
+                    found_total += (unsigned)first;
+                }
+                if (p.hist && 1 <= p.max_hop) {
+                    for (int o = 16; o; o >>= 1) found_total += __shfl_xor_sync(0xffffffffu, found_total, o);
+                    if (lane == 0 && found_total) atomicAdd(&p.hist[1], found_total);
+                }
+                found_total = 0;
+            }
+            Words<NW> grew;
+#pragma unroll
+            for (int q = 0; q < NW; q++) grew.w[q] = 0ULL;
             for (int v = gw; v < n; v += nw) {
-                const Words<NW> sv = sin[v];
+                Words<NW> sv;
+                if (d == 2) {
+                    sv = cur[v];   // seen so far: what was pushed, and itself
+                    const int b = v - s0;
+#pragma unroll
+                    for (int q = 0; q < NW; q++)
+                        if (b >= 64 * q && b < min(ns, 64 * q + 64)) sv.w[q] |= 1ULL << (b & 63);
+                } else {
+                    sv = sin[v];
+                }
                 Words<NW> need, acc;
                 bool any_need = false;
 #pragma unroll
                 for (int q = 0; q < NW; q++) {
-                    need.w[q] = full.w[q] & ~sv.w[q];
+                    need.w[q] = want.w[q] & ~sv.w[q];
                     any_need |= need.w[q] != 0ULL;
                     acc.w[q] = 0ULL;
                 }
@@ -123,11 +178,7 @@ k_msbfs_all(PathArgs p)
 #pragma unroll
                         for (int c = 0; c < 4; c++) {
                             const int32_t f = base + c * 32 + lane;
-                            if (f < e) {
-                                const Words<NW> fu = cur[p.C[f]];
-#pragma unroll
-                                for (int q = 0; q < NW; q++) acc.w[q] |= fu.w[q];
-                            }
+                            if (f < e) or_words<NW>(acc, cur + p.C[f]);
                         }
                         bool done = true;
 #pragma unroll
@@ -146,6 +197,7 @@ k_msbfs_all(PathArgs p)
                 for (int q = 0; q < NW; q++) {
                     nx.w[q] = acc.w[q] & need.w[q];
                     so.w[q] = sv.w[q] | nx.w[q];
+                    grew.w[q] |= nx.w[q];
                     cnt += __popcll(nx.w[q]);
                 }
                 if (lane == 0) {
@@ -159,11 +211,10 @@ k_msbfs_all(PathArgs p)
                 found_total += (unsigned)cnt;
             }
             if (lane == 0 && found_total && p.hist && d <= p.max_hop) atomicAdd(&p.hist[d], found_total);
-            if (__syncthreads_or(found_total != 0) && threadIdx.x == 0) p.flags[d % 3] = 1;
+            publish_active<NW>(grew, p.active + (d % 3) * NW);
             grid.sync();
-            if (tid == 0) p.flags[(d + 2) % 3] = 0;   // last read before this barrier, next written after the next
-            if (!((volatile int*)p.flags)[d % 3]) break;
-            diam = max(diam, d);
+            // last read before this barrier, next written after the next
+            if (tid < NW) p.active[((d + 2) % 3) * NW + tid] = 0ULL;
             Words<NW>* t = sin; sin = sout; sout = t;
             t = cur; cur = nxt; nxt = t;
         }
@@ -249,7 +300,7 @@ pg_status paths_prepare(pg_ctx* ctx, const pg_graph* g, int max_hop, PathArgs* a
     PG_TRY(pg_wst(ctx, "bfs.inv", (size_t)n + 1, &a->inv));
     PG_TRY(pg_wst(ctx, "bfs.eff", (size_t)n + 1, &a->eff));
     PG_TRY(pg_wst(ctx, "bfs.hist", (size_t)max_hop + 2, &a->hist));
-    PG_TRY(pg_wst(ctx, "bfs.flags", 4, &a->flags));
+    PG_TRY(pg_wst(ctx, "bfs.active", 24, &a->active));
     PG_TRY(pg_wst(ctx, "bfs.diam", 1, &a->diameter));
     PG_TRY(pg_wst(ctx, "bfs.out", 2, &a->out));
     // launch shape: sources per batch x CTAs per SM, from the autotuner
@@ -259,7 +310,7 @@ pg_status paths_prepare(pg_ctx* ctx, const pg_graph* g, int max_hop, PathArgs* a
     for (int nw : {4, 8})
         for (int c : {2, 4, 8})
             if (c <= (nw == 8 ? cap8 : cap4)) cands.push_back({nw, c});
-    const std::string key = tune_key("msbfs", n, g->nnz);
+    const std::string key = tune_key("msbfs_active", n, g->nnz);
     TuneChoice best{4, std::min(4, cap4)};
     PG_TRY(tune_pick(ctx, key, cands, &best, [&](const TuneChoice& c) -> pg_status {
         a->nw = c.a;
@@ -278,6 +329,7 @@ pg_status paths_enqueue(pg_ctx* ctx, PathArgs* a)
     PG_CUDA(ctx, cudaMemsetAsync(a->inv_far, 0, sizeof(double) * ((size_t)n + 1), ctx->stream));
     PG_CUDA(ctx, cudaMemsetAsync(a->hist, 0, sizeof(unsigned long long) * ((size_t)a->max_hop + 2), ctx->stream));
     PG_CUDA(ctx, cudaMemsetAsync(a->diameter, 0, sizeof(int), ctx->stream));
+    PG_CUDA(ctx, cudaMemsetAsync(a->front, 0, ((size_t)n + 1) * a->nw * sizeof(unsigned long long), ctx->stream));
     if (n > 0) {
         if (a->nw == 8) PG_TRY(launch_all<8>(ctx, *a, a->ctas_per_sm));
         else PG_TRY(launch_all<4>(ctx, *a, a->ctas_per_sm));

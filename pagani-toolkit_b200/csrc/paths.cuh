@@ -18,7 +18,7 @@ struct PathArgs {
     double* inv;               // sum_s 1/d(s, v)
     float* eff;                // inv / (n - 1)
     unsigned long long* hist;  // ordered pairs per distance (d <= max_hop)
-    int* flags;                // "a source grew at level d" (three, rotating)
+    unsigned long long* active;   // sources that grew at level d (three sets of nw words, rotating)
     int* diameter;
     double* out;               // [0] sum of inv, [1] Lp = n(n-1) / sum
 };

@@ -199,3 +199,29 @@ def test_fw_team_batches(ctx, sizes):
         cp_or, m_or = O.onnela(R, C, V)
         np.testing.assert_allclose(cp, cp_or, rtol=2.0 ** -22)
         assert cpm == pytest.approx(m_or, rel=2.0 ** -22)
+
+
+# ---------------------------------------------------------------- hop paths
+@pytest.mark.parametrize("n", [1, 2, 64, 255, 257, 511, 513, 1030])
+@pytest.mark.parametrize("kind", ["islands", "edgeless", "chain", "random"])
+def test_hop_paths_batches(ctx, n, kind):
+    """Batches of 256 and 512 sources with isolated sources, batches that have
+    no edge at all between batches that do, and many levels."""
+    rng = np.random.default_rng(n)
+    if kind == "edgeless":
+        edges = []
+    elif kind == "chain":
+        edges = [(i, i + 1) for i in range(n - 1) if i % 97]
+    elif kind == "islands":       # nodes 256.. isolated but for a pair at the end
+        m = min(n, 200)
+        edges = [tuple(rng.integers(0, m, 2)) for _ in range(3 * m)] + ([(n - 2, n - 1)] if n > 1 else [])
+    else:
+        edges = [tuple(rng.integers(0, n, 2)) for _ in range(4 * n)]
+    R, C, _ = G.csr_from_edges(n, edges)
+    eff, inv, lp, hist, diam = ctx.paths(ctx.graph(R, C), max_hop=128)
+    inv_or, hist_or, lp_or, d_or = O.bfs_paths(R, C, max_hop=128)
+    assert np.array_equal(hist, hist_or) and diam == d_or
+    if d_or <= 64:                # farther distances are added as they are found
+        assert np.array_equal(inv, inv_or)
+    np.testing.assert_allclose(inv, inv_or, rtol=1e-13)
+    assert lp == pytest.approx(lp_or, rel=1e-12)
