@@ -27,6 +27,7 @@
 // v'.k for the next step together.  Reductions are FP64 in a fixed order, so
 // results are deterministic.
 #include "pg_internal.cuh"
+#include "tma.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <chrono>
@@ -47,12 +48,21 @@ constexpr size_t SMEM_CAP = 220 * 1024;        // dynamic shared memory of a tea
 constexpr long long MEDIUM_EDGES = 1LL << 22;  // at most this many edges: one team per group
 constexpr int CLUSTER = 16;                    // largest team (CTAs of one cluster)
 constexpr long long MIN_CTA_EDGES = 8192;      // a team CTA keeps at least this many edges
-constexpr long long ASYNC_CTA_EDGES = 24576;   // dependency-driven phase: edges per team CTA before doubling
+// Dependency-driven phase: a team doubles its CTAs while each keeps more than
+// nnz / ASYNC_SHARE edges of the whole graph, within the bounds.  A small graph
+// has few groups in flight and is bound by its chain of power steps, so its
+// teams are wide; a large one fills the SMs and is bound by the teams' total
+// work, which wide teams increase.  Measured (dependency-driven phase, 2048 /
+// 6144 / 24576 edges): 5,000 nodes 52 / 56 / 75 ms, 16,000 259 / 277 / 364 ms,
+// 30,000 389 / 378 / 417 ms, 58,000 914 / 881 / 861 ms.
+constexpr long long ASYNC_MIN_EDGES = 2048, ASYNC_MAX_EDGES = 24576, ASYNC_SHARE = 1500;
+constexpr int SMALL_TEAM_ROWS = 1024;          // dependency-driven phase: teams of 256 threads up to here
 constexpr int RESERVE_SMS = 4;                 // dependency-driven phase: SMs kept free of teams
 constexpr size_t POOL_STREAMS = 128;           // dependency-driven phase: streams made ahead
 // Per group results: lambda, it0, res0, it1, res1, subP, subN, shifted, and
 // the device clock (ns) when its team started and ended.
 constexpr int OUT_W = 10;
+constexpr int TEAM_TIMEOUT = -1;   // it0 of a team whose exchange gave up
 
 __device__ __forceinline__ double nm_clock()
 {
@@ -387,7 +397,7 @@ __device__ __forceinline__ void local_argmax(const double* v, int n, int tid, in
 // Per-warp partials of up to four sums, two buffers used alternately: a
 // buffer is written again only after another barrier that every warp reaches
 // once it has read the buffer.
-struct Partials {
+struct __align__(16) Partials {
     double warp[2][32][4];
 };
 
@@ -607,7 +617,7 @@ __host__ __device__ inline int pow2_at_least(int x)
 // Byte offsets of the shared-memory parts of one team CTA; the slices take
 // what is left.
 struct TeamLayout {
-    size_t rep, kd, oy, oprev, obg, oR, key, soff, cols, need_min;
+    size_t rep, kd, yx, oy, oprev, obg, oR, key, soff, cols, need_min;
 };
 
 __host__ __device__ inline size_t team_take(size_t& at, size_t bytes)
@@ -617,12 +627,29 @@ __host__ __device__ inline size_t team_take(size_t& at, size_t bytes)
     return o;
 }
 
-__host__ __device__ inline TeamLayout team_layout(int n, int nown)
+// Rows of y that a cluster exchanges through its shared memories (longer
+// vectors meet in global memory: their copies would take the room of the
+// slices).
+constexpr int PUSH_ROWS = 2048;
+
+__host__ __device__ inline bool team_push(int n, int nb) { return nb > 1 && n <= PUSH_ROWS; }
+
+// rows start at even indices: a bulk copy moves 16-byte units
+__host__ __device__ inline int team_first(const int32_t* R, int n, int rank, int nb)
+{
+    const int r = team_split(R, n, rank, nb);
+    return rank >= nb ? r : r & ~1;
+}
+
+__host__ __device__ inline TeamLayout team_layout(int n, int nown, int nb)
 {
     TeamLayout t;
     size_t at = 0;
     t.rep = team_take(at, (size_t)(n + 1) * 8);
     t.kd = team_take(at, (size_t)n * 4);                       // degrees, exact as float
+    // two vectors of y, at the same offset in every CTA of the team (before
+    // everything whose size depends on the CTA): peers copy into them
+    t.yx = team_take(at, team_push(n, nb) ? (size_t)((n + 1) & ~1) * 8 * 2 : 0);
     t.oy = team_take(at, (size_t)nown * 8);
     t.oprev = team_take(at, (size_t)nown * 8);
     t.obg = team_take(at, (size_t)nown * 8);
@@ -652,7 +679,69 @@ struct Team {
     const float* wv;      // weighted tool, as in Group
     long long wn;
     int wmode;
+    bool push;            // y is exchanged through shared memory (clusters, n <= PUSH_ROWS)
+    double* yx;           // two vectors of y, used alternately
+    int ystride;
+    int nb, rank;
 };
+
+// Shared state of the exchange: a full barrier per vector, and whether a wait
+// ran out.
+struct TeamX {
+    unsigned long long full[2];
+    int failed;
+};
+
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank)
+{
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+    return a;
+}
+
+// All rows of y (ybuf: own rows written by this CTA) reach every CTA of the
+// team: one bulk copy of the own rows into each other CTA's shared memory,
+// which counts its bytes on that CTA's barrier.  No barrier of the cluster is
+// needed: a CTA writes a vector again two steps later, after it has received
+// the step between from every CTA, each of which had then received this one
+// and finished reading it.  16 CTAs, 700 rows: 1200 cycles with the wait for
+// the slowest CTA, against 1200 for a cluster barrier behind stores to global
+// memory and 600 more to read them back (5,000 nodes: 43.7 -> 38.2 ms).
+__device__ __forceinline__ void team_exchange(const Team& tm, double* ybuf, TeamX& tx, int step)
+{
+    using namespace pg_tma;
+    unsigned long long* bar = &tx.full[step & 1];
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    const uint32_t own = (uint32_t)((tm.nown + 1) & ~1) * 8, all = (uint32_t)((tm.n + 1) & ~1) * 8;
+    if (threadIdx.x == 0) mbar_expect_tx(bar, all - own);
+    if ((int)threadIdx.x < tm.nb && (int)threadIdx.x != tm.rank && own)
+        asm volatile(
+            "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+            ::"r"(cluster_addr(smem_u32(ybuf + tm.r0), threadIdx.x)), "r"(smem_u32(ybuf + tm.r0)), "r"(own),
+            "r"(cluster_addr(smem_u32(bar), threadIdx.x))
+            : "memory");
+    const uint32_t parity = (uint32_t)(step >> 1) & 1u;
+    auto done = [&]() {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        return ok != 0;
+    };
+    if (!done()) {
+        const unsigned long long t0 = gtimer();
+        while (!done())
+            if (*(volatile int*)&tx.failed || gtimer() - t0 > WAIT_NS) {
+                *(volatile int*)&tx.failed = 1;
+                break;
+            }
+    }
+}
 
 // own rows of y = B v from the sliced matrix, written to ydst[own row]
 // (WM = 1: every term of a row times the weight at the row's position)
@@ -666,28 +755,31 @@ __device__ __forceinline__ void team_slices(const Team& tm, double* ydst, double
     for (int s = wid; s < tm.nslices; s += nwarp) {
         const int b = tm.soff[s], it = (tm.soff[s + 1] - b) >> 5;
         const uint16_t* __restrict__ cs = tm.cols + b + lane;
-        double w = 1.0;
-        if (WM == 1) {
-            const int slot = s * RPS + lane / L;
-            w = slot < tm.nown ? wpos(tm.wv, tm.wn, tm.r0 + (int)tm.perm[slot]) : 0.0;
-        }
+        // the row's own terms first: their dependent loads run beside the gathers
+        const int slot = s * RPS + lane / L;
+        const bool own = slot < tm.nown;
+        const int lp = own ? (int)tm.perm[slot] : 0, p = tm.r0 + lp;
+        const double w = WM == 1 && own ? wpos(tm.wv, tm.wn, p) : 1.0;
+        const double diag = c * (double)tm.kd[p] + (tm.obg[lp] - beta) * rep[p];
         double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int j = 0;
-        for (; j + 3 < it; j += 4) {
-            const int c0 = cs[32 * j], c1 = cs[32 * j + 32], c2 = cs[32 * j + 64], c3 = cs[32 * j + 96];
-            a0 += wterm<WM>(rep[c0], w);
-            a1 += wterm<WM>(rep[c1], w);
-            a2 += wterm<WM>(rep[c2], w);
-            a3 += wterm<WM>(rep[c3], w);
+        // eight gathers in flight; the last turn's missing ones read the
+        // sentinel instead of running one by one
+        for (int j = 0; j < it; j += 8) {
+            int q[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) q[k] = j + k < it ? cs[32 * (j + k)] : tm.n;
+            a0 += wterm<WM>(rep[q[0]], w);
+            a1 += wterm<WM>(rep[q[1]], w);
+            a2 += wterm<WM>(rep[q[2]], w);
+            a3 += wterm<WM>(rep[q[3]], w);
+            a0 += wterm<WM>(rep[q[4]], w);
+            a1 += wterm<WM>(rep[q[5]], w);
+            a2 += wterm<WM>(rep[q[6]], w);
+            a3 += wterm<WM>(rep[q[7]], w);
         }
-        for (; j < it; j++) a0 += wterm<WM>(rep[cs[32 * j]], w);
         double y = (a0 + a1) + (a2 + a3);
         for (int o = L / 2; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-        const int slot = s * RPS + lane / L;
-        if (sub == 0 && slot < tm.nown) {
-            const int lp = (int)tm.perm[slot], p = tm.r0 + lp;
-            ydst[lp] = y - (c * (double)tm.kd[p] + (tm.obg[lp] - beta) * rep[p]);
-        }
+        if (sub == 0 && own) ydst[lp] = y - diag;
     }
 }
 
@@ -762,6 +854,66 @@ __device__ __forceinline__ void team_spmv(const Team& tm, double* ydst, double c
     else team_spmv_w<2>(tm, ydst, c, beta, lane, wid, nwarp);
 }
 
+// x / d for the reciprocal r = 1 / d rounded to nearest: two Newton steps on
+// the quotient with exact remainders (P. Markstein, IBM J. Res. Dev. 34(1),
+// 1990).  The result is the correctly rounded quotient while nothing under-
+// or overflows (checked against the division operator on 6e10 pairs).
+__device__ __forceinline__ double div_by(double x, double d, double r)
+{
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-d, q, x), r, q);
+    return __fma_rn(__fma_rn(-d, q, x), r, q);
+}
+
+// Sums over the 8 or 16 warps of a team CTA, in a fixed order, for the two
+// reductions of a step.  A step of a small group is these sums: 64-bit
+// shuffles (two each, one per clock and SM over all warps) took 1280 of its
+// 4050 cycles when every warp reduced every value by itself twice.
+//
+// One value: a shuffle tree per warp, then every thread adds the warps'
+// partials from 16-byte shared loads.
+__device__ __forceinline__ double team_sum1(Partials& s, double x, int& ph)
+{
+    double* f = &s.warp[ph][0][0];
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) f[threadIdx.x >> 5] = x;
+    __syncthreads();
+    const double2* p = (const double2*)f;
+    const double2 a = p[0], b = p[1], c = p[2], d = p[3];
+    double t = ((a.x + a.y) + (b.x + b.y)) + ((c.x + c.y) + (d.x + d.y));
+    if (blockDim.x > 256) {
+        const double2 e = p[4], g = p[5], h = p[6], i = p[7];
+        t += ((e.x + e.y) + (g.x + g.y)) + ((h.x + h.y) + (i.x + i.y));
+    }
+    ph ^= 1;
+    return t;
+}
+
+// Three values in 6 shuffles (instead of 15): the halves of a warp exchange
+// what they do not keep, so that after two exchanges each group of eight
+// lanes holds one value; the warps' partials are folded the same way.
+__device__ __forceinline__ void team_sum3(Partials& s, double (&x)[3], int& ph)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double* f = &s.warp[ph][0][0];
+    const bool hi = lane & 16, up = lane & 8;
+    // lower half: x0, x1; upper half: x2 (and nothing)
+    const double g0 = __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 16);
+    const double g1 = __shfl_xor_sync(0xffffffffu, hi ? x[1] : 0.0, 16);
+    const double k0 = (hi ? x[2] : x[0]) + g0, k1 = (hi ? 0.0 : x[1]) + g1;
+    double v = (up ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up ? k0 : k1, 8);
+    for (int o = 4; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((lane & 7) == 0) f[(lane >> 3) * 32 + w] = v;   // value lane / 8
+    __syncthreads();
+    const int q = lane >> 3, r = lane & 7;
+    v = f[q * 32 + r];
+    if (nw > 8) v += f[q * 32 + 8 + r];
+    for (int o = 4; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int k = 0; k < 3; k++) x[k] = __shfl_sync(0xffffffffu, v, 8 * k);
+    ph ^= 1;
+}
+
 // first index of the largest |v| over the whole copy, computed by one CTA
 __device__ __forceinline__ int block_argmax_abs(Partials& s, const double* v, int n, int& ph)
 {
@@ -778,11 +930,55 @@ __device__ __forceinline__ int block_argmax_abs(Partials& s, const double* v, in
     return bi == 0x7fffffff ? 0 : bi;
 }
 
+// |y|, then v' = y / |y| into the copy, and this thread's shares of |v' - v|^2,
+// |v' + v|^2 and v'.k, for at most NPT entries per thread: y is read once, and
+// all loads and quotients of a thread are issued together, without a branch
+// per entry (entries past n read the sentinel and count 0).  The per-thread
+// sums run over p = tid, tid + nthr, ..., as the loops for longer vectors.
+template <int NPT>
+__device__ __forceinline__ double team_normalise(const Team& tm, const double* ybuf, double (&x3)[3], Partials& ps,
+                                                 int& ph)
+{
+    const int tid = threadIdx.x, nthr = blockDim.x, n = tm.n;
+    double yv[NPT], vold[NPT], kd[NPT], sq = 0.0;
+#pragma unroll
+    for (int k = 0; k < NPT; k++) {
+        const int p = tid + k * nthr;
+        yv[k] = p < n ? ybuf[p] : 0.0;
+        vold[k] = tm.rep[min(p, n)];
+        kd[k] = (double)tm.kd[min(p, n - 1)];
+    }
+#pragma unroll
+    for (int k = 0; k < NPT; k++) sq += yv[k] * yv[k];
+    const double vnorm = sqrt(team_sum1(ps, sq, ph));
+    const double rnorm = 1.0 / vnorm;
+    if (vnorm > 1e-140 && vnorm < 1e140) {   // quotients through the reciprocal
+#pragma unroll
+        for (int k = 0; k < NPT; k++) yv[k] = div_by(yv[k], vnorm, rnorm);
+    } else {
+#pragma unroll
+        for (int k = 0; k < NPT; k++) yv[k] = tid + k * nthr < n ? yv[k] / vnorm : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < NPT; k++) {
+        const int p = tid + k * nthr;
+        const double d1 = yv[k] - vold[k], d2 = yv[k] + vold[k];
+        x3[0] += d1 * d1;
+        x3[1] += d2 * d2;
+        x3[2] += yv[k] * kd[k];
+        if (p < n) {
+            if ((unsigned)(p - tm.r0) < (unsigned)tm.nown) tm.oprev[p - tm.r0] = vold[k];
+            tm.rep[p] = yv[k];
+        }
+    }
+    return vnorm;
+}
+
 // Lead_Vector (Modularity_CPU.cpp:224-298) for a team: the reference's
 // per-entry arithmetic, sums in a fixed order over all rows.
 template <class Kind, bool W>
 __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, double beta, double err_sq, int* iters,
-                                   double* resid, Partials& ps, int& ph)
+                                   double* resid, Partials& ps, int& ph, TeamX& tx, int& xstep)
 {
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, wid = tid >> 5, nwarp = nthr >> 5;
     const int n = tm.n;
@@ -796,54 +992,37 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
     double vk = x1[0];
     // |v' - v|^2 and |v' + v|^2; sqrt(e) > EPSILON exactly when e > err_sq
     double s1 = 1.0, s2 = 1.0, vnorm = 0.0;
+    const double dM = (double)M, rM = 1.0 / dM;
     int iter = 0, yb = 0;
     while (s1 > err_sq && s2 > err_sq && iter < MAX_ITER) {
-        const double c = vk * 0.5 / (double)M;   // vk / 2 / M, the same double
-        double* ybuf = Kind::kCluster ? (yb ? gg.v0 : gg.v) : tm.oy;
+        const double c = div_by(vk * 0.5, dM, rM);   // vk / 2 / M, the same double
+        const bool push = Kind::kCluster && tm.push;
+        double* ybuf = !Kind::kCluster ? tm.oy : push ? tm.yx + (xstep & 1) * tm.ystride : yb ? gg.v0 : gg.v;
         team_spmv<W>(tm, Kind::kCluster ? ybuf + tm.r0 : ybuf, c, beta, lane, wid, nwarp);
-        Kind::barrier();
+        if (push) team_exchange(tm, ybuf, tx, xstep++);
+        else Kind::barrier();
         double x3[3] = {0.0, 0.0, 0.0};
-        if (n <= TEAM_NPT * nthr) {
-            // at most TEAM_NPT entries per thread: y is loaded once, all loads
-            // and divisions of a thread issued together; the per-thread sums
-            // run over p = tid, tid + nthr, ... as in the loops below
-            double yv[TEAM_NPT];
-            x1[0] = 0.0;
-#pragma unroll
-            for (int k = 0; k < TEAM_NPT; k++) {
-                const int p = tid + k * nthr;
-                yv[k] = p < n ? ybuf[p] : 0.0;
-            }
-#pragma unroll
-            for (int k = 0; k < TEAM_NPT; k++)
-                if (tid + k * nthr < n) x1[0] += yv[k] * yv[k];
-            block_sum(ps, x1, ph);
-            vnorm = sqrt(x1[0]);
-#pragma unroll
-            for (int k = 0; k < TEAM_NPT; k++) {
-                const int p = tid + k * nthr;
-                if (p < n) {
-                    const double vold = tm.rep[p];
-                    const double vp = yv[k] / vnorm;
-                    const double d1 = vp - vold, d2 = vp + vold;
-                    x3[0] += d1 * d1;
-                    x3[1] += d2 * d2;
-                    x3[2] += vp * (double)tm.kd[p];
-                    if ((unsigned)(p - tm.r0) < (unsigned)tm.nown) tm.oprev[p - tm.r0] = vold;
-                    tm.rep[p] = vp;
-                }
-            }
+        const int npt = (n + nthr - 1) / nthr;   // entries per thread
+        if (npt <= 1) {
+            vnorm = team_normalise<1>(tm, ybuf, x3, ps, ph);
+        } else if (npt <= 2) {
+            vnorm = team_normalise<2>(tm, ybuf, x3, ps, ph);
+        } else if (npt <= 4) {
+            vnorm = team_normalise<4>(tm, ybuf, x3, ps, ph);
+        } else if (npt <= TEAM_NPT) {
+            vnorm = team_normalise<TEAM_NPT>(tm, ybuf, x3, ps, ph);
         } else {
             x1[0] = 0.0;
             for (int p = tid; p < n; p += nthr) {
                 const double y = ybuf[p];
                 x1[0] += y * y;
             }
-            block_sum(ps, x1, ph);
-            vnorm = sqrt(x1[0]);
+            vnorm = sqrt(team_sum1(ps, x1[0], ph));
+            const bool normal = vnorm > 1e-140 && vnorm < 1e140;
+            const double rnorm = 1.0 / vnorm;
             for (int p = tid; p < n; p += nthr) {
                 const double vold = tm.rep[p];
-                const double vp = ybuf[p] / vnorm;
+                const double vp = normal ? div_by(ybuf[p], vnorm, rnorm) : ybuf[p] / vnorm;
                 const double d1 = vp - vold, d2 = vp + vold;
                 x3[0] += d1 * d1;
                 x3[1] += d2 * d2;
@@ -852,7 +1031,7 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
                 tm.rep[p] = vp;
             }
         }
-        block_sum(ps, x3, ph);
+        team_sum3(ps, x3, ph);
         s1 = x3[0];
         s2 = x3[1];
         vk = x3[2];
@@ -990,11 +1169,11 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
     const Group gg = global_group(in, gi);
     Team tm;
     tm.n = gg.ng;
-    tm.r0 = team_split(gg.sR, tm.n, rank, nb);
-    const int r1 = team_split(gg.sR, tm.n, rank + 1, nb);
+    tm.r0 = team_first(gg.sR, tm.n, rank, nb);
+    const int r1 = team_first(gg.sR, tm.n, rank + 1, nb);
     tm.nown = r1 - tm.r0;
     const int e0 = gg.sR[tm.r0];
-    const TeamLayout t = team_layout(tm.n, tm.nown);
+    const TeamLayout t = team_layout(tm.n, tm.nown, nb);
     tm.rep = (double*)(sm + t.rep);
     float* kd = (float*)(sm + t.kd);
     tm.kd = kd;
@@ -1026,19 +1205,47 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
     tm.soff = soff;
     tm.gcols = gg.sC + e0;
     tm.L = tm.nslices > 0 ? sL : lanes_per_row(tm.nown, tm.nown > 0 ? (long long)tm.oR[tm.nown] : 0, blockDim.x);
+    tm.nb = nb;
+    tm.rank = rank;
+    // a CTA without rows would send nothing, and the others could overtake it
+    tm.push = Kind::kCluster && team_push(tm.n, nb) &&
+              __syncthreads_and((int)threadIdx.x >= nb || team_first(gg.sR, tm.n, threadIdx.x + 1, nb) >
+                                                              team_first(gg.sR, tm.n, threadIdx.x, nb));
+    tm.yx = (double*)(sm + t.yx);
+    tm.ystride = (tm.n + 1) & ~1;
+    __shared__ TeamX tx;
+    if (Kind::kCluster) {
+        if (threadIdx.x == 0) {
+            pg_tma::mbar_init(&tx.full[0], 1);
+            pg_tma::mbar_init(&tx.full[1], 1);
+            tx.failed = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        Kind::barrier();   // every barrier exists before the first copy arrives
+    }
+    int xstep = 0;
     // both passes of Sub_Partition
     int it0, it1 = 0, ph = 0;
     double res0, res1 = 0.0;
-    double lam = team_lead_vector<Kind, W>(tm, gg, in.M, 0.0, in.err_sq, &it0, &res0, ps, ph);
+    double lam = team_lead_vector<Kind, W>(tm, gg, in.M, 0.0, in.err_sq, &it0, &res0, ps, ph, tx, xstep);
     const double below = gg.ng > in.gpu_rule_above ? -LAMBDA : 0.0;
     const bool shifted = lam < below;
-    if (shifted) lam += team_lead_vector<Kind, W>(tm, gg, in.M, -lam, in.err_sq, &it1, &res1, ps, ph);
+    if (shifted) lam += team_lead_vector<Kind, W>(tm, gg, in.M, -lam, in.err_sq, &it1, &res1, ps, ph, tx, xstep);
     double x2[2] = {0.0, 0.0};
     for (int p = threadIdx.x; p < tm.n; p += blockDim.x) {
         x2[0] += tm.rep[p] > 0.0;
         x2[1] += tm.rep[p] <= 0.0;
     }
     block_sum(ps, x2, ph);
+    if (Kind::kCluster) {
+        // a wait of any CTA that ran out is reported by the first one
+        if (threadIdx.x == 0 && rank != 0 && tx.failed) {
+            const uint32_t a = cluster_addr(pg_tma::smem_u32(&tx.failed), 0);
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(1) : "memory");
+        }
+        Kind::barrier();
+        if (tx.failed) it0 = TEAM_TIMEOUT;
+    }
     double o[OUT_W] = {lam, (double)it0, res0, (double)it1, res1, x2[0], x2[1], (double)shifted, t_start, 0.0};
     if (rank == 0 && threadIdx.x == 0) {
         o[9] = nm_clock();
@@ -1450,8 +1657,8 @@ struct NmAsync {
         auto need = [&](int c) {
             size_t m = 0;
             for (int r = 0; r < c; r++) {
-                const int a = team_split(rel.data(), n, r, c), b = team_split(rel.data(), n, r + 1, c);
-                m = std::max(m, team_layout(n, b - a).need_min);
+                const int a = team_first(rel.data(), n, r, c), b = team_first(rel.data(), n, r + 1, c);
+                m = std::max(m, team_layout(n, b - a, c).need_min);
             }
             return m;
         };
@@ -1489,8 +1696,11 @@ struct NmAsync {
         const Inputs& in = nd.in;
         uint16_t* sl = nd.sl;
         const int* gl = iota + nd.gi;
+        // a small group's step is bound by its two block-wide sums, which
+        // cost half with half the warps (5,000 nodes: 51.5 -> 47.7 ms)
+        const int threads = nd.n <= SMALL_TEAM_ROWS ? TEAM_THREADS / 2 : TEAM_THREADS;
         if (nd.c == 1) {
-            k_solo<<<1, TEAM_THREADS, smem_cap, st>>>(gl, in, (int)smem_cap, sl);
+            k_solo<<<1, threads, smem_cap, st>>>(gl, in, (int)smem_cap, sl);
         } else {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
@@ -1499,7 +1709,7 @@ struct NmAsync {
             attr[0].val.clusterDim.y = 1;
             attr[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3((unsigned)nd.c);
-            cfg.blockDim = dim3(TEAM_THREADS);
+            cfg.blockDim = dim3(threads);
             cfg.dynamicSmemBytes = smem_cap;
             cfg.stream = st;
             cfg.attrs = attr;
@@ -1519,6 +1729,7 @@ struct NmAsync {
         inflight -= tree[t].c;
         std::memcpy(tree[t].out, hout + (size_t)OUT_W * t, sizeof tree[t].out);
         const double* o = tree[t].out;
+        if ((int)o[1] == TEAM_TIMEOUT) return pg_fail(ctx, PG_ERR_TIMEOUT, "modularity: a team's exchange timed out");
         const long long subP = (long long)o[5], subN = (long long)o[6];
         tree[t].split = o[0] > LAMBDA && subP > 1 && subN > 1;
         if (!tree[t].split) {
@@ -1822,7 +2033,8 @@ static pg_status newman_run(pg_ctx* ctx, const pg_graph* g, const float* wv, lon
     int async_lo = -1, label_bound = 0, async_groups = 0, chain_groups = 0;
     double chain_ms = 0.0, span_ms = 0.0, busy_ctas = 0.0;
     std::vector<int> ref_of;
-    const long long async_cta_edges = ASYNC_CTA_EDGES;
+    const long long async_cta_edges =
+        std::min(ASYNC_MAX_EDGES, std::max(ASYNC_MIN_EDGES, (long long)g->nnz / ASYNC_SHARE));
     auto now = [] { return std::chrono::steady_clock::now(); };
     auto ms_since = [&](std::chrono::steady_clock::time_point t0) {
         return std::chrono::duration<double, std::milli>(now() - t0).count();
@@ -1892,8 +2104,8 @@ static pg_status newman_run(pg_ctx* ctx, const pg_graph* g, const float* wv, lon
             for (int p = 0; p <= ng; p++) rel[p] = (int32_t)(hsoff[hgoff[q] + p] - heoff[q]);
             size_t need = 0;
             for (int r = 0; r < c; r++) {
-                const int a = team_split(rel.data(), ng, r, c), b = team_split(rel.data(), ng, r + 1, c);
-                need = std::max(need, team_layout(ng, b - a).need_min);
+                const int a = team_first(rel.data(), ng, r, c), b = team_first(rel.data(), ng, r + 1, c);
+                need = std::max(need, team_layout(ng, b - a, c).need_min);
             }
             return need;
         };
@@ -2168,7 +2380,11 @@ static pg_status newman_run(pg_ctx* ctx, const pg_graph* g, const float* wv, lon
         }
         t_small += ms_since(t0);
         PG_TRY(pg_d2h(ctx, hout.data(), out, sizeof(double) * G * OUT_W));
-        for (int q : team) it_small += (long long)(hout[(size_t)q * OUT_W + 1] + hout[(size_t)q * OUT_W + 3]);
+        for (int q : team) {
+            if ((int)hout[(size_t)q * OUT_W + 1] == TEAM_TIMEOUT)
+                return pg_fail(ctx, PG_ERR_TIMEOUT, "modularity: a team's exchange timed out");
+            it_small += (long long)(hout[(size_t)q * OUT_W + 1] + hout[(size_t)q * OUT_W + 3]);
+        }
         // ---- decisions in round order (labels exactly as the sequential reference)
         std::vector<int> hbase(G, -1);
         std::vector<double> hcoef(G, 0.0);

@@ -225,3 +225,32 @@ def test_hop_paths_batches(ctx, n, kind):
         assert np.array_equal(inv, inv_or)
     np.testing.assert_allclose(inv, inv_or, rtol=1e-13)
     assert lp == pytest.approx(lp_or, rel=1e-12)
+
+
+# ------------------------------------------------------------------- Newman
+@pytest.mark.parametrize("n,deg", [(64, 6), (257, 12), (1000, 40), (1025, 60), (2047, 50), (2049, 90), (4200, 30)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_newman_team_sizes(ctx, n, deg, weighted):
+    """Single CTAs, clusters that exchange y through shared memory (up to 2048
+    rows) and through global memory, 256 and 512 threads, hubs that leave CTAs
+    of a cluster without rows: labels of the sequential oracle."""
+    rng = np.random.default_rng(n + deg)
+    block = np.arange(n) * 5 // n
+    edges = []
+    for _ in range(n * deg // 2):
+        a = int(rng.integers(n))
+        b = int(rng.integers(n))
+        if block[a] == block[b] or rng.random() < 0.08:
+            edges.append((a, b))
+    if n == 257:
+        edges += [(0, i) for i in range(1, n)] + [(1, i) for i in range(2, n)]
+    w = [np.float32(x) for x in rng.uniform(0.3, 1.0, len(edges))]
+    R, C, V = G.csr_from_edges(n, edges, w)
+    if weighted:
+        labels, Q, nm = ctx.newman_weighted(ctx.graph(R, C, V))
+        lo, Qo, nmo = O.newman_weighted(R, C, V)
+    else:
+        labels, Q, nm = ctx.newman(ctx.graph(R, C))
+        lo, Qo, nmo, _ = O.newman(R, C)
+    assert nm == nmo and np.array_equal(labels, lo)
+    assert Q == pytest.approx(Qo, abs=1e-9)
