@@ -428,7 +428,13 @@ pg_status ms_prepare(pg_ctx* ctx, const pg_graph* g, uint64_t seed, int64_t atte
     int per_sm = 0;
     PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_rounds, MS_THREADS, 0));
     if (per_sm < 1) return pg_fail(ctx, PG_ERR_INTERNAL, "maslov: kernel does not fit an SM");
-    a->grid = ctx->sm_count * std::min(per_sm, 4);
+    // One attempt of a round per thread, up to four CTAs per SM (then two): a
+    // round is three phases of a few dependent memory accesses, so on small
+    // graphs its barriers are what it costs, and they grow with the CTAs.
+    // 221k edges (6,900 attempts a round): 9.97 ms with four CTAs per SM, 4.61
+    // with 27 CTAs (one 16-CTA cluster and its hardware barrier: 5.86); 1.3M
+    // edges 12.9 -> 8.8 ms; from 4M edges on it is the full grid.
+    a->grid = (int)std::max(1LL, std::min((long long)ctx->sm_count * std::min(per_sm, 4), (B + MS_THREADS - 1) / MS_THREADS));
     return PG_OK;
 }
 
