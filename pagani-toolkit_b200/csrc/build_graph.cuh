@@ -167,15 +167,18 @@ pg_status launch_gram_tc(pg_ctx* ctx, const ZOperands& z, int mode, const EpiPar
 bool gram_tc_supported(pg_ctx* ctx, const ZOperands& z);
 
 // Radix selection state (device): the m-th largest of n uint64 keys is found
-// 8 bits per pass from the top; `prefix` holds its bits when done.
+// from the top, 11 bits per pass; `prefix` holds its bits when done.
 struct SelState {
     unsigned long long prefix, mask;
-    long long m;         // rank still to find inside the current prefix
-    long long above;     // number of keys strictly above the final key
+    long long m;            // rank still to find among the keys that match the prefix
+    long long matching;     // keys that match the prefix (at the end: keys equal to the result)
+    long long listed;       // matching keys copied to the list
+    unsigned int finished;  // blocks of the pass that are done
+    int from_list;          // the passes read the list instead of all keys
 };
-// m-th largest (1-based) of n keys; hist is 256 device counters.
-pg_status pg_radix_select(pg_ctx* ctx, const unsigned long long* keys, long long n, long long m,
-                          SelState* st_dev, unsigned long long* hist);
+// m-th largest (1-based) of n keys: result in st_dev->prefix, keys equal to it
+// still to take in st_dev->m.
+pg_status pg_radix_select(pg_ctx* ctx, const unsigned long long* keys, long long n, long long m, SelState* st_dev);
 // FP64 z-score statistics of a device T x N series (k_zstats): mean and root
 // sum of squares per voxel, sd = 0 for zero-variance voxels, counted in *nz.
 pg_status pg_zstats(pg_ctx* ctx, const float* dbold, int N, int T, double* mu, double* sd, int* nz);

@@ -254,3 +254,18 @@ def test_newman_team_sizes(ctx, n, deg, weighted):
         lo, Qo, nmo, _ = O.newman(R, C)
     assert nm == nmo and np.array_equal(labels, lo)
     assert Q == pytest.approx(Qo, abs=1e-9)
+
+
+# ------------------------------------------------------------ FP64 Gram blocks
+@pytest.mark.parametrize("N,T", [(2, 1), (5, 3), (127, 15), (128, 16), (129, 17), (257, 33), (600, 64), (1000, 240)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_correlation_packed_blocks(ctx, N, T, weighted):
+    """Edges of the 128-voxel blocks and of the 16- and 4-sample steps, with a
+    flat voxel and a pair of duplicates: every float of the FP64 oracle."""
+    bold = synth.bold_series(N, T, 3, 40 + N + T)
+    if N > 4:
+        bold[:, 1] = 2.0
+        bold[:, 3] = bold[:, 0]
+    r = ctx.correlation_packed(bold, weighted=weighted)
+    z, _ = O.zscore(bold)
+    assert np.array_equal(r, O.corr_packed(z, weighted=weighted).astype(np.float32))
