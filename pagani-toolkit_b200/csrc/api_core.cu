@@ -4,6 +4,7 @@
 #include <cstring>
 #include <cstdlib>
 #include <algorithm>
+#include <thread>
 #include <cmath>
 #include <new>
 
@@ -272,6 +273,63 @@ pg_status pg_d2h(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
     return PG_OK;
 }
 
+// Large results go through pinned staging buffers, several host threads each
+// copying its own chunks out while the next ones arrive: the driver's own
+// staging is one thread, and most of its time goes into the first touch of the
+// caller's fresh pages (50 MB: 10.9 -> 2.9 ms with eight threads).  Below 8 MB
+// the threads cost what they bring, and pinned or managed memory takes the
+// direct copy.  Synchronous, on the context stream.
+constexpr size_t D2H_LARGE_BYTES = 8u << 20;
+pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
+{
+    constexpr size_t CHUNK = 2u << 20;
+    constexpr int MAX_THREADS = 8;
+    const int nt = std::min(MAX_THREADS, (int)std::thread::hardware_concurrency() / 2);
+    if (bytes < D2H_LARGE_BYTES || nt < 2) return pg_d2h(ctx, dst, src, bytes);
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, dst) != cudaSuccess) cudaGetLastError();
+    else if (pa.type != cudaMemoryTypeUnregistered) return pg_d2h(ctx, dst, src, bytes);
+    unsigned char* stage;
+    PG_TRY(pg_hwst(ctx, "d2h.stage", 2 * CHUNK * MAX_THREADS, &stage));
+    cudaError_t err[MAX_THREADS] = {};
+    // thread t copies chunks t, t + nt, ... through two buffers of its own
+    auto work = [&](int t) {
+        cudaError_t e = cudaSetDevice(ctx->device);
+        cudaEvent_t ev[2] = {};
+        for (int k = 0; k < 2 && e == cudaSuccess; k++) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+        unsigned char* buf[2] = {stage + 2 * CHUNK * t, stage + 2 * CHUNK * t + CHUNK};
+        auto fetch = [&](size_t at, int k) {
+            if (at >= bytes || e != cudaSuccess) return;
+            e = cudaMemcpyAsync(buf[k], (const unsigned char*)src + at, std::min(CHUNK, bytes - at),
+                                cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[k], ctx->stream);
+        };
+        const size_t step = CHUNK * (size_t)nt;
+        int k = 0;
+        fetch(CHUNK * (size_t)t, 0);
+        for (size_t at = CHUNK * (size_t)t; at < bytes && e == cudaSuccess; at += step, k ^= 1) {
+            fetch(at + step, k ^ 1);
+            const cudaError_t w = cudaEventSynchronize(ev[k]);
+            if (e == cudaSuccess) e = w;
+            if (e == cudaSuccess) memcpy((unsigned char*)dst + at, buf[k], std::min(CHUNK, bytes - at));
+        }
+        for (cudaEvent_t v : ev)
+            if (v) cudaEventDestroy(v);
+        err[t] = e;
+    };
+    std::thread threads[MAX_THREADS];
+    int started = 1;   // this thread is number 0
+    try {
+        for (; started < nt; started++) threads[started] = std::thread(work, started);
+    } catch (...) {    // no thread to be had: theirs are done here
+    }
+    work(0);
+    for (int t = 1; t < started; t++) threads[t].join();
+    for (int t = started; t < nt; t++) work(t);
+    for (int t = 0; t < nt; t++) PG_CUDA(ctx, err[t]);
+    return pg_synchronize(ctx);
+}
+
 pg_status pg_h2d(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
 {
     if (!bytes) return PG_OK;
@@ -356,6 +414,12 @@ extern "C" pg_status pg_graph_to_csr(pg_ctx* ctx, const pg_graph* g, int32_t* R,
 {
     if (!ctx || !g) return pg_fail(ctx, PG_ERR_INVALID, "pg_graph_to_csr: null argument");
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
+    if (!on_device && sizeof(int32_t) * (size_t)g->nnz >= D2H_LARGE_BYTES) {
+        if (R) PG_TRY(pg_d2h(ctx, R, g->R, sizeof(int32_t) * ((size_t)g->n + 1)));
+        if (C) PG_TRY(pg_d2h_large(ctx, C, g->C, sizeof(int32_t) * (size_t)g->nnz));
+        if (V && g->V) PG_TRY(pg_d2h_large(ctx, V, g->V, sizeof(float) * (size_t)g->nnz));
+        return PG_OK;
+    }
     cudaMemcpyKind k = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     if (R) PG_CUDA(ctx, cudaMemcpyAsync(R, g->R, sizeof(int32_t) * ((size_t)g->n + 1), k, ctx->stream));
     if (C && g->nnz) PG_CUDA(ctx, cudaMemcpyAsync(C, g->C, sizeof(int32_t) * (size_t)g->nnz, k, ctx->stream));

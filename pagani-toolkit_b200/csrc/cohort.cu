@@ -730,7 +730,7 @@ extern "C" pg_status pg_correlation_packed(pg_ctx* ctx, const float* bold, int32
         bool timed_out = false;
         PG_TRY(gram64_run<GRAM_PACKED>(ctx, N, T, a, &timed_out));
         if (timed_out) return pg_fail(ctx, PG_ERR_TIMEOUT, "correlation Gram: a pipeline wait timed out");
-        PG_TRY(pg_d2h(ctx, r_packed + first, buf, sizeof(float) * (size_t)elems));
+        PG_TRY(pg_d2h_large(ctx, r_packed + first, buf, sizeof(float) * (size_t)elems));
     }
     return PG_OK;
 }
@@ -858,7 +858,7 @@ extern "C" pg_status pg_cohort_packed(pg_ctx* ctx, pg_cohort* c, float* r_packed
         const long long off = row * N - row * (row + 1) / 2;
         k_cohort_packed<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(c->keys, N, c->nb, row, r1 - row, buf);
         PG_LAUNCHED(ctx);
-        PG_TRY(pg_d2h(ctx, r_packed + off, buf, sizeof(float) * (size_t)elems));
+        PG_TRY(pg_d2h_large(ctx, r_packed + off, buf, sizeof(float) * (size_t)elems));
         row = r1;
     }
     return PG_OK;

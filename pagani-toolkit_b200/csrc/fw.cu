@@ -653,7 +653,7 @@ extern "C" pg_status pg_fw_paths(pg_ctx* ctx, const pg_graph* g, float* dist, fl
         PG_TRY(pg_wst(ctx, "fw.out", (size_t)n * n + 1, &tmp));
         k_fw_copy_out<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(b.gs, b.D, tmp);
         PG_LAUNCHED(ctx);
-        PG_TRY(pg_d2h(ctx, dist, tmp, sizeof(float) * (size_t)n * n));
+        PG_TRY(pg_d2h_large(ctx, dist, tmp, sizeof(float) * (size_t)n * n));
     }
     if (eff) PG_TRY(pg_d2h(ctx, eff, b.eff, sizeof(float) * n));
     return PG_OK;

@@ -113,6 +113,8 @@ pg_status pg_stream_pool(pg_ctx* ctx, size_t count);
 // Copies between host and device on the context stream, synchronous.
 pg_status pg_d2h(pg_ctx* ctx, void* dst, const void* src, size_t bytes);
 pg_status pg_h2d(pg_ctx* ctx, void* dst, const void* src, size_t bytes);
+// pg_d2h for results of many megabytes, copied out by several host threads.
+pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes);
 
 // Creates a graph object that owns freshly allocated device arrays.
 pg_status pg_graph_alloc(pg_ctx* ctx, int32_t n, int64_t nnz, bool weighted, pg_graph** out);

@@ -269,3 +269,25 @@ def test_correlation_packed_blocks(ctx, N, T, weighted):
     r = ctx.correlation_packed(bold, weighted=weighted)
     z, _ = O.zscore(bold)
     assert np.array_equal(r, O.corr_packed(z, weighted=weighted).astype(np.float32))
+
+
+@pytest.mark.parametrize("N", [2049, 3001])
+def test_large_results_reach_the_host(ctx, N):
+    """Results above 8 MB (staged by several threads), ends that divide no
+    chunk, against a copy of the same data made on the device side."""
+    import ctypes as ct
+
+    import pagani
+    import torch
+    bold = synth.bold_series(N, 20, 3, N)
+    r = ctx.correlation_packed(bold)
+    z, _ = O.zscore(bold)
+    assert r.nbytes > 8 << 20 and np.array_equal(r, O.corr_packed(z).astype(np.float32))
+    g, _ = ctx.build_graph(bold, mode="r", value=-0.05, sign="signed", weighted=True)
+    R, C, V = g.to_csr()
+    assert C.nbytes > 8 << 20
+    dev = [torch.empty(len(x), dtype=t, device="cuda") for x, t in ((R, torch.int32), (C, torch.int32),
+                                                                   (V, torch.float32))]
+    ctx._check(pagani.lib().pg_graph_to_csr(ctx.h, g.h, *[ct.c_void_p(d.data_ptr()) for d in dev], 1))
+    for host, d in zip((R, C, V), dev):
+        assert np.array_equal(host, d.cpu().numpy())
