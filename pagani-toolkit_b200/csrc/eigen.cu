@@ -119,16 +119,24 @@ __device__ __forceinline__ void ec_rows(const EcArgs& a, const double* vb, const
             q1 = split[lp * (nblk + 1) + b + 1];
         }
         double s0 = 0.0, s1 = 0.0;
-        for (; q + L < q1; q += 2 * L) {
-            if (W) {
-                s0 = __dadd_rn(s0, __dmul_rn((double)a.V[q], vb[cols[q]]));
-                s1 = __dadd_rn(s1, __dmul_rn((double)a.V[q + L], vb[cols[q + L]]));
-            } else {
-                s0 += vb[cols[q]];
-                s1 += vb[cols[q + L]];
+        // Eight entries of the lane in flight (the columns and weights come
+        // from L2); even ones go to s0, odd ones to s1.  25,211 nodes / 6.4M
+        // weighted entries: 2.30 ms for 82 steps with two at a time, 2.09 now.
+        for (; q < q1; q += 8 * L) {
+            int col[8];
+            float w[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const bool in = q + k * L < q1;
+                col[k] = in ? cols[q + k * L] : -1;
+                if (W) w[k] = in ? a.V[q + k * L] : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k += 2) {
+                if (col[k] >= 0) s0 = W ? __dadd_rn(s0, __dmul_rn((double)w[k], vb[col[k]])) : s0 + vb[col[k]];
+                if (col[k + 1] >= 0) s1 = W ? __dadd_rn(s1, __dmul_rn((double)w[k + 1], vb[col[k + 1]])) : s1 + vb[col[k + 1]];
             }
         }
-        if (q < q1) s0 = W ? __dadd_rn(s0, __dmul_rn((double)a.V[q], vb[cols[q]])) : s0 + vb[cols[q]];
         double y = s0 + s1;
         for (int o = L / 2; o; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
         if (act && sub == 0) ypart[lp] = b == 0 ? y : ypart[lp] + y;
@@ -210,6 +218,7 @@ __global__ void __launch_bounds__(EC_THREADS, 1) k_ec(EcArgs a)
         for (int b = 0; b < nblk; b++) {
             const int len = min(cb, n - b * cb);
             const double* src = uc + (size_t)b * cb;
+#pragma unroll 8
             for (int p = tid; p < len; p += nthr) vblk[p] = src[p] * inv;
             __syncthreads();
             ec_block<W>(L, a, vblk, split, nblk, nown, ypart, b, lane, wid, nwarp);

@@ -291,3 +291,18 @@ def test_large_results_reach_the_host(ctx, N):
     ctx._check(pagani.lib().pg_graph_to_csr(ctx.h, g.h, *[ct.c_void_p(d.data_ptr()) for d in dev], 1))
     for host, d in zip((R, C, V), dev):
         assert np.array_equal(host, d.cpu().numpy())
+
+
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 65])
+def test_participation_module_counts(ctx, K):
+    """Module counts around a warp, rows shorter and longer than 32 entries,
+    isolated nodes: the oracle's floats."""
+    R, C, V = G.random_weighted(150, 0.4, K)
+    R2 = np.concatenate([R, [R[-1], R[-1]]]).astype(np.int32)      # two isolated nodes
+    mod = (np.random.default_rng(K).integers(1, K + 1, 152)).astype(np.float32)
+    mod[0] = K
+    for v in (V, None):
+        g = ctx.graph(R2, C, v)
+        pc, pn, k = ctx.participation(g, mod)
+        pc_or, pn_or, k_or = O.participation(R2, C, v, mod)
+        assert k == k_or and np.array_equal(pc, pc_or) and np.array_equal(pn, pn_or)
