@@ -461,7 +461,11 @@ pg_status launch_brandes(pg_ctx* ctx, BCArgs& a, int batch_first, int batch_last
     int per_sm = 0;
     PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_brandes, THREADS, 0));
     if (per_sm < 1) return pg_fail(ctx, PG_ERR_INTERNAL, "brandes kernel cannot be resident");
-    int grid = per_sm * ctx->sm_count;
+    // four CTAs per SM hide the latency of the gathers; below 8,192 nodes a
+    // level hands each warp of two CTAs per SM a few nodes at most, and the
+    // barriers between levels cost less (5,000 nodes: 12.5 -> 11.9 ms)
+    if (a.n < 8192) per_sm = std::min(per_sm, 2);
+    const int grid = per_sm * ctx->sm_count;
     void* args[] = {(void*)&a, (void*)&batch_first, (void*)&batch_last, (void*)&fwd_first, (void*)&fwd_last};
     const int prof = pg_prof_begin(ctx, "k_brandes");
     PG_CUDA(ctx, cudaLaunchCooperativeKernel((void*)k_brandes, dim3(grid), dim3(THREADS), args, 0, ctx->stream));
