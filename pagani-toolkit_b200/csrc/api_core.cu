@@ -278,7 +278,8 @@ pg_status pg_d2h(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
 // staging is one thread, and most of its time goes into the first touch of the
 // caller's fresh pages (50 MB: 10.9 -> 2.9 ms with eight threads).  Below 8 MB
 // the threads cost what they bring, and pinned or managed memory takes the
-// direct copy.  Synchronous, on the context stream.
+// direct copy, as does everything where the 32 MB of staging cannot be had.
+// Synchronous, on the context stream.
 constexpr size_t D2H_LARGE_BYTES = 8u << 20;
 pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
 {
@@ -290,7 +291,7 @@ pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
     if (cudaPointerGetAttributes(&pa, dst) != cudaSuccess) cudaGetLastError();
     else if (pa.type != cudaMemoryTypeUnregistered) return pg_d2h(ctx, dst, src, bytes);
     unsigned char* stage;
-    PG_TRY(pg_hwst(ctx, "d2h.stage", 2 * CHUNK * MAX_THREADS, &stage));
+    if (pg_hwst(ctx, "d2h.stage", 2 * CHUNK * MAX_THREADS, &stage) != PG_OK) return pg_d2h(ctx, dst, src, bytes);
     cudaError_t err[MAX_THREADS] = {};
     // thread t copies chunks t, t + nt, ... through two buffers of its own
     auto work = [&](int t) {

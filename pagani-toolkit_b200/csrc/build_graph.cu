@@ -1,7 +1,8 @@
 // build_graph.cu -- network construction (CUCorMat) on the device:
-//   z-score (FP64) -> Gram tiles with fused threshold epilogue (histogram
-//   pass, then emit pass) -> FP64 recheck of the guard band -> exact k-th
-//   key selection (sparsity mode) -> undirected pairs -> sorted CSR.
+//   z-score (FP64) -> Gram tiles with fused threshold epilogue (a sampled
+//   histogram and one full pass, or a histogram and an emit pass) -> FP64
+//   recheck of the guard band -> exact k-th key selection (sparsity mode) ->
+//   adjacency bits or undirected pairs -> sorted CSR.
 // The dense correlation matrix is never stored.
 #include "build_graph.cuh"
 #include <cmath>
@@ -799,9 +800,12 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     // passes over N^2 bits (0.45 ms at 58,000 nodes) beat the list's degree
     // count, scatter and sort (62 us per million edges): from 1.3e-3 N^2 edges
     // on, and always where every pair would be listed (at most 1 MB of bits).
-    // Weights need the list; the bits may take 8 GiB.
+    // Weights need the list; the bits may take 8 GiB, and where they cannot be
+    // had the (then smaller) list serves.
     auto bits_pay = [&](long long edges) {
-        return !weighted && bit_bytes <= (8ULL << 30) && (list_all || (double)edges >= 1.3e-3 * (double)N * (double)N);
+        return !weighted && bit_bytes <= (8ULL << 30) &&
+               (list_all || (double)edges >= 1.3e-3 * (double)N * (double)N) &&
+               pg_wst(ctx, "b.bits", (size_t)N * bit_words, &bits) == PG_OK;
     };
     // room for the decided edges (cap_total with the band's)
     auto prepare_decided = [&]() -> pg_status {

@@ -350,13 +350,14 @@ pg_status onnela_prepare(pg_ctx* ctx, const pg_graph* g, int first_n, float* cp_
     if (a->smem_general > ctx->smem_optin - 4096)
         return pg_fail(ctx, PG_ERR_TOO_LARGE, "Onnela: n=%d too large", g->n);
     // the table of k_onnela takes twice the bitmap's shared memory, beside the
-    // row's roots: graphs beyond it (about 850,000 nodes) take the general kernel
+    // row's roots: graphs beyond it (about 850,000 nodes) take the general
+    // kernel, and so do those whose table of roots finds no memory
     a->smem = words * 8;
     a->fast = a->smem + ONNELA_ROW * 8 + 1024 <= ctx->smem_optin;
     PG_TRY(pg_wst(ctx, "on.state", 1, &a->state));
     if (a->fast) {
-        PG_TRY(pg_wst(ctx, "on.roots", (size_t)g->nnz, &a->roots));
-        PG_TRY(pg_wst(ctx, "on.up", (size_t)g->n, &a->up));
+        a->fast = pg_wst(ctx, "on.roots", (size_t)g->nnz, &a->roots) == PG_OK &&
+                  pg_wst(ctx, "on.up", (size_t)g->n, &a->up) == PG_OK;
         if (a->smem + ONNELA_ROW * 8 > 48 * 1024 - 1024)
             PG_CUDA(ctx, cudaFuncSetAttribute(k_onnela, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a->smem));
     }

@@ -562,9 +562,10 @@ __device__ void sub_partition(const Group& g, const Inputs& in, int gi, Red& red
 // A team is one CTA, or a thread-block cluster of up to 16 CTAs, that owns
 // one group.  Every CTA keeps the whole vector of the group in shared memory
 // (plus a zero sentinel at index n) and computes y = B v for an
-// edge-balanced range of own rows.  A cluster CTA publishes its rows of y in
-// global memory (two buffers used alternately) and, after one cluster barrier
-// per step, reads all of y back; then every CTA normalises the whole vector
+// edge-balanced range of own rows.  A cluster CTA copies its rows of y into
+// every other CTA's shared memory (up to PUSH_ROWS rows), or publishes them in
+// global memory and, after one cluster barrier per step, reads all of y back
+// (two buffers used alternately either way); then every CTA normalises the whole vector
 // and forms |y|, |v' -+ v| and v'.k itself, over all rows in one fixed order.
 // All CTAs of a team therefore hold bit-identical vectors and sums and take
 // the same decisions, with no reduction across CTAs.
