@@ -180,8 +180,11 @@ class _Quiet:
 
 
 def cpu_baseline(n_sample=4000, threads=None):
-    with _Quiet():
-        return _cpu_baseline(n_sample, threads)
+    try:
+        with _Quiet():
+            return _cpu_baseline(n_sample, threads)
+    except FileNotFoundError as e:    # oracle/_ref is built from the reference's sources
+        return {"unavailable": f"the reference's CPU code is not built here ({os.path.basename(str(e).split()[0])})"}
 
 
 def _cpu_stage_times(ref, O, synth, n, threads):
@@ -257,7 +260,10 @@ def run_reference(args, rank, world):
     if rank != 0:
         return
     for _ in range(args.warmup):
-        cpu_baseline()
+        first = cpu_baseline()
+        if "unavailable" in first:
+            print(json.dumps({"impl": "reference", "unavailable": first["unavailable"]}), flush=True)
+            return
     vals = []
     t0 = time.perf_counter()
     for _ in range(args.steps):
