@@ -13,14 +13,16 @@
 // being swept stay in L2 and a barrier has only the team's arrivals:
 //   A  the team's rows: +inf, 0 on the diagonal, 1/w for the edges;
 //   then for every 64-wide k-block round kb:
-//   1  the row and column panels: the min-plus product with the closed
-//      diagonal block (its diagonal is 0, so the product keeps the panel);
+//   1  the row and column panels, closed in place against the closed diagonal
+//      block (64 steps in order, eight at a time);
 //   2  every other block: d_ij = min(d_ij, d_i,kb (x) d_kb,j); the diagonal
 //      block of the next round comes first and is closed at once (64 steps in
 //      registers), so no phase of its own waits for it;
 //   C  per-row sums of 1/d (CUBFW_Lp.cpp:77-104);
 // and at the end, per graph, Lp and the mean clustering.  The k-block width
-// is fixed (64), so the distances depend neither on the teams nor on the grid.
+// is fixed (64), every block is closed in the same order of steps and the
+// per-graph sums run over the nodes in order, so no result depends on the
+// teams or on the grid.
 #include "pg_internal.cuh"
 #include <algorithm>
 #include <cmath>
@@ -196,6 +198,11 @@ struct __align__(16) FwSmem {
             float2 b[B / 2][B];     // right operand, rows k and k + 1 interleaved: b[k / 2][j]
         } prod;
         struct {
+            float dg[B][B + 4];     // the closed diagonal block (transposed for a column panel)
+            float rows[2][8][B];    // the eight rows whose steps come next
+            float tr[B][B + 1];     // for turning a column panel
+        } panel;
+        struct {
             float row[2][B];        // row k of the block being closed
             float col[2][B];        // column k
         } close;
@@ -226,6 +233,20 @@ struct Tile {
             *(float2*)(dst + (long long)(i0 + 8 * r) * ld + j) = make_float2(v[r][0], v[r][1]);
             *(float2*)(dst + (long long)(i0 + 8 * r) * ld + j + 32) = make_float2(v[r][2], v[r][3]);
         }
+    }
+    // the block's transpose (no bank is hit twice by a warp, either way)
+    __device__ __forceinline__ void transpose(float (*tr)[B + 1])
+    {
+        const int i0 = group_thread() >> 4, j = 2 * (group_thread() & 15);
+#pragma unroll
+        for (int r = 0; r < TR; r++)
+#pragma unroll
+            for (int x = 0; x < 4; x++) tr[i0 + 8 * r][j + (x & 1) + 16 * (x & 2)] = v[r][x];
+        group_sync();
+#pragma unroll
+        for (int r = 0; r < TR; r++)
+#pragma unroll
+            for (int x = 0; x < 4; x++) v[r][x] = tr[j + (x & 1) + 16 * (x & 2)][i0 + 8 * r];
     }
 };
 
@@ -281,6 +302,95 @@ __device__ __forceinline__ void min_plus(FwSmem& sm, Tile& c, const float* a, co
         }
     }
     group_sync();   // the operands are overwritten next
+}
+
+// A panel block closed against the closed diagonal block dg, in place: step k
+// is s_ij = min(s_ij, dg_ik + s_kj) in a row panel, and the same of the
+// transposed blocks in a column panel.  The steps' order is part of the
+// result: a product with the untouched panel is as exact, but it associates
+// the FP32 sums of paths of three and more edges the other way round, which
+// moves distances by their last bit.
+// Eight steps at a time, with one barrier: every thread takes the eight rows
+// s_k.. of its four columns from shared memory, brings them to their own steps
+// (a triangle of updates, done by all eight owners of a column alike), and
+// folds them into its tile as min_plus does.  The minima are exact, so this
+// equals the 64 steps, which took a barrier each (2,500 nodes: 2.02 ms, with
+// the panels as plain products 1.85, with 64 barriers a panel 2.82).
+__device__ __forceinline__ void close_panel(FwSmem& sm, Tile& c, const float* dg, float* d, int ld, bool row, int kn)
+{
+    const int t = group_thread(), i0 = t >> 4, j0 = 2 * (t & 15);
+    c.load(d, ld);
+#pragma unroll
+    for (int it = 0; it < B * B / 4 / GT; it++) {
+        const int q = t + it * GT;
+        if (row) {
+            const int i = q >> 4, j = (q & 15) << 2;
+            *(float4*)&sm.panel.dg[i][j] = *(const float4*)(dg + (long long)i * ld + j);
+        } else {   // a warp stores 32 consecutive words
+            const int i = q & (B - 1), j = (q >> 6) << 2;
+            const float4 x = *(const float4*)(dg + (long long)i * ld + j);
+            sm.panel.dg[j][i] = x.x;
+            sm.panel.dg[j + 1][i] = x.y;
+            sm.panel.dg[j + 2][i] = x.z;
+            sm.panel.dg[j + 3][i] = x.w;
+        }
+    }
+    if (!row) c.transpose(sm.panel.tr);
+#pragma unroll 1
+    for (int k0 = 0; k0 < kn; k0 += 8) {
+        float (*buf)[B] = sm.panel.rows[(k0 >> 3) & 1];
+        float own[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+            own[x] = c.v[0][x];
+#pragma unroll
+            for (int r = 1; r < TR; r++) own[x] = k0 == 8 * r ? c.v[r][x] : own[x];
+        }
+        *(float2*)&buf[i0][j0] = make_float2(own[0], own[1]);
+        *(float2*)&buf[i0][j0 + 32] = make_float2(own[2], own[3]);
+        group_sync();   // the other buffer is written next, this one after another barrier
+        float2 b[4][4];   // rows k0 + 2 h, + 1 of the thread's columns
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            const float2 x = *(const float2*)&buf[2 * h][j0], y = *(const float2*)&buf[2 * h + 1][j0];
+            const float2 z = *(const float2*)&buf[2 * h][j0 + 32], w = *(const float2*)&buf[2 * h + 1][j0 + 32];
+            b[h][0] = make_float2(x.x, y.x);
+            b[h][1] = make_float2(x.y, y.y);
+            b[h][2] = make_float2(z.x, w.x);
+            b[h][3] = make_float2(z.y, w.y);
+        }
+        // the rows at their own steps
+#pragma unroll
+        for (int k = 1; k < 8; k++) {
+            const float4 lo = *(const float4*)&sm.panel.dg[k0 + k][k0], hi = *(const float4*)&sm.panel.dg[k0 + k][k0 + 4];
+            const float2 a[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                float& s = (k & 1) ? b[k / 2][x].y : b[k / 2][x].x;
+#pragma unroll
+                for (int h = 0; h < k / 2; h++) {
+                    const float2 p = add2(a[h], b[h][x]);
+                    s = min3f(s, p.x, p.y);
+                }
+                if (k & 1) s = fminf(s, a[k / 2].x + b[k / 2][x].x);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < TR; r++) {
+            const float4 lo = *(const float4*)&sm.panel.dg[i0 + 8 * r][k0], hi = *(const float4*)&sm.panel.dg[i0 + 8 * r][k0 + 4];
+            const float2 a[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+#pragma unroll
+            for (int h = 0; h < 4; h++)
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    const float2 p = add2(a[h], b[h][x]);
+                    c.v[r][x] = min3f(c.v[r][x], p.x, p.y);
+                }
+        }
+    }
+    if (!row) c.transpose(sm.panel.tr);
+    c.store(d, ld);
+    group_sync();   // shared memory is overwritten next
 }
 
 // Closure of a diagonal block held in registers: row k and column k do not
@@ -393,10 +503,7 @@ __device__ __forceinline__ void fw_graph(const FwBatch& p, const FWGraph& g, Tea
             const bool row = t < m;
             int other = row ? t : t - m;
             if (other >= kb) other++;
-            float* d = row ? blk(p.D, g, kb, other) : blk(p.D, g, other, kb);
-            c.load(d, g.np);
-            min_plus(sm, c, row ? dg : d, row ? d : dg, g.np, kn);
-            c.store(d, g.np);
+            close_panel(sm, c, dg, row ? blk(p.D, g, kb, other) : blk(p.D, g, other, kb), g.np, row, kn);
         }
         team.sync();
         // 2: the other blocks, the next round's diagonal block first
@@ -516,17 +623,19 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_fw_batch(FwBatch p)
         }
     }
     grid.sync();
-    // ---- a warp per graph: fixed strided sums and a shuffle tree
+    // ---- a warp per graph: sums over the nodes in order (reads 32 at a time)
     for (long long gi = gw; gi < p.ng; gi += nw) {
         const FWGraph g = p.gs[gi];
         double t = 0.0, m = 0.0;
-        for (int u = lane; u < g.n; u += 32) {
-            t += p.rowsum[g.node0 + u];
-            if (p.onnela) m += (double)p.cp[g.out0 + u];
-        }
-        for (int o = 16; o; o >>= 1) {
-            t += __shfl_xor_sync(0xffffffffu, t, o);
-            m += __shfl_xor_sync(0xffffffffu, m, o);
+        for (int u0 = 0; u0 < g.n; u0 += 32) {
+            const bool in = u0 + lane < g.n;
+            const double x = in ? p.rowsum[g.node0 + u0 + lane] : 0.0;
+            const float y = in && p.onnela ? p.cp[g.out0 + u0 + lane] : 0.0f;
+            const int cnt = min(32, g.n - u0);
+            for (int k = 0; k < cnt; k++) {
+                t += __shfl_sync(0xffffffffu, x, k);
+                m += (double)__shfl_sync(0xffffffffu, y, k);
+            }
         }
         if (lane == 0) {
             p.lp[g.index] = t > 0.0 ? 1.0 / (t / g.n / (g.n - 1)) : INFINITY;
