@@ -196,6 +196,13 @@ extern "C" pg_status pg_debug_stall_next_gram(pg_ctx* ctx, uint64_t wait_ns)
     return PG_OK;
 }
 
+extern "C" pg_status pg_debug_stall_next_team(pg_ctx* ctx, uint64_t wait_ns)
+{
+    if (!ctx) return PG_ERR_INVALID;
+    ctx->debug_team_stall_ns = wait_ns;
+    return PG_OK;
+}
+
 // --------------------------------------------------------------- workspace
 pg_status pg_ws(pg_ctx* ctx, const char* key, size_t bytes, void** out)
 {

@@ -75,6 +75,8 @@ struct FwBatch {
     double* cw;                 // per entry of every graph: (V / vmax)^(1/3)
     int32_t* up;                // per node: where the entries of its row with a column above it begin
     int onnela;                 // compute the clustering
+    unsigned max_spins;         // reads of the counter that a team barrier waits for
+    int hold;                   // failure-path test hook: a CTA of every team does not arrive
     double* rowsum;             // per node, in processing order
     float* eff;                 // per node, in the caller's order
     double* lp;                 // per graph, in the caller's order; then 1.0 after a timeout
@@ -433,27 +435,43 @@ __device__ __forceinline__ void close_block(FwSmem& sm, Tile& c)
 // Barrier of a team's CTAs (all resident: the launch is cooperative).  The
 // wait is bounded; after a timeout nobody waits any more and the host reports
 // an error.
+constexpr unsigned MAX_SPINS = 1u << 27;
 struct Team {
     unsigned* arrived;
     int* timeout;
-    unsigned size, target;
+    unsigned size, target, max_spins;
+    bool hold;          // test hook: this CTA's first arrival waits for a peer to give up
     __device__ void sync()
     {
         __syncthreads();
         target += size;
         if (threadIdx.x == 0) {
+            if (hold)
+                for (unsigned spins = 0; spins < MAX_SPINS && !*(volatile int*)timeout; spins++) {}
             __threadfence();
             atomicAdd(arrived, 1u);
             volatile unsigned* seen = arrived;
             for (unsigned spins = 0; *seen < target; spins++) {
-                if (spins > (1u << 27) || *(volatile int*)timeout) {
+                if (spins > max_spins || *(volatile int*)timeout) {
                     atomicExch(timeout, 1);
                     break;
                 }
             }
             __threadfence();
         }
+        hold = false;
         __syncthreads();
+    }
+    // The barrier, then the graph that the team's first CTA took, or -1 after
+    // a timeout.  One thread reads both for its CTA: another team may raise
+    // the timeout between two reads, and a CTA whose threads saw different
+    // values would leave some of them in the sweep and the others behind it.
+    __device__ int sync_graph(const int* graph, int& shared_slot)
+    {
+        sync();
+        if (threadIdx.x == 0) shared_slot = *(volatile int*)timeout ? -1 : *(volatile const int*)graph;
+        __syncthreads();
+        return shared_slot;   // written again only behind the next barrier
     }
 };
 
@@ -612,12 +630,13 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_fw_batch(FwBatch p)
         const int n_cta = gridDim.x, t = (int)((long long)blockIdx.x * p.teams / n_cta);
         const int first = (int)(((long long)t * n_cta + p.teams - 1) / p.teams);
         const int end = (int)(((long long)(t + 1) * n_cta + p.teams - 1) / p.teams);
-        Team team{&p.ctl->arrived[t], &p.ctl->timeout, (unsigned)(end - first), 0u};
+        Team team{&p.ctl->arrived[t], &p.ctl->timeout, (unsigned)(end - first), 0u, p.max_spins,
+                  p.hold && end - first > 1 && blockIdx.x == end - 1};
+        __shared__ int s_graph;
         for (;;) {
             if (blockIdx.x == first && threadIdx.x == 0) *(volatile int*)&p.ctl->graph[t] = atomicAdd(&p.ctl->queue, 1);
-            team.sync();
-            const int gi = *(volatile int*)&p.ctl->graph[t];
-            if (gi >= p.ng || *(volatile int*)&p.ctl->timeout) break;
+            const int gi = team.sync_graph(&p.ctl->graph[t], s_graph);
+            if (gi < 0 || gi >= p.ng) break;
             const FWGraph g = p.gs[gi];
             fw_graph(p, g, team, sm, grp * (end - first) + (blockIdx.x - first), GROUPS * (end - first));
         }
@@ -717,8 +736,13 @@ static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, boo
     return PG_OK;
 }
 
-static pg_status fw_launch(pg_ctx* ctx, const FwBatch& b)
+static pg_status fw_launch(pg_ctx* ctx, FwBatch b)
 {
+    // a pending failure-path test stall applies to this launch only (a read of
+    // the counter takes about half a microsecond)
+    b.hold = ctx->debug_team_stall_ns != 0;
+    b.max_spins = b.hold ? (unsigned)std::min<unsigned long long>(ctx->debug_team_stall_ns / 500, MAX_SPINS) : MAX_SPINS;
+    ctx->debug_team_stall_ns = 0;
     PG_CUDA(ctx, cudaMemsetAsync(b.ctl, 0, sizeof(FwControl), ctx->stream));
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeCooperative;

@@ -40,6 +40,9 @@ struct pg_ctx {
     // failure-path test hook (pg_debug_stall_next_gram): the next tcgen05 Gram
     // launch waits this long on a barrier nothing arrives on, then gives up
     unsigned long long debug_gram_stall_ns = 0;
+    // the same for teams of CTAs (pg_debug_stall_next_team): a CTA of every
+    // team of the next such launch holds back until the others gave up
+    unsigned long long debug_team_stall_ns = 0;
 };
 
 struct pg_graph {
