@@ -8,10 +8,10 @@
 // the device (the reference streams 3072^2 blocks over PCIe per phase and
 // pads every graph to 3072).  The launch first computes, over the whole grid,
 // the weight maxima, the cube roots of the normalised weights and the Onnela
-// clustering of every node; then its CTAs work in teams, each of which takes
-// one graph after another from a queue (largest first), so that the matrices
-// being swept stay in L2 and a barrier has only the team's arrivals:
-//   A  the team's rows: +inf, 0 on the diagonal, 1/w for the edges;
+// clustering of every node; then its CTAs work in teams (one, but for very
+// large batches: fw_plan.h), each of which takes one bundle of graphs after
+// another from a queue (largest first) and sweeps its graphs in step:
+//   A  the rows: +inf, 0 on the diagonal, 1/w for the edges;
 //   then for every 64-wide k-block round kb:
 //   1  the row and column panels, closed in place against the closed diagonal
 //      block (64 steps in order, eight at a time);
@@ -24,6 +24,7 @@
 // per-graph sums run over the nodes in order, so no result depends on the
 // teams or on the grid.
 #include "pg_internal.cuh"
+#include "fw_plan.h"
 #include <algorithm>
 #include <cmath>
 #include <cooperative_groups.h>
@@ -53,15 +54,19 @@ struct FWGraph {
     long long edge0;    // offset of its entries in cw
     int32_t node0;      // its nodes in processing order
     int32_t out0;       // and in the caller's concatenated outputs
+    // sums over the graphs before it (the table has one entry more, for the totals):
+    long long row0;     // padded rows
+    long long panel0;   // panel blocks of a round, 2 (nb - 1)
+    long long inner0;   // other blocks of a round without a diagonal one, (nb - 1)^2 - 1 (0 for one block)
 };
 
 struct FwControl {
     int onnela_next;    // dynamic node scheduler
-    int queue;          // next graph
+    int queue;          // next bundle
     int timeout;        // a team barrier gave up
     int pad;
     unsigned arrived[MAX_TEAMS];
-    int graph[MAX_TEAMS];   // the graph a team works on
+    int bundle[MAX_TEAMS];  // the bundle a team works on
 };
 
 struct FwBatch {
@@ -69,6 +74,8 @@ struct FwBatch {
     int ng;
     int total_nodes;
     int teams;
+    int bundles;
+    const int* bundle0;         // first graph of every bundle, and ng
     FwControl* ctl;
     float* D;
     float* vmax;                // per graph
@@ -316,7 +323,7 @@ __device__ __forceinline__ void min_plus(FwSmem& sm, Tile& c, const float* a, co
 // s_k.. of its four columns from shared memory, brings them to their own steps
 // (a triangle of updates, done by all eight owners of a column alike), and
 // folds them into its tile as min_plus does.  The minima are exact, so this
-// equals the 64 steps, which took a barrier each (2,500 nodes: 2.02 ms, with
+// equals the 64 steps, which took a barrier each (2,500 nodes: 2.06 ms, with
 // the panels as plain products 1.85, with 64 barriers a panel 2.82).
 __device__ __forceinline__ void close_panel(FwSmem& sm, Tile& c, const float* dg, float* d, int ld, bool row, int kn)
 {
@@ -462,14 +469,14 @@ struct Team {
         hold = false;
         __syncthreads();
     }
-    // The barrier, then the graph that the team's first CTA took, or -1 after
+    // The barrier, then the bundle that the team's first CTA took, or -1 after
     // a timeout.  One thread reads both for its CTA: another team may raise
     // the timeout between two reads, and a CTA whose threads saw different
     // values would leave some of them in the sweep and the others behind it.
-    __device__ int sync_graph(const int* graph, int& shared_slot)
+    __device__ int sync_bundle(const int* bundle, int& shared_slot)
     {
         sync();
-        if (threadIdx.x == 0) shared_slot = *(volatile int*)timeout ? -1 : *(volatile const int*)graph;
+        if (threadIdx.x == 0) shared_slot = *(volatile int*)timeout ? -1 : *(volatile const int*)bundle;
         __syncthreads();
         return shared_slot;   // written again only behind the next barrier
     }
@@ -482,67 +489,118 @@ __device__ __forceinline__ int graph_at(const FwBatch& p, int gi, long long x)
     return gi;
 }
 
-// Floyd-Warshall of one graph by the CTAs of a team; this group is number vb
-// of the team's nvb.
-__device__ __forceinline__ void fw_graph(const FwBatch& p, const FWGraph& g, Team& team, FwSmem& sm, int vb, int nvb)
+// the graph among [a, b) whose share of a task list holds task x (counted over
+// all graphs); SUM is the table's running sum of the list
+template <long long FWGraph::*SUM>
+__device__ __forceinline__ int task_graph(const FwBatch& p, int a, int b, long long x)
+{
+    int lo = a, hi = b - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (p.gs[mid].*SUM <= x) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Floyd-Warshall of the graphs [a, b) by the CTAs of a team, all in step: a
+// round's blocks of all graphs that have it form one task list.  This group is
+// number vb of the team's nvb.
+__device__ __forceinline__ void fw_bundle(const FwBatch& p, int a, int b, Team& team, FwSmem& sm, int vb, int nvb)
 {
     const int lane = group_thread() & 31, gw = vb * (GT / 32) + (group_thread() >> 5), nw = nvb * (GT / 32);
     // ---- A: a warp per row (init_block, FormBlock.cpp:64)
-    for (int i = gw; i < g.np; i += nw) {
-        float* d = p.D + g.off + (long long)i * g.np;
-        for (int j = 4 * lane; j < g.np; j += 128) {
-            float4 v = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
-            if (i >= j && i < j + 4) ((float*)&v)[i - j] = 0.0f;
-            *(float4*)(d + j) = v;
-        }
-        __syncwarp();   // the row is filled before its edges are written
-        if (i >= g.n) continue;
-        const int32_t s = g.R[i], e = g.R[i + 1];
-        for (int32_t q = s + lane; q < e; q += 32) {
-            const int j = g.C[q];
-            if (j != i) d[j] = g.V ? __fdiv_rn(1.0f, g.V[q]) : 1.0f;
+    {
+        const long long first = p.gs[a].row0, rows = p.gs[b].row0 - first;
+        int gi = a;
+        for (long long x = gw; x < rows; x += nw) {
+            while (x >= p.gs[gi + 1].row0 - first) gi++;
+            const FWGraph g = p.gs[gi];
+            const int i = (int)(x - (g.row0 - first));
+            float* d = p.D + g.off + (long long)i * g.np;
+            for (int j = 4 * lane; j < g.np; j += 128) {
+                float4 v = make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+                if (i >= j && i < j + 4) ((float*)&v)[i - j] = 0.0f;
+                *(float4*)(d + j) = v;
+            }
+            __syncwarp();   // the row is filled before its edges are written
+            if (i >= g.n) continue;
+            const int32_t s = g.R[i], e = g.R[i + 1];
+            for (int32_t q = s + lane; q < e; q += 32) {
+                const int j = g.C[q];
+                if (j != i) d[j] = g.V ? __fdiv_rn(1.0f, g.V[q]) : 1.0f;
+            }
         }
     }
     team.sync();
     Tile c;
-    if (vb == 0) {   // the first diagonal block; the others are closed as soon as they are final
+    // the first diagonal blocks; the others are closed as soon as they are final
+    for (int gi = a + vb; gi < b; gi += nvb) {
+        const FWGraph g = p.gs[gi];
         float* d = blk(p.D, g, 0, 0);
         c.load(d, g.np);
         close_block(sm, c);
         c.store(d, g.np);
     }
     team.sync();
-    const int m = g.nb - 1;
-    for (int kb = 0; kb < g.nb && m > 0; kb++) {
+    // graphs [a, act) have more than kb blocks, [a, an) more than kb + 1
+    const int rounds = p.gs[a].nb > 1 ? p.gs[a].nb : 0;
+    int act = b, an = b;
+    for (int kb = 0; kb < rounds; kb++) {
+        while (act > a && p.gs[act - 1].nb <= kb) act--;
+        while (an > a && p.gs[an - 1].nb <= kb + 1) an--;
         // 1: row and column panels
-        const float* dg = blk(p.D, g, kb, kb);
-        const int kn = min(B, g.n - kb * B);   // rows and columns kb * B + kn.. are padding
-        for (int t = vb; t < 2 * m; t += nvb) {
-            const bool row = t < m;
-            int other = row ? t : t - m;
+        const long long first = p.gs[a].panel0, panels = p.gs[act].panel0 - first;
+        for (long long t = vb; t < panels; t += nvb) {
+            const FWGraph g = p.gs[task_graph<&FWGraph::panel0>(p, a, act, first + t)];
+            const int local = (int)(first + t - g.panel0), m = g.nb - 1;
+            const bool row = local < m;
+            int other = row ? local : local - m;
             if (other >= kb) other++;
-            close_panel(sm, c, dg, row ? blk(p.D, g, kb, other) : blk(p.D, g, other, kb), g.np, row, kn);
+            // rows and columns past n are padding
+            close_panel(sm, c, blk(p.D, g, kb, kb), row ? blk(p.D, g, kb, other) : blk(p.D, g, other, kb), g.np, row,
+                        min(B, g.n - kb * B));
         }
         team.sync();
-        // 2: the other blocks, the next round's diagonal block first
-        const bool last = kb + 1 == g.nb;
-        for (int t = vb; t < m * m; t += nvb) {
-            // block (kb + 1, kb + 1) is number kb (m + 1) of the m x m others
-            int local = t;
-            if (!last) local = t == 0 ? kb * (m + 1) : t <= kb * (m + 1) ? t - 1 : t;
+        // 2: the other blocks, the next round's diagonal blocks first; then
+        // the rest of their graphs' blocks, then those of graphs in their last round
+        const long long inner = p.gs[a].inner0, n_inner = p.gs[an].inner0 - inner;
+        const long long total = (an - a) + n_inner + (long long)(act - an) * kb * kb;
+        for (long long t = vb; t < total; t += nvb) {
+            int gi, local;
+            const bool diagonal = t < an - a;
+            long long x = t - (an - a);
+            if (diagonal) {
+                gi = a + (int)t;
+                local = kb * p.gs[gi].nb;   // block (kb + 1, kb + 1) of the others
+            } else if (x < n_inner) {
+                gi = task_graph<&FWGraph::inner0>(p, a, an, inner + x);
+                local = (int)(inner + x - p.gs[gi].inner0);
+                local += local >= kb * p.gs[gi].nb;
+            } else {
+                x -= n_inner;
+                gi = an + (int)(x / (kb * kb));
+                local = (int)(x % (kb * kb));
+            }
+            const FWGraph g = p.gs[gi];
+            const int m = g.nb - 1;
             int bi = local / m, bj = local % m;
             if (bi >= kb) bi++;
             if (bj >= kb) bj++;
             float* d = blk(p.D, g, bi, bj);
             c.load(d, g.np);
-            min_plus(sm, c, blk(p.D, g, bi, kb), blk(p.D, g, kb, bj), g.np, kn);
-            if (!last && t == 0) close_block(sm, c);
+            min_plus(sm, c, blk(p.D, g, bi, kb), blk(p.D, g, kb, bj), g.np, min(B, g.n - kb * B));
+            if (diagonal) close_block(sm, c);
             c.store(d, g.np);
         }
         team.sync();
     }
     // ---- C: row sums of 1/d over finite, non-tiny distances (CUBFW_Lp.cpp:77-83,99-104)
-    for (int u = gw; u < g.n; u += nw) {
+    const int end = p.gs[b].node0;
+    int gi = a;
+    for (long long x = (long long)p.gs[a].node0 + gw; x < end; x += nw) {
+        gi = graph_at(p, gi, x);
+        const FWGraph g = p.gs[gi];
+        const int u = (int)x - g.node0;
         const float* row = p.D + g.off + (long long)u * g.np;
         double acc = 0.0;
         for (int v0 = lane; v0 < g.n; v0 += 128) {
@@ -555,7 +613,7 @@ __device__ __forceinline__ void fw_graph(const FwBatch& p, const FWGraph& g, Tea
         }
         for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) {
-            p.rowsum[g.node0 + u] = acc;
+            p.rowsum[x] = acc;
             float e = g.n > 1 ? (float)(acc / (double)(g.n - 1)) : 0.0f;
             if (e < 1.0f / (float)g.n) e = 0.0f;
             p.eff[g.out0 + u] = e;
@@ -632,13 +690,13 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_fw_batch(FwBatch p)
         const int end = (int)(((long long)(t + 1) * n_cta + p.teams - 1) / p.teams);
         Team team{&p.ctl->arrived[t], &p.ctl->timeout, (unsigned)(end - first), 0u, p.max_spins,
                   p.hold && end - first > 1 && blockIdx.x == end - 1};
-        __shared__ int s_graph;
+        __shared__ int s_bundle;
         for (;;) {
-            if (blockIdx.x == first && threadIdx.x == 0) *(volatile int*)&p.ctl->graph[t] = atomicAdd(&p.ctl->queue, 1);
-            const int gi = team.sync_graph(&p.ctl->graph[t], s_graph);
-            if (gi < 0 || gi >= p.ng) break;
-            const FWGraph g = p.gs[gi];
-            fw_graph(p, g, team, sm, grp * (end - first) + (blockIdx.x - first), GROUPS * (end - first));
+            if (blockIdx.x == first && threadIdx.x == 0) *(volatile int*)&p.ctl->bundle[t] = atomicAdd(&p.ctl->queue, 1);
+            const int q = team.sync_bundle(&p.ctl->bundle[t], s_bundle);
+            if (q < 0 || q >= p.bundles) break;
+            fw_bundle(p, p.bundle0[q], p.bundle0[q + 1], team, sm, grp * (end - first) + (blockIdx.x - first),
+                      GROUPS * (end - first));
         }
     }
     grid.sync();
@@ -680,8 +738,8 @@ static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, boo
     std::iota(order.begin(), order.end(), 0);
     auto nb_of = [&](int i) { return std::max(1, (graphs[i]->n + B - 1) / B); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return nb_of(x) > nb_of(y); });
-    std::vector<FWGraph> tab(ng);
-    std::vector<int> out0(ng);
+    std::vector<FWGraph> tab((size_t)ng + 1);
+    std::vector<int> out0(ng), blocks(ng);
     long long edges = 0, off = 0;
     int nodes = 0, nmax = 1;
     for (int i = 0; i < ng; i++) {
@@ -689,27 +747,38 @@ static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, boo
         nodes += graphs[i]->n;
     }
     nodes = 0;
-    double work = 0.0, work_max = 0.0;
+    long long row0 = 0, panel0 = 0, inner0 = 0;
     for (int q = 0; q < ng; q++) {
         const pg_graph* g = graphs[order[q]];
         if (onnela && !g->V) return pg_fail(ctx, PG_ERR_INVALID, "Onnela clustering needs a weighted graph");
-        const int nb = nb_of(order[q]);
-        tab[q] = {g->R, g->C, g->V, g->n, nb * B, nb, order[q], off, edges, nodes, out0[order[q]]};
+        const int nb = blocks[q] = nb_of(order[q]);
+        tab[q] = {g->R, g->C, g->V, g->n, nb * B, nb, order[q], off, edges, nodes, out0[order[q]],
+                  row0, panel0, inner0};
+        row0 += nb * B;
+        panel0 += 2LL * (nb - 1);
+        inner0 += nb > 1 ? (long long)(nb - 1) * (nb - 1) - 1 : 0;
         off += (long long)nb * B * nb * B;
         nodes += g->n;
         edges += g->nnz;
         nmax = std::max(nmax, (int)g->n);
-        const double w = (double)nb * nb * nb;
-        work += w;
-        work_max = std::max(work_max, w);
     }
+    tab[ng].node0 = nodes;
+    tab[ng].row0 = row0;
+    tab[ng].panel0 = panel0;
+    tab[ng].inner0 = inner0;
     if (onnela && nmax > ONNELA_MAX_N)
         return pg_fail(ctx, PG_ERR_TOO_LARGE, "Onnela in the batched launch: n=%d above %d", nmax, ONNELA_MAX_N);
     FwBatch& b = *P;
     memset(&b, 0, sizeof b);
     FWGraph* dtab;
     PG_TRY(pg_wst(ctx, "fw.D", (size_t)off, &b.D));
-    PG_TRY(pg_wst(ctx, "fw.tab", (size_t)ng, &dtab));
+    // the bundles' first graphs lie behind the table: one upload
+    const FwPlan plan = fw_batch_plan(blocks.data(), ng, ctx->sm_count, MAX_TEAMS);
+    const size_t tab_bytes = sizeof(FWGraph) * ((size_t)ng + 1), cut_bytes = sizeof(int) * plan.bundle0.size();
+    std::vector<unsigned char> blob(tab_bytes + cut_bytes);
+    memcpy(blob.data(), tab.data(), tab_bytes);
+    memcpy(blob.data() + tab_bytes, plan.bundle0.data(), cut_bytes);
+    PG_TRY(pg_ws(ctx, "fw.tab", blob.size(), (void**)&dtab));
     PG_TRY(pg_wst(ctx, "fw.ctl", 1, &b.ctl));
     if (onnela) {
         PG_TRY(pg_wst(ctx, "fw.cw", (size_t)edges + 1, &b.cw));
@@ -721,16 +790,14 @@ static pg_status fw_plan(pg_ctx* ctx, const pg_graph* const* graphs, int ng, boo
     PG_TRY(pg_wst(ctx, "fw.rows", (size_t)nodes + 1, &b.rowsum));
     PG_TRY(pg_wst(ctx, "fw.eff", (size_t)nodes + 1, &b.eff));
     PG_TRY(pg_wst(ctx, "fw.lp", (size_t)ng + 1, &b.lp));
-    PG_TRY(pg_h2d(ctx, dtab, tab.data(), sizeof(FWGraph) * ng));
+    PG_TRY(pg_h2d(ctx, dtab, blob.data(), blob.size()));
+    b.teams = plan.teams;
+    b.bundles = (int)plan.bundle0.size() - 1;
+    b.bundle0 = (const int*)((const unsigned char*)dtab + tab_bytes);
     b.gs = dtab;
     b.ng = ng;
     b.total_nodes = nodes;
     b.onnela = onnela;
-    // As many teams as leave the largest graph, alone on its team, at most
-    // half of the batch's time, and at least four SMs (16 blocks at once) per
-    // team: one graph gets the whole GPU, 512 region graphs 37 teams (17.9 ms;
-    // with every phase over all graphs and the whole grid 20.7 ms).
-    b.teams = (int)std::max(1.0, std::min({(double)MAX_TEAMS, ctx->sm_count / 4.0, 0.5 * work / std::max(work_max, 1.0)}));
     PG_CUDA(ctx, cudaFuncSetAttribute(k_fw_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(GROUPS * sizeof(FwSmem))));
     return PG_OK;

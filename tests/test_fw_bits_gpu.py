@@ -87,3 +87,17 @@ def test_distances_to_the_last_bit(ctx, n, r, both_ways):
     assert np.array_equal(dist.reshape(n, n), want)
     eff_w, lp_w = _eff_lp(want)
     assert np.array_equal(eff, eff_w) and lp == lp_w
+
+
+def test_bundles_of_teams_to_the_last_bit(ctx):
+    """So many graphs that teams of CTAs take them in bundles, and the same
+    graphs a few at a time: sizes mixed so that bundles hold several."""
+    made = [_region_graph(n, 0.3, n) for n in (60, 65, 90, 100, 128, 130, 190, 200)]
+    gs = [ctx.graph(*csr) for csr, _ in made]
+    pick = np.random.default_rng(1).integers(0, len(gs), 1600)
+    out = ctx.fw_batched([gs[q] for q in pick])
+    few = ctx.fw_batched(gs)
+    want = [_eff_lp(_closed(D)) for _, D in made]
+    for q, (eff, lp, cp, cpm) in zip(pick, out):
+        assert np.array_equal(eff, want[q][0]) and lp == want[q][1]
+        assert np.array_equal(cp, few[q][2]) and cpm == few[q][3]
