@@ -461,10 +461,15 @@ pg_status launch_brandes(pg_ctx* ctx, BCArgs& a, int batch_first, int batch_last
     int per_sm = 0;
     PG_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_brandes, THREADS, 0));
     if (per_sm < 1) return pg_fail(ctx, PG_ERR_INTERNAL, "brandes kernel cannot be resident");
-    // four CTAs per SM hide the latency of the gathers; below 8,192 nodes a
-    // level hands each warp of two CTAs per SM a few nodes at most, and the
-    // barriers between levels cost less (5,000 nodes: 12.5 -> 11.9 ms)
-    if (a.n < 8192) per_sm = std::min(per_sm, 2);
+    // Four CTAs per SM hide the latency of the gathers.  On small graphs a
+    // level hands each warp a few nodes at most and the barriers between
+    // levels weigh more: voxel graphs, which have more levels than random ones
+    // of the same size, are faster with fewer CTAs to 8,000 nodes and beyond,
+    // random ones of 50 neighbours only up to these bounds (ms with 4 / 3 / 2
+    // CTAs, random: 2,000 nodes 2.0 / 1.8 / 1.7, 3,000 3.1 / 2.8 / 3.1, 5,000
+    // 6.2 / 5.9 / 6.8, 6,500 9.0 / 8.8 / 10.0, 8,000 13.0 / 13.8 / 15.6;
+    // voxels, 1 %: 2,000 4.5 / 4.3 / 4.1, 5,000 19.1 / 18.1 / 17.3).
+    per_sm = std::min(per_sm, a.n < 2560 ? 2 : a.n < 6656 ? 3 : 4);
     const int grid = per_sm * ctx->sm_count;
     void* args[] = {(void*)&a, (void*)&batch_first, (void*)&batch_last, (void*)&fwd_first, (void*)&fwd_last};
     const int prof = pg_prof_begin(ctx, "k_brandes");
