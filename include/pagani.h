@@ -73,10 +73,11 @@ pg_status   pg_profile_get(pg_ctx* ctx, const char* kernel, int64_t* launches, d
  * and the call (pg_build_graph) returns PG_ERR_TIMEOUT.  The context stays
  * usable.  Applies to one launch; 0 clears it. */
 pg_status   pg_debug_stall_next_gram(pg_ctx* ctx, uint64_t wait_ns);
-/* The same for kernels whose CTAs work in teams (pg_fw_paths,
- * pg_fw_batched): in the next such launch one CTA of every team holds back
- * its first arrival until another has waited wait_ns for it and given up; the
- * call returns PG_ERR_TIMEOUT. */
+/* The same for kernels whose CTAs work in teams (pg_fw_paths, pg_fw_batched,
+ * and the clusters of pg_newman and pg_newman_weighted that exchange their
+ * vector through shared memory): in the next such call one CTA of every team
+ * holds back its first arrival until another has waited wait_ns for it and
+ * given up; the call returns PG_ERR_TIMEOUT. */
 pg_status   pg_debug_stall_next_team(pg_ctx* ctx, uint64_t wait_ns);
 
 /* ------------------------------------------------------------- graphs */

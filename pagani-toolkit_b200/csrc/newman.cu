@@ -515,6 +515,7 @@ struct Inputs {
     double* hout;
     double* hv;
     int* hdone;
+    unsigned long long stall_ns;   // failure-path test hook, 0: off (pg_debug_stall_next_team)
 };
 
 __device__ __forceinline__ Group global_group(const Inputs& in, int gi)
@@ -684,13 +685,18 @@ struct Team {
     double* yx;           // two vectors of y, used alternately
     int ystride;
     int nb, rank;
+    unsigned long long wait_ns;
+    bool hold;            // test hook: this CTA sends nothing
 };
 
-// Shared state of the exchange: a full barrier per vector, and whether a wait
-// ran out.
+// Shared state of the exchange: a full barrier per vector; whether a wait of a
+// thread of this CTA ran out; whether one of any CTA of the team did; and
+// (after that) the steps that every CTA sent.
 struct TeamX {
     unsigned long long full[2];
+    int stop;
     int failed;
+    int sent[CLUSTER];
 };
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank)
@@ -708,13 +714,33 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int rank)
 // and finished reading it.  16 CTAs, 700 rows: 1200 cycles with the wait for
 // the slowest CTA, against 1200 for a cluster barrier behind stores to global
 // memory and 600 more to read them back (5,000 nodes: 43.7 -> 38.2 ms).
-__device__ __forceinline__ void team_exchange(const Team& tm, double* ybuf, TeamX& tx, int step)
+// Bytes of a CTA's rows of y (whole 16-byte units: rows start at even indices)
+__device__ __forceinline__ uint32_t team_bytes(int rows) { return (uint32_t)((rows + 1) & ~1) * 8; }
+
+__device__ __forceinline__ void team_set(int* where, int value, int rank)
+{
+    const uint32_t a = cluster_addr(pg_tma::smem_u32(where), rank);
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(value) : "memory");
+}
+
+// A thread whose wait runs out, or that sees that a peer's did, sets tx.stop;
+// behind the next block barrier the whole CTA reads the same answer and leaves
+// the step loop before it sends again.
+__device__ __forceinline__ void team_exchange(const Team& tm, double* ybuf, TeamX& tx, int& steps)
 {
     using namespace pg_tma;
+    const int step = steps;
     unsigned long long* bar = &tx.full[step & 1];
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    const uint32_t own = (uint32_t)((tm.nown + 1) & ~1) * 8, all = (uint32_t)((tm.n + 1) & ~1) * 8;
+    if (tm.hold) {
+        const unsigned long long t0 = gtimer();
+        while (!*(volatile int*)&tx.failed && gtimer() - t0 < WAIT_NS) {}
+        *(volatile int*)&tx.stop = 1;
+        return;
+    }
+    steps++;
+    const uint32_t own = team_bytes(tm.nown), all = team_bytes(tm.n);
     if (threadIdx.x == 0) mbar_expect_tx(bar, all - own);
     if ((int)threadIdx.x < tm.nb && (int)threadIdx.x != tm.rank && own)
         asm volatile(
@@ -737,11 +763,46 @@ __device__ __forceinline__ void team_exchange(const Team& tm, double* ybuf, Team
     if (!done()) {
         const unsigned long long t0 = gtimer();
         while (!done())
-            if (*(volatile int*)&tx.failed || gtimer() - t0 > WAIT_NS) {
-                *(volatile int*)&tx.failed = 1;
+            if (*(volatile int*)&tx.failed || gtimer() - t0 > tm.wait_ns) {
+                *(volatile int*)&tx.stop = 1;
                 break;
             }
     }
+}
+
+// After a failure that every CTA of the team knows of (all have stopped
+// sending): waits, within the limit, for the copies still on their way into
+// this CTA, so that none arrives in shared memory that is no longer its own.
+// The last step that this CTA sent (steps - 1) is armed for all its peers' rows;
+// peers that never sent it are taken off.  Peers that got everything of that
+// step may have sent the next one, which is not armed here yet.
+__device__ __forceinline__ void team_drain(const Team& tm, const Group& gg, TeamX& tx, int steps)
+{
+    using namespace pg_tma;
+    if ((int)threadIdx.x < tm.nb) team_set(&tx.sent[tm.rank], steps, threadIdx.x);
+    cg::this_cluster().sync();
+    if (threadIdx.x == 0) {
+        uint32_t missing = 0, next = 0;
+        for (int r = 0; r < tm.nb; r++) {
+            if (r == tm.rank) continue;
+            const uint32_t bytes = team_bytes(team_first(gg.sR, tm.n, r + 1, tm.nb) - team_first(gg.sR, tm.n, r, tm.nb));
+            if (tx.sent[r] < steps) missing += bytes;
+            if (tx.sent[r] > steps) next += bytes;
+        }
+        if (steps > 0) {
+            unsigned long long* bar = &tx.full[(steps - 1) & 1];
+            if (missing)
+                asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(missing)
+                             : "memory");
+            mbar_wait(bar, (uint32_t)((steps - 1) >> 1) & 1u);
+        }
+        if (next) {
+            unsigned long long* bar = &tx.full[steps & 1];
+            mbar_expect_tx(bar, next);
+            mbar_wait(bar, (uint32_t)(steps >> 1) & 1u);
+        }
+    }
+    __syncthreads();
 }
 
 // own rows of y = B v from the sliced matrix, written to ydst[own row]
@@ -976,7 +1037,11 @@ __device__ __forceinline__ double team_normalise(const Team& tm, const double* y
 }
 
 // Lead_Vector (Modularity_CPU.cpp:224-298) for a team: the reference's
-// per-entry arithmetic, sums in a fixed order over all rows.
+// per-entry arithmetic, sums in a fixed order over all rows.  When a wait of
+// the exchange runs out, the CTA whose it was leaves the loop at once, for all
+// its threads alike, and raises tx.failed in every CTA of the team before the
+// cluster barrier behind the loop, so that all of them return there (the
+// result is not used); the barriers stay matched whichever step each was in.
 template <class Kind, bool W>
 __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, double beta, double err_sq, int* iters,
                                    double* resid, Partials& ps, int& ph, TeamX& tx, int& xstep)
@@ -1000,7 +1065,7 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
         const bool push = Kind::kCluster && tm.push;
         double* ybuf = !Kind::kCluster ? tm.oy : push ? tm.yx + (xstep & 1) * tm.ystride : yb ? gg.v0 : gg.v;
         team_spmv<W>(tm, Kind::kCluster ? ybuf + tm.r0 : ybuf, c, beta, lane, wid, nwarp);
-        if (push) team_exchange(tm, ybuf, tx, xstep++);
+        if (push) team_exchange(tm, ybuf, tx, xstep);
         else Kind::barrier();
         double x3[3] = {0.0, 0.0, 0.0};
         const int npt = (n + nthr - 1) / nthr;   // entries per thread
@@ -1032,7 +1097,13 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
                 tm.rep[p] = vp;
             }
         }
+        // behind the block barrier of |y|'s sum: set by no one until the next exchange
+        const int stop = Kind::kCluster ? *(volatile int*)&tx.stop : 0;
         team_sum3(ps, x3, ph);
+        if (stop) {
+            if (tid < tm.nb) team_set(&tx.failed, 1, tid);
+            break;
+        }
         s1 = x3[0];
         s2 = x3[1];
         vk = x3[2];
@@ -1043,6 +1114,7 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
     *resid = fmin(sqrt(s1), sqrt(s2));
     // the labels are assigned from v; the sign test below reads v0 of any row
     Kind::barrier();   // the y buffers are free again
+    if (Kind::kCluster && *(volatile int*)&tx.failed) return 0.0;
     for (int lp = tid; lp < tm.nown; lp += nthr) {
         gg.v[tm.r0 + lp] = tm.rep[tm.r0 + lp];
         gg.v0[tm.r0 + lp] = tm.oprev[lp];
@@ -1208,6 +1280,8 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
     tm.L = tm.nslices > 0 ? sL : lanes_per_row(tm.nown, tm.nown > 0 ? (long long)tm.oR[tm.nown] : 0, blockDim.x);
     tm.nb = nb;
     tm.rank = rank;
+    tm.wait_ns = in.stall_ns ? in.stall_ns : pg_tma::WAIT_NS;
+    tm.hold = in.stall_ns && rank == nb - 1;
     // a CTA without rows would send nothing, and the others could overtake it
     tm.push = Kind::kCluster && team_push(tm.n, nb) &&
               __syncthreads_and((int)threadIdx.x >= nb || team_first(gg.sR, tm.n, threadIdx.x + 1, nb) >
@@ -1219,7 +1293,7 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
         if (threadIdx.x == 0) {
             pg_tma::mbar_init(&tx.full[0], 1);
             pg_tma::mbar_init(&tx.full[1], 1);
-            tx.failed = 0;
+            tx.failed = tx.stop = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         Kind::barrier();   // every barrier exists before the first copy arrives
@@ -1230,7 +1304,9 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
     double res0, res1 = 0.0;
     double lam = team_lead_vector<Kind, W>(tm, gg, in.M, 0.0, in.err_sq, &it0, &res0, ps, ph, tx, xstep);
     const double below = gg.ng > in.gpu_rule_above ? -LAMBDA : 0.0;
-    const bool shifted = lam < below;
+    // the failure is the same in every CTA of the team from here on
+    bool failed = Kind::kCluster && *(volatile int*)&tx.failed;
+    const bool shifted = !failed && lam < below;
     if (shifted) lam += team_lead_vector<Kind, W>(tm, gg, in.M, -lam, in.err_sq, &it1, &res1, ps, ph, tx, xstep);
     double x2[2] = {0.0, 0.0};
     for (int p = threadIdx.x; p < tm.n; p += blockDim.x) {
@@ -1239,13 +1315,12 @@ k_nm_team(const int* __restrict__ glist, Inputs in, int smem_bytes, uint16_t* __
     }
     block_sum(ps, x2, ph);
     if (Kind::kCluster) {
-        // a wait of any CTA that ran out is reported by the first one
-        if (threadIdx.x == 0 && rank != 0 && tx.failed) {
-            const uint32_t a = cluster_addr(pg_tma::smem_u32(&tx.failed), 0);
-            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(1) : "memory");
+        failed = *(volatile int*)&tx.failed;
+        if (failed) {
+            team_drain(tm, gg, tx, xstep);
+            it0 = TEAM_TIMEOUT;
         }
-        Kind::barrier();
-        if (tx.failed) it0 = TEAM_TIMEOUT;
+        Kind::barrier();   // no CTA ends while a peer may still read its rows
     }
     double o[OUT_W] = {lam, (double)it0, res0, (double)it1, res1, x2[0], x2[1], (double)shifted, t_start, 0.0};
     if (rank == 0 && threadIdx.x == 0) {
@@ -1934,6 +2009,8 @@ static pg_status newman_run(pg_ctx* ctx, const pg_graph* g, const float* wv, lon
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     // log lines are handed to `log` when the call succeeds, so that a call
     // run again (see pg_newman) reports every round once
+    const unsigned long long stall_ns = ctx->debug_team_stall_ns;   // applies to this call only
+    ctx->debug_team_stall_ns = 0;
     std::vector<std::string> lines;
     auto emit = [&](const char* l) { lines.emplace_back(l); };
     const bool weighted = wv != nullptr;
@@ -2097,6 +2174,7 @@ static pg_status newman_run(pg_ctx* ctx, const pg_graph* g, const float* wv, lon
         in.v = v; in.v0 = v0; in.M = M; in.gpu_rule_above = gpu_rule_above; in.out = out; in.err_sq = err_sq;
         in.wv = wv; in.wn = wn;
         in.hout = nullptr; in.hv = nullptr; in.hdone = nullptr;
+        in.stall_ns = stall_ns;
         // Shared memory of the largest CTA of group q split over c CTAs,
         // before its sliced columns
         auto team_need = [&](int q, int c) {
