@@ -32,6 +32,7 @@
 // argument reduction and Taylor series), so keys, edges and weights are
 // bit-identical to the oracle's.
 #include "build_graph.cuh"
+#include "quotient.cuh"
 #include "tma.cuh"
 #include <cuda.h>
 #include <cstring>
@@ -94,26 +95,6 @@ __device__ double d_exp(double x)
     if (k > 1023) return __dmul_rn(__dmul_rn(p, pow2i(1023)), pow2i((int)k - 1023));
     if (k < -1022) return __dmul_rn(__dmul_rn(p, pow2i((int)k + 600)), pow2i(-600));
     return __dmul_rn(p, pow2i((int)k));
-}
-
-// a / b, correctly rounded, for normal a and b whose quotient is normal: the
-// reciprocal by Newton's iteration from the hardware's approximation, then
-// two quotient corrections with exact remainders (P. Markstein, IBM J. Res.
-// Dev. 34(1), 1990; checked against the division operator on 6e10 pairs).
-// Unlike the operator it has no branch, so several run side by side.
-__device__ __forceinline__ double div_normal(double a, double b)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-b, q, a), y, q);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
 // fisher_trans (CorMat.cpp:35-41) in FP64 of K values at once: r >= 1 ->
