@@ -27,6 +27,7 @@
 // v'.k for the next step together.  Reductions are FP64 in a fixed order, so
 // results are deterministic.
 #include "pg_internal.cuh"
+#include "quotient.cuh"
 #include "tma.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
@@ -916,17 +917,6 @@ __device__ __forceinline__ void team_spmv(const Team& tm, double* ydst, double c
     else team_spmv_w<2>(tm, ydst, c, beta, lane, wid, nwarp);
 }
 
-// x / d for the reciprocal r = 1 / d rounded to nearest: two Newton steps on
-// the quotient with exact remainders (P. Markstein, IBM J. Res. Dev. 34(1),
-// 1990).  The result is the correctly rounded quotient while nothing under-
-// or overflows (checked against the division operator on 6e10 pairs).
-__device__ __forceinline__ double div_by(double x, double d, double r)
-{
-    double q = __dmul_rn(x, r);
-    q = __fma_rn(__fma_rn(-d, q, x), r, q);
-    return __fma_rn(__fma_rn(-d, q, x), r, q);
-}
-
 // Sums over the 8 or 16 warps of a team CTA, in a fixed order, for the two
 // reductions of a step.  A step of a small group is these sums: 64-bit
 // shuffles (two each, one per clock and SM over all warps) took 1280 of its
@@ -1014,7 +1004,7 @@ __device__ __forceinline__ double team_normalise(const Team& tm, const double* y
     for (int k = 0; k < NPT; k++) sq += yv[k] * yv[k];
     const double vnorm = sqrt(team_sum1(ps, sq, ph));
     const double rnorm = 1.0 / vnorm;
-    if (vnorm > 1e-140 && vnorm < 1e140) {   // quotients through the reciprocal
+    if (div_by_divisor(vnorm)) {   // quotients through the reciprocal
 #pragma unroll
         for (int k = 0; k < NPT; k++) yv[k] = div_by(yv[k], vnorm, rnorm);
     } else {
@@ -1084,11 +1074,11 @@ __device__ double team_lead_vector(const Team& tm, const Group& gg, int M, doubl
                 x1[0] += y * y;
             }
             vnorm = sqrt(team_sum1(ps, x1[0], ph));
-            const bool normal = vnorm > 1e-140 && vnorm < 1e140;
+            const bool quick = div_by_divisor(vnorm);
             const double rnorm = 1.0 / vnorm;
             for (int p = tid; p < n; p += nthr) {
                 const double vold = tm.rep[p];
-                const double vp = normal ? div_by(ybuf[p], vnorm, rnorm) : ybuf[p] / vnorm;
+                const double vp = quick ? div_by(ybuf[p], vnorm, rnorm) : ybuf[p] / vnorm;
                 const double d1 = vp - vold, d2 = vp + vold;
                 x3[0] += d1 * d1;
                 x3[1] += d2 * d2;

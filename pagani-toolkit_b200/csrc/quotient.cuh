@@ -30,3 +30,17 @@ __device__ __forceinline__ double div_normal(double a, double b)
     q = __fma_rn(__fma_rn(-b, q, a), y, q);
     return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
+
+// x / d for r = 1 / d rounded to nearest, x and x / d below 2^400 in magnitude
+// and a d that div_by_divisor admits (an entry by its vector's norm, a sum by a
+// count).  x is scaled so that no remainder underflows: without that, quotients
+// of an x below 2^-968 could be an ulp off.  A quotient below the normal numbers is rounded twice (its
+// last bit may differ from the operator's); a zero has either sign.
+__device__ __forceinline__ double div_by(double x, double d, double r)
+{
+    const double xs = __dmul_rn(x, 0x1p+600);
+    double q = __dmul_rn(xs, r);
+    q = __fma_rn(__fma_rn(-d, q, xs), r, q);
+    return __dmul_rn(__fma_rn(__fma_rn(-d, q, xs), r, q), 0x1p-600);
+}
+__device__ __forceinline__ bool div_by_divisor(double d) { return d > 0x1p-200 && d < 0x1p+200; }

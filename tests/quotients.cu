@@ -22,7 +22,7 @@ __device__ bool same(double x, double y)
     return __double_as_longlong(x) == __double_as_longlong(y) || (x == 0.0 && y == 0.0);
 }
 
-enum { ATANH_ARGUMENT = 0, SERIES = 1 };
+enum { ATANH_ARGUMENT = 0, SERIES = 1, NORMALISE = 2, MEAN_DEGREE = 3 };
 
 __global__ void k_check(int kind, unsigned long long seed, long long n, unsigned long long* bad)
 {
@@ -34,12 +34,19 @@ __global__ void k_check(int kind, unsigned long long seed, long long n, unsigned
             if (q % 3 == 0) x = copysign(1.0 - (double)(g % 4096 + 1) * 0x1p-53, x);
             const double a = __dadd_rn(1.0, x), b = __dsub_rn(1.0, x);
             wrong += !same(div_normal(a, b), __ddiv_rn(a, b));
-        } else {                             // (m - 1) / (m + 1), m in [sqrt(1/2), sqrt(2)), many next to 1
+        } else if (kind == SERIES) {         // (m - 1) / (m + 1), m in [sqrt(1/2), sqrt(2)), many next to 1
             double m = 0.70710678118654757 + 0.70710678118654757 * (double)(g >> 11) * 0x1p-53;
             if (q % 3 == 0) m = 1.0 + any(h, -52, -3);
             if (q % 1024 == 0) m = 1.0;
             const double a = __dsub_rn(m, 1.0), b = __dadd_rn(m, 1.0);
             wrong += !same(div_normal(a, b), __ddiv_rn(a, b));
+        } else {                             // an entry of any exponent by its norm, or a sum by the edge count
+            const double x = q % 64 == 0 ? 0.0 : any(h, -1023, 399);
+            double d = kind == NORMALISE ? fabs(any(g, -200, 199)) : (double)(g % 2147483647u + 1);
+            if (kind == NORMALISE && q % 5 == 0) d = __longlong_as_double(__double_as_longlong(d) | 0xfffffffffffffLL);
+            const double w = __ddiv_rn(x, d);
+            if (!div_by_divisor(d) || fabs(w) >= 0x1p+400 || (w != 0.0 && fabs(w) < 0x1p-1022)) continue;
+            wrong += !same(div_by(x, d, 1.0 / d), w);
         }
     }
     if (wrong) atomicAdd(bad, wrong);

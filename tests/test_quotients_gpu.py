@@ -24,9 +24,10 @@ def mismatches(tmp_path_factory):
     return f
 
 
-@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
 def test_quotients_equal_the_division_operator(mismatches, kind):
-    """(1 + x) / (1 - x) and (m - 1) / (m + 1) of the Fisher transform."""
+    """(1 + x) / (1 - x) and (m - 1) / (m + 1) of the Fisher transform; a
+    vector's entries, of any exponent, by its norm; a sum by the edge count."""
     assert mismatches(kind, 12345 + kind, 1 << 28) == 0
 
 
