@@ -726,8 +726,8 @@ pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const flo
         if (st == PG_OK && w) st = pg_wst(ctx, "sort.V", (size_t)(2 * npairs), &Vt);
         if (st != PG_OK) { pg_graph_free(g); return st; }
         k_pair_scatter<<<grid, 256, 0, ctx->stream>>>(pairs, w, npairs, cursor, Ct, Vt);
-        ctx->launches++;
-        st = launch_row_sort(ctx, g->R, n, Ct, Vt, g->C, g->V);
+        st = [&]() -> pg_status { PG_LAUNCHED(ctx); return PG_OK; }();
+        if (st == PG_OK) st = launch_row_sort(ctx, g->R, n, Ct, Vt, g->C, g->V);
         if (st != PG_OK) { pg_graph_free(g); return st; }
     }
     *out = g;

@@ -537,7 +537,10 @@ static pg_status csr_from_bits(pg_ctx* ctx, int n, const uint32_t* bits, int wor
     }
     if (n_edges > 0) {
         k_bits_csr<<<grid, 256, 0, ctx->stream>>>(bits, words, n, g->R, g->C, g->nnz);
-        ctx->launches++;
+        if (pg_status st = [&]() -> pg_status { PG_LAUNCHED(ctx); return PG_OK; }(); st != PG_OK) {
+            pg_graph_free(g);
+            return st;
+        }
     }
     *out = g;
     return PG_OK;
