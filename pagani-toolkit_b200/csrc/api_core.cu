@@ -334,8 +334,12 @@ pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
     work(0);
     for (int t = 1; t < started; t++) threads[t].join();
     for (int t = started; t < nt; t++) work(t);
+    // whatever a thread met, nothing is on its way into the staging buffers
+    // when they are left to their next user
+    const cudaError_t synced = cudaStreamSynchronize(ctx->stream);
     for (int t = 0; t < nt; t++) PG_CUDA(ctx, err[t]);
-    return pg_synchronize(ctx);
+    PG_CUDA(ctx, synced);
+    return PG_OK;
 }
 
 pg_status pg_h2d(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
