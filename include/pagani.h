@@ -79,6 +79,10 @@ pg_status   pg_debug_stall_next_gram(pg_ctx* ctx, uint64_t wait_ns);
  * holds back its first arrival until another has waited wait_ns for it and
  * given up; the call returns PG_ERR_TIMEOUT. */
 pg_status   pg_debug_stall_next_team(pg_ctx* ctx, uint64_t wait_ns);
+/* Failure-path test hook: the context's device workspace may hold at most
+ * `bytes` (0: no limit), as if the device had no more; calls that need more
+ * return PG_ERR_NOMEM.  Graphs are not counted. */
+pg_status   pg_debug_memory_limit(pg_ctx* ctx, uint64_t bytes);
 
 /* ------------------------------------------------------------- graphs */
 /* Replaces the .csr reads of every metric tool (e.g. U/Cp/Cp/Cp_main.cpp:107-116,

@@ -204,9 +204,52 @@ extern "C" pg_status pg_debug_stall_next_team(pg_ctx* ctx, uint64_t wait_ns)
 }
 
 // --------------------------------------------------------------- workspace
+bool pg_ws_reclaim(pg_ctx* ctx)
+{
+    bool any = false;
+    for (auto& kv : ctx->ws) {
+        pg_ctx::Buf& b = kv.second;
+        if (!b.idle || !b.p) continue;
+        if (!any) cudaStreamSynchronize(ctx->stream);
+        cudaFree(b.p);
+        b = pg_ctx::Buf{};
+        any = true;
+    }
+    return any;
+}
+
+void pg_ws_idle(pg_ctx* ctx, const char* key)
+{
+    auto it = ctx->ws.find(key);
+    if (it != ctx->ws.end()) it->second.idle = true;
+}
+
+cudaError_t pg_malloc(pg_ctx* ctx, void** out, size_t bytes)
+{
+    auto take = [&]() {
+        size_t held = bytes;
+        for (const auto& kv : ctx->ws) held += kv.second.bytes;
+        return ctx->debug_memory_limit && held > ctx->debug_memory_limit ? cudaErrorMemoryAllocation : cudaMalloc(out, bytes);
+    };
+    cudaError_t e = take();
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (pg_ws_reclaim(ctx)) e = take();
+    }
+    return e;
+}
+
+extern "C" pg_status pg_debug_memory_limit(pg_ctx* ctx, uint64_t bytes)
+{
+    if (!ctx) return PG_ERR_INVALID;
+    ctx->debug_memory_limit = bytes;
+    return PG_OK;
+}
+
 pg_status pg_ws(pg_ctx* ctx, const char* key, size_t bytes, void** out)
 {
     auto& b = ctx->ws[key];
+    b.idle = false;
     if (b.bytes < bytes) {
         if (b.p) {
             PG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -215,7 +258,7 @@ pg_status pg_ws(pg_ctx* ctx, const char* key, size_t bytes, void** out)
             b.bytes = 0;
         }
         size_t want = bytes + bytes / 8;  // head room for slowly growing sizes
-        cudaError_t e = cudaMalloc(&b.p, want);
+        cudaError_t e = pg_malloc(ctx, &b.p, want);
         if (e != cudaSuccess) {
             cudaGetLastError();
             b.p = nullptr;
@@ -361,10 +404,17 @@ pg_status pg_graph_alloc(pg_ctx* ctx, int32_t n, int64_t nnz, bool weighted, pg_
     g->nnz = nnz;
     // stream-ordered on the context stream (pg_graph_free's cudaFree waits for
     // the device before the blocks return to the pool)
-    cudaError_t e = cudaMallocAsync((void**)&g->R, sizeof(int32_t) * ((size_t)n + 1), ctx->stream);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&g->C, sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1), ctx->stream);
-    if (e == cudaSuccess && weighted)
-        e = cudaMallocAsync((void**)&g->V, sizeof(float) * (size_t)(nnz > 0 ? nnz : 1), ctx->stream);
+    auto take = [&](void** p, size_t bytes) {
+        cudaError_t r = cudaMallocAsync(p, bytes, ctx->stream);
+        if (r == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (pg_ws_reclaim(ctx)) r = cudaMallocAsync(p, bytes, ctx->stream);
+        }
+        return r;
+    };
+    cudaError_t e = take((void**)&g->R, sizeof(int32_t) * ((size_t)n + 1));
+    if (e == cudaSuccess) e = take((void**)&g->C, sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1));
+    if (e == cudaSuccess && weighted) e = take((void**)&g->V, sizeof(float) * (size_t)(nnz > 0 ? nnz : 1));
     if (e != cudaSuccess) {
         cudaGetLastError();
         cudaFree(g->R); cudaFree(g->C); cudaFree(g->V);

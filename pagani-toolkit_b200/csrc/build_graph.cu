@@ -715,6 +715,8 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         return pg_fail(ctx, PG_ERR_INVALID, "unknown threshold mode %d", o.mode);
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     *out = nullptr;
+    // up to N^2 / 8 bytes of adjacency bits and the lists: for this call
+    const WsIdleAtExit<8> idle{ctx, {"b.bits", "b.wide", "b.wide_r", "b.band", "b.band_r", "b.key64", "b.pairs", "b.pw"}};
     pg_build_info inf;
     memset(&inf, 0, sizeof inf);
     const long long M1 = (long long)N * (N - 1) / 2;

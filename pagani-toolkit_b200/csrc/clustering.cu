@@ -422,6 +422,7 @@ extern "C" pg_status pg_clustering(pg_ctx* ctx, const pg_graph* g, int32_t kind,
     if (!ctx || !g || !cp) return pg_fail(ctx, PG_ERR_INVALID, "pg_clustering: null argument");
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     const int n = g->n;
+    const WsIdleAtExit<2> idle{ctx, {"on.roots", "on.up"}};   // 8 bytes per entry, for this call
     float* dcp;
     double* dmean;
     PG_TRY(pg_wst(ctx, "cl.cp", (size_t)n + 1, &dcp));

@@ -562,7 +562,7 @@ pg_status cohort_keys(pg_ctx* ctx, pg_cohort* c)
 {
     if (c->subjects < 1) return pg_fail(ctx, PG_ERR_INVALID, "cohort has no subjects");
     if (c->keys_valid) return PG_OK;
-    if (!c->keys) PG_CUDA(ctx, cudaMalloc(&c->keys, sizeof(unsigned long long) * (size_t)c->nelem));
+    if (!c->keys) PG_CUDA(ctx, pg_malloc(ctx, (void**)&c->keys, sizeof(unsigned long long) * (size_t)c->nelem));
     const int grid = block_grid(ctx, c->ntiles);
     if (c->fisher)
         k_cohort_keys<true><<<grid, 256, 0, ctx->stream>>>(c->acc, c->N, c->nb, c->ntiles, (double)c->subjects, c->keys);
@@ -592,7 +592,7 @@ extern "C" pg_status pg_cohort_create(pg_ctx* ctx, int32_t N, int32_t fisher, in
     c->fisher = fisher != 0;
     c->weighted = weighted != 0;
     c->M1 = (long long)N * (N - 1) / 2;
-    cudaError_t e = cudaMalloc(&c->acc, sizeof(double) * (size_t)c->nelem);
+    cudaError_t e = pg_malloc(ctx, (void**)&c->acc, sizeof(double) * (size_t)c->nelem);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->acc, 0, sizeof(double) * (size_t)c->nelem, ctx->stream);
     if (e != cudaSuccess) {
         const long long nelem = c->nelem;

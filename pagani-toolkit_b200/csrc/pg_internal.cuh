@@ -21,7 +21,8 @@ struct pg_ctx {
     int64_t launches = 0;
     std::string err;
     // Reusable device buffers keyed by name; grown on demand.
-    struct Buf { void* p = nullptr; size_t bytes = 0; };
+    // idle: no call uses it at present (pg_ws_idle); it goes when memory is short.
+    struct Buf { void* p = nullptr; size_t bytes = 0; bool idle = false; };
     std::map<std::string, Buf> ws;
     // Pinned host staging for small D2H/H2D transfers.
     void* pinned = nullptr;
@@ -43,6 +44,7 @@ struct pg_ctx {
     // the same for teams of CTAs (pg_debug_stall_next_team): a CTA of every
     // team of the next such launch holds back until the others gave up
     unsigned long long debug_team_stall_ns = 0;
+    size_t debug_memory_limit = 0;   // test hook (pg_debug_memory_limit): most device memory of the workspace
 };
 
 struct pg_graph {
@@ -93,6 +95,26 @@ int pg_prof_begin(pg_ctx* ctx, const char* name);
 void pg_prof_end(pg_ctx* ctx, int handle);
 
 // ------------------------------------------------------------- workspace
+// cudaMalloc that gives the idle workspace back where memory is short.
+cudaError_t pg_malloc(pg_ctx* ctx, void** out, size_t bytes);
+// Frees every idle buffer of the workspace (waits for the context stream);
+// false if there was none.
+bool pg_ws_reclaim(pg_ctx* ctx);
+// Until the next pg_ws of that key, the buffer may be freed for another one.
+// For scratch that a call holds for its own duration only and that later calls
+// of the context would otherwise find missing; all its users have been
+// enqueued on the context stream.
+void pg_ws_idle(pg_ctx* ctx, const char* key);
+// The same at the end of a scope, for a list of keys.
+template <size_t K>
+struct WsIdleAtExit {
+    pg_ctx* ctx;
+    const char* keys[K];
+    ~WsIdleAtExit()
+    {
+        for (const char* k : keys) pg_ws_idle(ctx, k);
+    }
+};
 // Device buffer named `key`, at least `bytes` long (contents undefined).
 pg_status pg_ws(pg_ctx* ctx, const char* key, size_t bytes, void** out);
 template <class T>

@@ -88,6 +88,7 @@ pg_status run_surrogates(pg_ctx* ctx, const pg_graph* g, int32_t subject, const 
                          double* lp_r, int32_t* replays)
 {
     const int nr = o.n_random;
+    const WsIdleAtExit<2> idle{ctx, {"on.roots", "on.up"}};
     SurrogateChain c{};
     c.weighted = g->V != nullptr;
     c.sg.ctx = ctx;
@@ -116,6 +117,8 @@ pg_status run_surrogates(pg_ctx* ctx, const pg_graph* g, int32_t subject, const 
     // path set-up look at them (the autotuner runs on this surrogate)
     PG_TRY(ms_enqueue(ctx, g, &c.ms));
     PG_TRY(ms_rows_enqueue(ctx, g, &c.ms, c.sg.C, c.sg.V));
+    // the last buffers are Onnela's roots, which can be done without
+    PG_TRY(paths_prepare(ctx, &c.sg, 0, &c.pa));
     if (c.weighted) {
         PG_TRY(onnela_prepare(ctx, &c.sg, 0, c.cp, c.cp_mean, &c.onn));
         PG_TRY(onnela_enqueue(ctx, &c.onn));
@@ -123,7 +126,6 @@ pg_status run_surrogates(pg_ctx* ctx, const pg_graph* g, int32_t subject, const 
         PG_TRY(binary_cp_prepare(ctx, g->n, &c.bin));
         PG_TRY(binary_cp_enqueue(ctx, &c.bin, c.sg.R, c.sg.C, c.sg.n, c.cp, nullptr, c.cp_mean));
     }
-    PG_TRY(paths_prepare(ctx, &c.sg, 0, &c.pa));
     PG_TRY(paths_enqueue(ctx, &c.pa));
     k_sr_collect<<<1, 1, 0, ctx->stream>>>(c.cp_mean, c.pa.out, c.cp_r, c.lp_r, c.round);
     PG_LAUNCHED(ctx);

@@ -33,7 +33,7 @@ EXPORTS = [
     "pg_cohort_create", "pg_cohort_add", "pg_cohort_graph", "pg_cohort_packed", "pg_cohort_info",
     "pg_cohort_free", "pg_profile_enable", "pg_profile_reset", "pg_profile_get",
     "pg_run_opts_default", "pg_surrogate_seed", "pg_run_subjects", "pg_debug_stall_next_gram",
-    "pg_debug_stall_next_team",
+    "pg_debug_stall_next_team", "pg_debug_memory_limit",
 ]
 
 
@@ -145,6 +145,7 @@ def lib():
         L.pg_run_subjects.argtypes = [vp, P(Subject), i32, P(RunOpts)]
         L.pg_debug_stall_next_gram.argtypes = [vp, ct.c_uint64]
         L.pg_debug_stall_next_team.argtypes = [vp, ct.c_uint64]
+        L.pg_debug_memory_limit.argtypes = [vp, ct.c_uint64]
         _lib = L
     return _lib
 

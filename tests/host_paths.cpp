@@ -36,12 +36,52 @@ static int large_copy_that_fails(pg_ctx* ctx)
     return 0;
 }
 
+// scratch that no call uses goes when memory is short, and only then
+static int idle_buffers_make_room(pg_ctx* ctx)
+{
+    void *a, *b, *c;
+    fake::device_limit = 1000;
+    CHECK(pg_ws(ctx, "a", 400, &a) == PG_OK);
+    CHECK(pg_ws(ctx, "b", 400, &b) == PG_OK);
+    CHECK(pg_ws(ctx, "c", 400, &c) == PG_ERR_NOMEM);      // both are in use
+    pg_ws_idle(ctx, "a");
+    CHECK(pg_ws(ctx, "a", 400, &c) == PG_OK && c == a);   // taken again: the same buffer, in use
+    CHECK(pg_ws(ctx, "c", 400, &c) == PG_ERR_NOMEM);
+    pg_ws_idle(ctx, "a");
+    CHECK(pg_ws(ctx, "c", 400, &c) == PG_OK);
+    CHECK(fake::device_bytes == 2 * 450);
+    CHECK(ctx->ws["a"].p == nullptr && ctx->ws["b"].p == b);
+    // graphs too
+    pg_ws_idle(ctx, "b");
+    const int32_t R[3] = {0, 1, 2}, C[2] = {1, 0};
+    pg_graph* g = nullptr;
+    fake::device_limit = 905;
+    CHECK(pg_graph_from_csr(ctx, R, C, nullptr, 2, 2, 0, &g) == PG_OK);
+    CHECK(ctx->ws["b"].p == nullptr && ctx->ws["c"].p == c);
+    CHECK(pg_graph_free(g) == PG_OK);
+    CHECK(fake::device_bytes == 450);
+    return 0;
+}
+
+// no pinned memory for the staging buffers: the plain copy
+static int large_copy_without_staging(pg_ctx* ctx)
+{
+    const size_t bytes = 20u << 20;
+    std::vector<unsigned char> src(bytes, 7), dst(bytes, 0);
+    fake::host_limit = 1 << 20;
+    CHECK(pg_d2h_large(ctx, dst.data(), src.data(), bytes) == PG_OK);
+    CHECK(dst == src && fake::copies == 1);
+    return 0;
+}
+
 int main(int argc, char** argv)
 {
     pg_ctx* ctx;
     if (argc < 2 || pg_create(&ctx, 0) != PG_OK) return 2;
     int rc = 2;
     if (!strcmp(argv[1], "large_copy_that_fails")) rc = large_copy_that_fails(ctx);
+    if (!strcmp(argv[1], "idle_buffers_make_room")) rc = idle_buffers_make_room(ctx);
+    if (!strcmp(argv[1], "large_copy_without_staging")) rc = large_copy_without_staging(ctx);
     pg_destroy(ctx);
     if (rc == 0) puts("ok");
     return rc;

@@ -26,7 +26,7 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["large_copy_that_fails"])
+@pytest.mark.parametrize("name", ["large_copy_that_fails", "large_copy_without_staging", "idle_buffers_make_room"])
 def test_host_path(harness, name):
     r = subprocess.run([harness, name], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr

@@ -1,0 +1,46 @@
+"""Calls in little device memory (a limit on the context's workspace stands in
+for a full device): scratch of one call does not stay in the way of the next."""
+import numpy as np
+import pytest
+
+import pagani
+from pagani import synth
+from tests import graphs as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _limit(c, bytes_):
+    pagani.lib().pg_debug_memory_limit(c.h, int(bytes_))
+
+
+def test_scratch_of_a_build_makes_room(ctx):
+    bold = synth.bold_series(9000, 48, 6, 9000)
+    fw = G.random_weighted(2500, 0.01, 1)
+    want = ctx.fw_paths(ctx.graph(*fw))
+    with pagani.Context(0) as c:
+        _limit(c, 60e6)                       # the build holds 46 MB, the sweep wants 30 more
+        g, _ = c.build_graph(bold, mode="s", value=6.0)
+        h = c.graph(*fw)
+        eff, lp = c.fw_paths(h)
+        assert np.array_equal(eff, want[0]) and lp == want[1]
+        del g, h
+
+
+def test_roots_of_onnela_make_room(ctx):
+    R, C, V = G.random_weighted(3000, 0.25, 2)         # 2.2 million entries: 18 MB of roots
+    want = ctx.clustering(ctx.graph(R, C, V), kind="onnela")[0]
+    fw = G.random_weighted(1200, 0.02, 3)
+    lp = ctx.fw_paths(ctx.graph(*fw))[1]
+    with pagani.Context(0) as c:
+        g, h = c.graph(R, C, V), c.graph(*fw)
+        _limit(c, 22e6)
+        assert np.array_equal(c.clustering(g, kind="onnela")[0], want)
+        assert c.fw_paths(h)[1] == lp
+        _limit(c, 2e6)                        # no room for roots: the kernel that needs none
+        with pagani.Context(0) as d:
+            _limit(d, 2e6)
+            k = d.graph(R, C, V)
+            np.testing.assert_allclose(d.clustering(k, kind="onnela")[0], want, rtol=2.0 ** -22)
+            del k
+        del g, h
