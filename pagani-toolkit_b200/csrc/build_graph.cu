@@ -366,10 +366,14 @@ k_sel_pass(const unsigned long long* __restrict__ keys, long long n, SelState* _
 
 pg_status pg_radix_select(pg_ctx* ctx, const unsigned long long* keys, long long n, long long m, SelState* st_dev)
 {
-    const long long cap = std::min(8LL << 20, n / 16 + 1024);
+    long long cap = std::min(8LL << 20, n / 16 + 1024);
+    const WsIdleAtExit<1> idle{ctx, {"sel.list"}};
     unsigned long long *hist, *list;
     PG_TRY(pg_wst(ctx, "sel.hist", SEL_BINS, &hist));
-    PG_TRY(pg_wst(ctx, "sel.list", (size_t)cap, &list));
+    if (pg_wst(ctx, "sel.list", (size_t)cap, &list) != PG_OK) {   // every pass reads all keys then
+        cap = 0;
+        list = nullptr;
+    }
     SelState* init;
     PG_TRY(pg_hwst(ctx, "sel.init", 1, &init));
     *init = SelState{0ULL, 0ULL, m, n, 0LL, 0u, 0};
@@ -703,13 +707,10 @@ static pg_status run_gram(pg_ctx* ctx, const ZOperands& z, int precision, int mo
 // build; at 58,000 nodes lists for every pair would take 47 GB.
 constexpr long long LIST_ALL_PAIRS = 1LL << 22;
 
-extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, int32_t T,
-                                    const pg_build_opts* opts_in, pg_graph** out, pg_build_info* info)
+// lean: the route that needs least memory, lists sized by a full histogram.
+static pg_status build_graph(pg_ctx* ctx, const float* bold, int N, int T, const pg_build_opts& o, bool lean,
+                             pg_graph** out, pg_build_info* info)
 {
-    if (!ctx || !bold || !out || N < 1 || T < 1)
-        return pg_fail(ctx, PG_ERR_INVALID, "pg_build_graph: bad arguments (N=%d T=%d)", N, T);
-    pg_build_opts o;
-    if (opts_in) o = *opts_in; else pg_build_opts_default(&o);
     if (!(o.guard >= 0.0) || o.guard > 0.5) return pg_fail(ctx, PG_ERR_INVALID, "guard %g out of range", o.guard);
     if (o.mode != PG_THRESH_R && o.mode != PG_THRESH_SPARSITY)
         return pg_fail(ctx, PG_ERR_INVALID, "unknown threshold mode %d", o.mode);
@@ -786,7 +787,7 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         for (int b = 0; b < HIST_BINS; b++) s += h[b];
         return s;
     };
-    const bool list_all = o.mode == PG_THRESH_R && M1 <= LIST_ALL_PAIRS;
+    const bool list_all = !lean && o.mode == PG_THRESH_R && M1 <= LIST_ALL_PAIRS;
     const bool no_band = g == 0.0 && o.mode == PG_THRESH_R;
     const long long ntiles = (long long)(z.Np / 128) * (z.Np / 128 + 1) / 2;
     const int bit_words = z.Np / 32;
@@ -808,7 +809,7 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     // Weights need the list; the bits may take 8 GiB, and where they cannot be
     // had the (then smaller) list serves.
     auto bits_pay = [&](long long edges) {
-        return !weighted && bit_bytes <= (8ULL << 30) &&
+        return !lean && !weighted && bit_bytes <= (8ULL << 30) &&
                (list_all || (double)edges >= 1.3e-3 * (double)N * (double)N) &&
                pg_wst(ctx, "b.bits", (size_t)N * bit_words, &bits) == PG_OK;
     };
@@ -872,7 +873,7 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     // two sampled tiles per SM it costs no more than the sample.
     float floor_key = key_lo;
     bool one_pass = false;
-    const bool sampled = !list_all && (o.mode == PG_THRESH_R || k_edges > 0) && ntiles >= 16LL * ctx->sm_count;
+    const bool sampled = !list_all && (o.mode == PG_THRESH_R ? !lean : k_edges > 0) && ntiles >= 16LL * ctx->sm_count;
     if (sampled) {
         PG_TRY(hist_pass(o.mode == PG_THRESH_R ? r_floor : key_lo, 8));
         const double f = (double)(hist_total() + (o.mode == PG_THRESH_R ? (long long)hbelow[0] : 0)) / (double)M1;
@@ -917,7 +918,7 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
         cap_pairs = room(n_above);
         cap_band = no_band ? 0 : room(n_list);
         cap_total = cap_pairs + cap_band;
-        if (fits && cap_pairs <= (long long)INT32_MAX) {
+        if (fits && !lean && cap_pairs <= (long long)INT32_MAX) {   // lean: the sample places the floor only
             use_bits = bits_pay(k_edges >= 0 ? k_edges : cap_pairs);
             if (use_bits) cap_pairs = cap_total = M1;
             PG_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
@@ -1139,4 +1140,22 @@ extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, i
     if (info) *info = inf;
     *out = gph;
     return PG_OK;
+}
+
+extern "C" pg_status pg_build_graph(pg_ctx* ctx, const float* bold, int32_t N, int32_t T,
+                                    const pg_build_opts* opts_in, pg_graph** out, pg_build_info* info)
+{
+    if (!ctx || !bold || !out || N < 1 || T < 1)
+        return pg_fail(ctx, PG_ERR_INVALID, "pg_build_graph: bad arguments (N=%d T=%d)", N, T);
+    pg_build_opts o;
+    if (opts_in) o = *opts_in; else pg_build_opts_default(&o);
+    pg_status st = build_graph(ctx, bold, N, T, o, false, out, info);
+    if (st == PG_ERR_NOMEM) {
+        // sampled list sizes, lists of every pair and adjacency bits want room
+        // to spare: where that is missing, the route that sizes its lists
+        // exactly, in memory that holds nothing else of the first attempt
+        pg_ws_reclaim(ctx);
+        st = build_graph(ctx, bold, N, T, o, true, out, info);
+    }
+    return st;
 }

@@ -1,5 +1,6 @@
 """Calls in little device memory (a limit on the context's workspace stands in
-for a full device): scratch of one call does not stay in the way of the next."""
+for a full device): routes that want room to spare give way to those that do
+not, and scratch of one call does not stay in the way of the next."""
 import numpy as np
 import pytest
 
@@ -12,6 +13,29 @@ pytestmark = pytest.mark.gpu
 
 def _limit(c, bytes_):
     pagani.lib().pg_debug_memory_limit(c.h, int(bytes_))
+
+
+# limits: what a build with exactly sized lists needs, with a tenth to spare
+@pytest.mark.parametrize("N,T,mb,kw", [
+    (2000, 100, 6, dict(mode="r", value=0.6)), (2000, 100, 6, dict(mode="r", value=0.6, weighted=True)),
+    (2000, 100, 6, dict(mode="s", value=1.0)), (9000, 48, 10.5, dict(mode="r", value=0.6, weighted=True)),
+    (9000, 48, 10.5, dict(mode="s", value=0.05)), (9000, 48, 30.5, dict(mode="s", value=1.0, precision="fp32"))])
+def test_build_with_exact_lists(ctx, N, T, mb, kw):
+    bold = synth.bold_series(N, T, 6, N)
+    g, info = ctx.build_graph(bold, **kw)
+    R, C, V = g.to_csr()
+    with pagani.Context(0) as c:
+        _limit(c, mb * 1e6)
+        g2, info2 = c.build_graph(bold, **kw)
+        R2, C2, V2 = g2.to_csr()
+        assert np.array_equal(R, R2) and np.array_equal(C, C2) and info["tau"] == info2["tau"]
+        assert np.array_equal(V, V2) if V is not None else V2 is None
+        with pagani.Context(0) as none:      # and an error, not a crash, where nothing fits
+            _limit(none, 1e6)
+            with pytest.raises(pagani.PaganiError) as e:
+                none.build_graph(bold, **kw)
+            assert e.value.status == 3
+        del g2
 
 
 def test_scratch_of_a_build_makes_room(ctx):
