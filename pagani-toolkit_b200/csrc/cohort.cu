@@ -661,9 +661,10 @@ extern "C" pg_status pg_cohort_add(pg_ctx* ctx, pg_cohort* c, const float* bold,
     if (!bold || T < 1) return pg_fail(ctx, PG_ERR_INVALID, "pg_cohort_add: bad arguments (T=%d)", T);
     PG_CUDA(ctx, cudaSetDevice(ctx->device));
     PG_TRY(gram64_operands(ctx, bold, c->N, T, input_on_device != 0));
-    c->keys_valid = false;
-    c->subjects++;
-    if (c->M1 == 0) return PG_OK;
+    if (c->M1 == 0) {
+        c->subjects++;
+        return PG_OK;
+    }
     CohortArgs a = {};
     a.ntiles = c->ntiles;
     a.acc = c->acc;
@@ -675,6 +676,10 @@ extern "C" pg_status pg_cohort_add(pg_ctx* ctx, pg_cohort* c, const float* bold,
         c->broken = true;   // the accumulator may hold part of this subject
         return pg_fail(ctx, PG_ERR_TIMEOUT, "cohort Gram: a pipeline wait timed out; the cohort is unusable");
     }
+    // a subject counts once its sums are in (a call that could not get its
+    // scratch leaves the average as it was)
+    c->keys_valid = false;
+    c->subjects++;
     return PG_OK;
 }
 

@@ -68,3 +68,34 @@ def test_roots_of_onnela_make_room(ctx):
             np.testing.assert_allclose(d.clustering(k, kind="onnela")[0], want, rtol=2.0 ** -22)
             del k
         del g, h
+
+
+def test_subject_that_could_not_be_added_does_not_count(ctx):
+    """The largest limit at which an add still fails: all but its last buffer."""
+    bolds = [synth.bold_series(260, 40, 4, s) for s in (1, 2)]
+
+    def add(limit):
+        with pagani.Context(0) as c, c.cohort(260, fisher=True) as avg:
+            _limit(c, limit)
+            try:
+                avg.add(bolds[0])
+                ok = True
+            except pagani.PaganiError as e:
+                assert e.status == 3
+                ok = False
+            assert avg.subjects == int(ok)
+            _limit(c, 0)
+            avg.add(bolds[1])
+            return ok, avg.packed()
+    with ctx.cohort(260, fisher=True) as alone:
+        alone.add(bolds[1])
+        want = alone.packed()
+    lo, hi = 1 << 10, 1 << 24
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        ok, packed = add(mid)
+        if ok:
+            hi = mid
+        else:
+            lo = mid
+            assert np.array_equal(packed, want)
