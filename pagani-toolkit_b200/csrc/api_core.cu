@@ -84,7 +84,6 @@ extern "C" pg_status pg_destroy(pg_ctx* ctx)
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (auto& kv : ctx->ws) cudaFree(kv.second.p);
-    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     for (auto& kv : ctx->hws) cudaFreeHost(kv.second.p);
     for (auto& st : ctx->pool) cudaStreamDestroy(st);
     for (auto& e : ctx->ev) cudaEventDestroy(e);
@@ -267,19 +266,6 @@ pg_status pg_ws(pg_ctx* ctx, const char* key, size_t bytes, void** out)
         b.bytes = want;
     }
     *out = b.p;
-    return PG_OK;
-}
-
-pg_status pg_pinned(pg_ctx* ctx, size_t bytes, void** out)
-{
-    if (ctx->pinned_bytes < bytes) {
-        if (ctx->pinned) cudaFreeHost(ctx->pinned);
-        ctx->pinned = nullptr;
-        ctx->pinned_bytes = 0;
-        PG_CUDA(ctx, cudaMallocHost(&ctx->pinned, bytes));
-        ctx->pinned_bytes = bytes;
-    }
-    *out = ctx->pinned;
     return PG_OK;
 }
 
@@ -741,19 +727,6 @@ pg_status launch_row_sort(pg_ctx* ctx, const int32_t* R, int32_t n, const int32_
     k_row_bitmap_sort<<<grid, 256, smem, ctx->stream>>>(R, n, Cin, Vin, Cout, Vout);
     PG_LAUNCHED(ctx);
     return PG_OK;
-}
-
-pg_status pg_csr_sort_rows(pg_ctx* ctx, pg_graph* g)
-{
-    if (g->nnz == 0) return PG_OK;
-    int32_t* Ct;
-    float* Vt = nullptr;
-    PG_TRY(pg_wst(ctx, "sort.C", (size_t)g->nnz, &Ct));
-    if (g->V) PG_TRY(pg_wst(ctx, "sort.V", (size_t)g->nnz, &Vt));
-    PG_CUDA(ctx, cudaMemcpyAsync(Ct, g->C, sizeof(int32_t) * g->nnz, cudaMemcpyDeviceToDevice, ctx->stream));
-    if (g->V)
-        PG_CUDA(ctx, cudaMemcpyAsync(Vt, g->V, sizeof(float) * g->nnz, cudaMemcpyDeviceToDevice, ctx->stream));
-    return launch_row_sort(ctx, g->R, g->n, Ct, Vt, g->C, g->V);
 }
 
 pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const float* w, int64_t npairs,

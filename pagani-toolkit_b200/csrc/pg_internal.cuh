@@ -24,9 +24,6 @@ struct pg_ctx {
     // idle: no call uses it at present (pg_ws_idle); it goes when memory is short.
     struct Buf { void* p = nullptr; size_t bytes = 0; bool idle = false; };
     std::map<std::string, Buf> ws;
-    // Pinned host staging for small D2H/H2D transfers.
-    void* pinned = nullptr;
-    size_t pinned_bytes = 0;
     // Pinned host buffers keyed by name, grown on demand, and a pool of
     // non-blocking streams: for host loops that keep many streams busy.
     std::map<std::string, Buf> hws;
@@ -122,8 +119,6 @@ inline pg_status pg_wst(pg_ctx* ctx, const char* key, size_t count, T** out)
 {
     return pg_ws(ctx, key, count * sizeof(T) + 256, (void**)out);
 }
-// Pinned host staging buffer of at least `bytes`.
-pg_status pg_pinned(pg_ctx* ctx, size_t bytes, void** out);
 // Pinned host buffer named `key`, at least `bytes` long (contents undefined;
 // growing it synchronises the device).
 pg_status pg_hws(pg_ctx* ctx, const char* key, size_t bytes, void** out);
@@ -151,8 +146,6 @@ pg_status pg_csr_from_pairs(pg_ctx* ctx, int32_t n, const int2* pairs, const flo
                             int64_t npairs, pg_graph** out);
 // Row offsets R[n+1] from the row counts; the counts become the row starts.
 pg_status pg_row_offsets(pg_ctx* ctx, int32_t* cnt, int32_t n, int32_t* R);
-// Sorts the columns of every row ascending (carrying V when present).
-pg_status pg_csr_sort_rows(pg_ctx* ctx, pg_graph* g);
 // Row sort of a CSR whose rows are filled but unordered: Cin/Vin -> Cout/Vout
 // (Vin may be null).  Only launches kernels (capture-safe once the kernel's
 // shared-memory attribute has been set by a first call).
