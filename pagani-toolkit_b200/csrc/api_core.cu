@@ -312,11 +312,13 @@ pg_status pg_d2h(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
 // Large results go through pinned staging buffers, several host threads each
 // copying its own chunks out while the next ones arrive: the driver's own
 // staging is one thread, and most of its time goes into the first touch of the
-// caller's fresh pages (50 MB: 10.9 -> 2.9 ms with eight threads).  Below 8 MB
-// the threads cost what they bring, and pinned or managed memory takes the
-// direct copy, as does everything where the 32 MB of staging cannot be had.
-// Synchronous, on the context stream.
-constexpr size_t D2H_LARGE_BYTES = 8u << 20;
+// caller's fresh pages (50 MB: 10.9 -> 2.9 ms with eight threads).  Below 16 MB
+// starting the threads costs what they bring where the pages have been touched
+// before, as an allocator's mostly have (distances of 1,500 nodes, 9 MB: copy
+// 0.55 ms alone, 0.65 with threads; 16 MB 0.93 / 0.85; 32 MB 1.9 / 1.4), and
+// pinned or managed memory takes the direct copy, as does everything where the
+// 32 MB of staging cannot be had.  Synchronous, on the context stream.
+constexpr size_t D2H_LARGE_BYTES = 16u << 20;
 pg_status pg_d2h_large(pg_ctx* ctx, void* dst, const void* src, size_t bytes)
 {
     constexpr size_t CHUNK = 2u << 20;
