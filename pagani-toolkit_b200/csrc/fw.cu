@@ -208,7 +208,8 @@ struct __align__(16) FwSmem {
         } prod;
         struct {
             float dg[B][B + 4];     // the closed diagonal block (transposed for a column panel)
-            float rows[2][8][B];    // the eight rows whose steps come next
+            float rows[8][B];       // the eight rows whose steps come next
+            float2 b[4][B];         // the same at their own steps, two and two interleaved
             float tr[B][B + 1];     // for turning a column panel
         } panel;
         struct {
@@ -319,15 +320,19 @@ __device__ __forceinline__ void min_plus(FwSmem& sm, Tile& c, const float* a, co
 // result: a product with the untouched panel is as exact, but it associates
 // the FP32 sums of paths of three and more edges the other way round, which
 // moves distances by their last bit.
-// Eight steps at a time, with one barrier: every thread takes the eight rows
-// s_k.. of its four columns from shared memory, brings them to their own steps
-// (a triangle of updates, done by all eight owners of a column alike), and
+// Eight steps at a time: their rows go to shared memory, a thread per column
+// brings them to their own steps (a triangle of updates), and every thread
 // folds them into its tile as min_plus does.  The minima are exact, so this
-// equals the 64 steps, which took a barrier each (2,500 nodes: 2.06 ms, with
-// the panels as plain products 1.85, with 64 barriers a panel 2.82).
+// equals the 64 steps, which took a barrier each (2,500 nodes: 2.02 ms, with
+// the panels as plain products 1.85, with 64 barriers a panel 2.82; with the
+// triangle in every thread and one barrier instead of two 2.06).
 __device__ __forceinline__ void close_panel(FwSmem& sm, Tile& c, const float* dg, float* d, int ld, bool row, int kn)
 {
     const int t = group_thread(), i0 = t >> 4, j0 = 2 * (t & 15);
+    // the solvers: two warps of the group, other ones in every second group (an
+    // SM's four schedulers each hold a warp of every group)
+    const int j = t & (B - 1);
+    const bool solver = (t >> 6) == ((threadIdx.x >> 7) & 1);
     c.load(d, ld);
 #pragma unroll
     for (int it = 0; it < B * B / 4 / GT; it++) {
@@ -347,7 +352,6 @@ __device__ __forceinline__ void close_panel(FwSmem& sm, Tile& c, const float* dg
     if (!row) c.transpose(sm.panel.tr);
 #pragma unroll 1
     for (int k0 = 0; k0 < kn; k0 += 8) {
-        float (*buf)[B] = sm.panel.rows[(k0 >> 3) & 1];
         float own[4];
 #pragma unroll
         for (int x = 0; x < 4; x++) {
@@ -355,46 +359,48 @@ __device__ __forceinline__ void close_panel(FwSmem& sm, Tile& c, const float* dg
 #pragma unroll
             for (int r = 1; r < TR; r++) own[x] = k0 == 8 * r ? c.v[r][x] : own[x];
         }
-        *(float2*)&buf[i0][j0] = make_float2(own[0], own[1]);
-        *(float2*)&buf[i0][j0 + 32] = make_float2(own[2], own[3]);
-        group_sync();   // the other buffer is written next, this one after another barrier
-        float2 b[4][4];   // rows k0 + 2 h, + 1 of the thread's columns
+        *(float2*)&sm.panel.rows[i0][j0] = make_float2(own[0], own[1]);
+        *(float2*)&sm.panel.rows[i0][j0 + 32] = make_float2(own[2], own[3]);
+        group_sync();
+        if (solver) {
+            float2 s[4];   // rows k0 + 2 h, + 1 of column j
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-            const float2 x = *(const float2*)&buf[2 * h][j0], y = *(const float2*)&buf[2 * h + 1][j0];
-            const float2 z = *(const float2*)&buf[2 * h][j0 + 32], w = *(const float2*)&buf[2 * h + 1][j0 + 32];
-            b[h][0] = make_float2(x.x, y.x);
-            b[h][1] = make_float2(x.y, y.y);
-            b[h][2] = make_float2(z.x, w.x);
-            b[h][3] = make_float2(z.y, w.y);
-        }
-        // the rows at their own steps
+            for (int h = 0; h < 4; h++) s[h] = make_float2(sm.panel.rows[2 * h][j], sm.panel.rows[2 * h + 1][j]);
 #pragma unroll
-        for (int k = 1; k < 8; k++) {
-            const float4 lo = *(const float4*)&sm.panel.dg[k0 + k][k0], hi = *(const float4*)&sm.panel.dg[k0 + k][k0 + 4];
-            const float2 a[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
-#pragma unroll
-            for (int x = 0; x < 4; x++) {
-                float& s = (k & 1) ? b[k / 2][x].y : b[k / 2][x].x;
+            for (int k = 1; k < 8; k++) {
+                const float4 lo = *(const float4*)&sm.panel.dg[k0 + k][k0], hi = *(const float4*)&sm.panel.dg[k0 + k][k0 + 4];
+                const float2 a[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+                float& v = (k & 1) ? s[k / 2].y : s[k / 2].x;
 #pragma unroll
                 for (int h = 0; h < k / 2; h++) {
-                    const float2 p = add2(a[h], b[h][x]);
-                    s = min3f(s, p.x, p.y);
+                    const float2 p = add2(a[h], s[h]);
+                    v = min3f(v, p.x, p.y);
                 }
-                if (k & 1) s = fminf(s, a[k / 2].x + b[k / 2][x].x);
+                if (k & 1) v = fminf(v, a[k / 2].x + s[k / 2].x);
             }
+#pragma unroll
+            for (int h = 0; h < 4; h++) sm.panel.b[h][j] = s[h];
+        }
+        group_sync();   // `rows` is free; `b` is written again behind the next barrier
+        float4 bl[4], bh[4];
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            bl[h] = *(const float4*)&sm.panel.b[h][j0];
+            bh[h] = *(const float4*)&sm.panel.b[h][j0 + 32];
         }
 #pragma unroll
         for (int r = 0; r < TR; r++) {
             const float4 lo = *(const float4*)&sm.panel.dg[i0 + 8 * r][k0], hi = *(const float4*)&sm.panel.dg[i0 + 8 * r][k0 + 4];
             const float2 a[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
 #pragma unroll
-            for (int h = 0; h < 4; h++)
-#pragma unroll
-                for (int x = 0; x < 4; x++) {
-                    const float2 p = add2(a[h], b[h][x]);
-                    c.v[r][x] = min3f(c.v[r][x], p.x, p.y);
-                }
+            for (int h = 0; h < 4; h++) {
+                const float2 s0 = add2(a[h], make_float2(bl[h].x, bl[h].y)), s1 = add2(a[h], make_float2(bl[h].z, bl[h].w));
+                const float2 s2 = add2(a[h], make_float2(bh[h].x, bh[h].y)), s3 = add2(a[h], make_float2(bh[h].z, bh[h].w));
+                c.v[r][0] = min3f(c.v[r][0], s0.x, s0.y);
+                c.v[r][1] = min3f(c.v[r][1], s1.x, s1.y);
+                c.v[r][2] = min3f(c.v[r][2], s2.x, s2.y);
+                c.v[r][3] = min3f(c.v[r][3], s3.x, s3.y);
+            }
         }
     }
     if (!row) c.transpose(sm.panel.tr);
