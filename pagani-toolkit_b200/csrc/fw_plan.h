@@ -18,9 +18,9 @@ struct FwPlan {
 // bundles of about 1 MB of matrices (an SM's share of a round is several
 // blocks, what is being swept stays in L2, a barrier has four arrivals): the
 // busiest team's work must be within a quarter of an even share.  Measured,
-// teams against one: 512 graphs of 90 to 1024 nodes 10.7 / 11.2 ms, 512 of 90
-// to 520 3.8 / 4.1; where this rule has one team, 64 graphs of 90 to 1024 3.2
-// / 1.7 ms, 16 of 90 to 520 0.72 / 0.41, one of 1500 with 60 of 120 10.1 / 1.2.
+// teams against one: 512 graphs of 90 to 1024 nodes 10.6 / 10.9 ms, 512 of 90
+// to 520 3.9 / 4.0; where this rule has one team, 64 graphs of 90 to 1024 3.6
+// / 1.6 ms, 16 of 90 to 520 0.69 / 0.38, one of 1500 with 60 of 120 10.0 / 1.1.
 inline FwPlan fw_batch_plan(const int* nb, int ng, int sm_count, int max_teams)
 {
     constexpr double BUNDLE_BYTES = 1 << 20, UNEVEN = 1.25;
