@@ -69,10 +69,13 @@ pg_status tune_pick(pg_ctx* ctx, const std::string& key, const std::vector<TuneC
         std::lock_guard<std::mutex> lk(g_mu);
         load_locked();
         auto it = g_table.find(key);
-        if (it != g_table.end()) {
-            *best = it->second;
-            return PG_OK;
-        }
+        // a choice saved by another build of the kernel may not fit an SM any more
+        if (it != g_table.end())
+            for (const TuneChoice& c : cands)
+                if (c.a == it->second.a && c.b == it->second.b) {
+                    *best = c;
+                    return PG_OK;
+                }
     }
     const char* off = getenv("PAGANI_TUNE");
     if ((off && off[0] == '0') || cands.size() < 2) return PG_OK;

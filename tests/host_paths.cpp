@@ -6,6 +6,7 @@
 #include <thread>
 #include <vector>
 #include "../pagani-toolkit_b200/csrc/pg_internal.cuh"
+#include "../pagani-toolkit_b200/csrc/tune.cuh"
 #include "fake_cudart.h"
 
 #define CHECK(x)                                            \
@@ -74,6 +75,25 @@ static int large_copy_without_staging(pg_ctx* ctx)
     return 0;
 }
 
+// a tuning file from another build: its choice is not among the candidates
+static int saved_choice_that_does_not_fit(pg_ctx* ctx)
+{
+    const char* path = getenv("PAGANI_TUNE_CACHE");
+    CHECK(path);
+    const std::string key = tune_key("test", 1000, 8000), other = tune_key("test", 100000, 800000);
+    FILE* f = fopen(path, "w");
+    CHECK(f);
+    fprintf(f, "%s 4 4 0.1\n%s 8 2 0.1\n", key.c_str(), other.c_str());
+    fclose(f);
+    const std::vector<TuneChoice> cands = {{4, 2}, {8, 2}};
+    TuneChoice best{0, 0};
+    int runs = 0;
+    auto run = [&](const TuneChoice&) -> pg_status { runs++; return PG_OK; };
+    CHECK(tune_pick(ctx, other, cands, &best, run) == PG_OK && best.a == 8 && best.b == 2 && runs == 0);
+    CHECK(tune_pick(ctx, key, cands, &best, run) == PG_OK && best.b == 2 && runs == 4);
+    return 0;
+}
+
 int main(int argc, char** argv)
 {
     pg_ctx* ctx;
@@ -82,6 +102,7 @@ int main(int argc, char** argv)
     if (!strcmp(argv[1], "large_copy_that_fails")) rc = large_copy_that_fails(ctx);
     if (!strcmp(argv[1], "idle_buffers_make_room")) rc = idle_buffers_make_room(ctx);
     if (!strcmp(argv[1], "large_copy_without_staging")) rc = large_copy_without_staging(ctx);
+    if (!strcmp(argv[1], "saved_choice_that_does_not_fit")) rc = saved_choice_that_does_not_fit(ctx);
     pg_destroy(ctx);
     if (rc == 0) puts("ok");
     return rc;

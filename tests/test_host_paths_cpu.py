@@ -17,7 +17,7 @@ def harness(tmp_path_factory):
     inc = os.path.join(os.path.dirname(HERE), "include")
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(NVCC))), "include")
     objs, exe = [], str(d / "host_paths")
-    for src in (os.path.join(PKG, "csrc", "api_core.cu"), os.path.join(HERE, "host_paths.cpp")):
+    for src in (os.path.join(PKG, "csrc", "api_core.cu"), os.path.join(PKG, "csrc", "tune.cu"), os.path.join(HERE, "host_paths.cpp")):
         objs.append(str(d / (os.path.basename(src) + ".o")))
         subprocess.run([NVCC, "-x", "cu", "-gencode", "arch=compute_100a,code=sm_100a", "-O1", "-std=c++17", f"-I{inc}",
                         "-c", src, "-o", objs[-1]], check=True)
@@ -26,7 +26,9 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("name", ["large_copy_that_fails", "large_copy_without_staging", "idle_buffers_make_room"])
-def test_host_path(harness, name):
-    r = subprocess.run([harness, name], capture_output=True, text=True, timeout=120)
+@pytest.mark.parametrize("name", ["large_copy_that_fails", "large_copy_without_staging", "idle_buffers_make_room",
+                                  "saved_choice_that_does_not_fit"])
+def test_host_path(harness, name, tmp_path):
+    r = subprocess.run([harness, name], capture_output=True, text=True, timeout=120,
+                       env=dict(os.environ, PAGANI_TUNE_CACHE=str(tmp_path / "tune.txt")))
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
