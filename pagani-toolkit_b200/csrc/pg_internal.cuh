@@ -57,10 +57,13 @@ struct pg_graph {
 // ---------------------------------------------------------------- errors
 pg_status pg_fail(pg_ctx* ctx, pg_status s, const char* fmt, ...);
 
+// The runtime's record of the error is cleared: it would be taken for the next
+// call's launch error.
 #define PG_CUDA(ctx, call)                                                              \
     do {                                                                                \
         cudaError_t e_ = (call);                                                        \
         if (e_ != cudaSuccess) {                                                        \
+            cudaGetLastError();                                                         \
             return pg_fail((ctx), e_ == cudaErrorMemoryAllocation ? PG_ERR_NOMEM         \
                                                                   : PG_ERR_CUDA,        \
                            "%s:%d %s: %s", __FILE__, __LINE__, #call,                   \

@@ -94,6 +94,18 @@ static int saved_choice_that_does_not_fit(pg_ctx* ctx)
     return 0;
 }
 
+// the error of a call that failed is not taken for the next call's launch error
+static int error_that_is_over(pg_ctx* ctx)
+{
+    char a[8] = {}, b[8] = {};
+    fake::fail_copy = 0;
+    CHECK(pg_d2h(ctx, a, b, sizeof a) == PG_ERR_CUDA);
+    fake::fail_copy = -1;
+    int32_t cnt[3] = {1, 1, 0}, R[3] = {};
+    CHECK(pg_row_offsets(ctx, cnt, 2, R) == PG_OK);   // two launches, each checked
+    return 0;
+}
+
 int main(int argc, char** argv)
 {
     pg_ctx* ctx;
@@ -103,6 +115,7 @@ int main(int argc, char** argv)
     if (!strcmp(argv[1], "idle_buffers_make_room")) rc = idle_buffers_make_room(ctx);
     if (!strcmp(argv[1], "large_copy_without_staging")) rc = large_copy_without_staging(ctx);
     if (!strcmp(argv[1], "saved_choice_that_does_not_fit")) rc = saved_choice_that_does_not_fit(ctx);
+    if (!strcmp(argv[1], "error_that_is_over")) rc = error_that_is_over(ctx);
     pg_destroy(ctx);
     if (rc == 0) puts("ok");
     return rc;

@@ -27,7 +27,7 @@ def harness(tmp_path_factory):
 
 
 @pytest.mark.parametrize("name", ["large_copy_that_fails", "large_copy_without_staging", "idle_buffers_make_room",
-                                  "saved_choice_that_does_not_fit"])
+                                  "saved_choice_that_does_not_fit", "error_that_is_over"])
 def test_host_path(harness, name, tmp_path):
     r = subprocess.run([harness, name], capture_output=True, text=True, timeout=120,
                        env=dict(os.environ, PAGANI_TUNE_CACHE=str(tmp_path / "tune.txt")))
